@@ -19,7 +19,7 @@
 #include <vector>
 
 #include "../../include/ap26.h"
-#include "ap26_kernels.cuh"
+#include "ap26_class.cuh"
 #include "ap26_hostcore.h"
 
 namespace ap26 {
@@ -165,6 +165,13 @@ __global__ void chunk_begin_kernel(DevState *st, int ring) {
   st->chain_next[ring] = 0;
 }
 
+// The same for a class-sieve launch over units [begin, ...) of the run.
+__global__ void class_begin_kernel(DevState *st, int ring, unsigned long long begin) {
+  st->tile_next = begin;
+  st->cand_count[ring] = 0;
+  st->chain_next[ring] = 0;
+}
+
 __global__ void chunk_end_kernel(DevState *st, long long cand_cap, int ring) {
   unsigned long long c = st->cand_count[ring];
   st->cand_total += c;
@@ -251,8 +258,60 @@ __global__ void chain_explicit_kernel(const KJob *job, const int64_t *n, long lo
   }
 }
 
+// Fills the constant tables of the current device (synchronous).
+static cudaError_t upload_constants() {
+  uint16_t trip[NUM_TRIPLES];
+  if (ap26h_triples(trip) != NUM_TRIPLES) return cudaErrorUnknown;
+  PrimeParam params[NPRIMES], single[NSINGLE];
+  for (int g = 0; g < NPRIMES; g++) params[g] = make_param(g);
+  for (int i = 0; i < NSINGLE; i++)
+    single[i] = make_param_p(PRIMES[FIRST_SINGLE + i], single_off(i));
+  ResParam res[NDENSE + 1];
+  int str[NDENSE], slot[NSLOTS];
+  uint16_t task[NTASKS];
+  int nt = 0;
+  for (int k = 0; k <= NDENSE; k++) {
+    const PrimeParam p = make_param_p(k < NDENSE ? DENSE_M[k] : CLASSES, 0);
+    res[k] = ResParam{p.p, p.A, p.B, p.C, p.k, p.M};
+    if (k == NDENSE) break;
+    str[k] = dense_str_off(k);
+    for (int b = 0; b < (DENSE_M[k] + 31) / 32; b++)
+      for (int w = 0; w < 4; w++) task[nt++] = (uint16_t)(k | b << 5 | w << 8);
+  }
+  for (int i = 0; i < NSLOTS; i++) slot[i] = slot_base(i);
+  cudaError_t e;
+  if ((e = cudaMemcpyToSymbol(c_triples, trip, sizeof(trip))) != cudaSuccess) return e;
+  if ((e = cudaMemcpyToSymbol(c_params, params, sizeof(params))) != cudaSuccess) return e;
+  if ((e = cudaMemcpyToSymbol(c_single, single, sizeof(single))) != cudaSuccess) return e;
+  if ((e = cudaMemcpyToSymbol(c_res, res, sizeof(res))) != cudaSuccess) return e;
+  if ((e = cudaMemcpyToSymbol(c_task, task, sizeof(task))) != cudaSuccess) return e;
+  if ((e = cudaMemcpyToSymbol(c_dense_str, str, sizeof(str))) != cudaSuccess) return e;
+  return cudaMemcpyToSymbol(c_slot_base, slot, sizeof(slot));
+}
+
 // Argument blocks are only built through these, so no field can be left
 // value-initialised (a null counter pointer would fault on the device).
+static ClassArgs class_args(const KJob *jobs, int job, const ClassPlan *plan,
+                            const uint32_t *tables, DevState *st, unsigned long long unit_base,
+                            unsigned long long unit_end, Cand *cand, long long cand_cap,
+                            unsigned long long *cand_count, unsigned long long *job_counts,
+                            int count_only) {
+  ClassArgs a;
+  a.jobs = jobs;
+  a.job = job;
+  a.plan = plan;
+  a.tables = tables;
+  a.st = st;
+  a.unit_end = unit_end;
+  a.unit_base = unit_base;
+  a.cand = cand;
+  a.cand_cap = cand_cap;
+  a.cand_count = cand_count;
+  a.job_counts = job_counts;
+  a.count_only = count_only;
+  return a;
+}
+
 static SieveArgs sieve_args(const KJob *jobs, int njobs, const uint32_t *tables, DevState *st,
                             Cand *cand, long long cand_cap, unsigned long long *job_counts,
                             int count_only, unsigned long long *cand_count) {
@@ -422,6 +481,8 @@ struct JobSet {
   int njobs = 0;
   int chunk_tiles = 0;
   bool count_only = false;
+  bool by_class = false;              // whole K-jobs: the class sieve, else the window sieve
+  int chunk_units = 0;                // class sieve: units per launch
   unsigned long long nchunks = 0, nprof = 0;
   int launches = 0;
 };
@@ -472,6 +533,7 @@ struct ap26_ctx {
   JobSet main;                                 // every synchronous entry point
   Cand *d_cand[2] = {nullptr, nullptr};        // two candidate rings (overlapped form)
   long long cand_cap = 0;
+  ClassPlan *d_plan = nullptr;                 // class sieve: the K-job being sieved
   // graphs
   std::vector<GraphEntry> graphs;
   unsigned long long graph_clock = 0;
@@ -695,13 +757,10 @@ extern "C" int ap26_create(int device, const ap26_opts *opts, ap26_ctx **out) {
       CKC(cudaEventCreateWithFlags(&ctx->chain_done[r], cudaEventDisableTiming));
     }
     // constant tables
-    uint16_t trip[NUM_TRIPLES];
-    int nt = ap26h_triples(trip);
-    if (nt != NUM_TRIPLES) { rc = AP26_E_ARG; goto fail; }
-    CKC(cudaMemcpyToSymbol(c_triples, trip, sizeof(trip)));
-    PrimeParam params[NPRIMES];
-    for (int g = 0; g < NPRIMES; g++) params[g] = make_param(g);
-    CKC(cudaMemcpyToSymbol(c_params, params, sizeof(params)));
+    CKC(upload_constants());
+    CKC(cudaFuncSetAttribute(class_sieve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             CLASS_SMEM));
+    CKC(cudaMalloc(&ctx->d_plan, sizeof(ClassPlan)));
     // the set-up kernels sort each K's lattice order in 64 KB of shared memory
     CKC(cudaFuncSetAttribute(setup_jobs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)ORDER_SMEM));
@@ -749,6 +808,7 @@ extern "C" void ap26_destroy(ap26_ctx *ctx) {
   }
   cudaFree(ctx->d_units);
   cudaFree(ctx->d_pool);
+  cudaFree(ctx->d_plan);
   cudaFree(ctx->d_cand[0]); cudaFree(ctx->d_cand[1]);
   for (int r = 0; r < 2; r++) {
     if (ctx->sieve_done[r]) cudaEventDestroy(ctx->sieve_done[r]);
@@ -851,6 +911,16 @@ static int ensure_prof_events(ap26_ctx *ctx, unsigned long long n) {
   return AP26_OK;
 }
 
+// Class-sieve units per launch for chunks of chunk_tiles tiles of tile_n53
+// starts (at least one unit), made equal over a K's launches.
+static int class_chunk_units(int chunk_tiles, int64_t tile_n53) {
+  const int64_t most = std::max<int64_t>(
+      1, std::min<int64_t>(UNITS_PER_K, (int64_t)chunk_tiles * tile_n53 * UNITS_PER_K / N53_PER_K));
+  const int64_t n = (UNITS_PER_K + most - 1) / most;
+  return (int)((UNITS_PER_K + n - 1) / n);
+}
+static int class_chunks(int chunk_units) { return (UNITS_PER_K + chunk_units - 1) / chunk_units; }
+
 // The whole run of S.h_jobs[0..njobs): H2D of the jobs and the run state,
 // set-up, per chunk of chunk_tiles tiles chunk_begin -> sieve -> chain ->
 // chunk_end (the chain walk of chunk c on the second stream while chunk c+1
@@ -887,9 +957,28 @@ static cudaError_t emit_run(ap26_ctx *ctx, JobSet &S, const uint32_t *tables, in
     const int r = two_streams ? (int)(c & 1) : 0;
     // ring r is free once the chain walk of chunk c-2 has read it
     if (two_streams && c >= 2) EM(cudaStreamWaitEvent(s, ctx->chain_done[r], 0));
-    chunk_begin_kernel<<<1, 1, 0, s>>>(S.d_st, r);
-    if (c < S.nprof) EM(cudaEventRecordWithFlags(ctx->prof_events[2 * c], s, flag));
-    V.kernel<<<ctx->sieve_blocks, V.WARPS * 32, V.smem(), s>>>(sa[r]);
+    if (S.by_class) {
+      const int per_job = class_chunks(S.chunk_units), j = (int)(c / per_job);
+      const unsigned long long base = (unsigned long long)j * UNITS_PER_K,
+                               begin = base + (c % per_job) * S.chunk_units,
+                               end = std::min(begin + S.chunk_units, base + UNITS_PER_K);
+      if (begin == base) {   // the job's plan, over the previous job's
+        EM(cudaMemsetAsync(ctx->d_plan->vfill, 0, sizeof(ctx->d_plan->vfill), s));
+        class_plan_count_kernel<<<ctx->num_sms * 4, 256, 0, s>>>(S.d_jobs + j, ctx->d_plan);
+        class_plan_scan_kernel<<<1, 1024, 0, s>>>(ctx->d_plan);
+        class_plan_scatter_kernel<<<ctx->num_sms * 8, 256, 0, s>>>(S.d_jobs + j, ctx->d_plan);
+      }
+      class_begin_kernel<<<1, 1, 0, s>>>(S.d_st, r, begin);
+      if (c < S.nprof) EM(cudaEventRecordWithFlags(ctx->prof_events[2 * c], s, flag));
+      class_sieve_kernel<<<ctx->num_sms, CLASS_WARPS * 32, CLASS_SMEM, s>>>(
+          class_args(S.d_jobs, j, ctx->d_plan, tables, S.d_st, base, end, ctx->d_cand[r],
+                     ctx->cand_cap, &S.d_st->cand_count[r], S.d_job_counts,
+                     S.count_only ? 1 : 0));
+    } else {
+      chunk_begin_kernel<<<1, 1, 0, s>>>(S.d_st, r);
+      if (c < S.nprof) EM(cudaEventRecordWithFlags(ctx->prof_events[2 * c], s, flag));
+      V.kernel<<<ctx->sieve_blocks, V.WARPS * 32, V.smem(), s>>>(sa[r]);
+    }
     if (c < S.nprof) EM(cudaEventRecordWithFlags(ctx->prof_events[2 * c + 1], s, flag));
     if (two_streams) {
       chunk_end_kernel<<<1, 1, 0, s>>>(S.d_st, ctx->cand_cap, r);
@@ -974,20 +1063,27 @@ static int enqueue_jobs(ap26_ctx *ctx, JobSet &S, int njobs, bool count_only, bo
   S.h_st->total_tiles = tiles;
   S.njobs = njobs;
   S.count_only = count_only;
-  S.nchunks = tiles ? (tiles + chunk_tiles - 1) / chunk_tiles : 0;
+  S.by_class = njobs > 0;
+  for (int j = 0; j < njobs; j++)
+    if (S.h_jobs[j].q_begin != 0 || S.h_jobs[j].q_end != N53_PER_K) S.by_class = false;
+  S.chunk_units = class_chunk_units(chunk_tiles, tile_n53);
+  S.nchunks = S.by_class ? (unsigned long long)njobs * class_chunks(S.chunk_units)
+              : tiles    ? (tiles + chunk_tiles - 1) / chunk_tiles
+                         : 0;
   const bool two_streams = overlap && !count_only && S.nchunks > 1;
   // sieve launches timed with events: the first kProfChunks chunks at most
   constexpr unsigned long long kProfChunks = 4096;
   S.nprof = (ctx->opts.profile && &S == &ctx->main) ? std::min(S.nchunks, kProfChunks) : 0;
   if ((rc = ensure_prof_events(ctx, S.nprof)) != AP26_OK) return rc;
-  S.launches = 1 + (int)S.nchunks * (count_only ? 3 : 4) + (count_only ? 0 : 1);
+  S.launches = 1 + (int)S.nchunks * (count_only ? 3 : 4) + (count_only ? 0 : 1) +
+               (S.by_class ? 3 * njobs : 0);
   CK(cudaEventRecord(S.t0, ctx->stream));
   bool launched = false;
   if (ctx->opts.use_graphs > 0) {
     const long long key[7] = {(long long)(uintptr_t)&S, ctx->variant, njobs,
                               (long long)S.nchunks, chunk_tiles,
                               (count_only ? 1 : 0) | (two_streams ? 2 : 0) | (build_tables ? 4 : 0) |
-                                  ((long long)S.nprof << 3),
+                                  (S.by_class ? 8 : 0) | ((long long)S.nprof << 4),
                               (long long)(uintptr_t)tables};
     GraphEntry *hit = nullptr;
     for (auto &g : ctx->graphs)
@@ -1050,7 +1146,13 @@ static int collect_run(ap26_ctx *ctx, JobSet &S, cudaStream_t cs, ap26_stats *st
     stats->sieve_cells = n53 * J59 * WORDS;
     stats->sieve_launches = (int32_t)S.nchunks;
     if (S.nprof) {
-      if (S.nprof < S.nchunks) {
+      if (S.nprof < S.nchunks && S.by_class) {
+        const int per_job = class_chunks(S.chunk_units);
+        int64_t units = (int64_t)(S.nprof / per_job) * UNITS_PER_K;
+        units += std::min<int64_t>((int64_t)(S.nprof % per_job) * S.chunk_units, UNITS_PER_K);
+        stats->sieve_cells = (int64_t)((double)units / UNITS_PER_K * (double)N53_PER_K) * J59 * WORDS;
+        stats->sieve_launches = (int32_t)S.nprof;
+      } else if (S.nprof < S.nchunks) {
         // only the first nprof chunks were timed; all of them are full
         const int64_t tile_n53 = (int64_t)kVariants[ctx->variant].WARPS * 32;
         stats->sieve_cells = (int64_t)(S.nprof * (unsigned long long)S.chunk_tiles) *
@@ -2081,12 +2183,7 @@ static int noalloc_setup(int device, NoallocDevice **out) {
   if (!d.ready) {
     void *p = nullptr;
     if (cudaGetSymbolAddress(&p, g_noalloc_scratch) != cudaSuccess) return AP26_E_CUDA;
-    uint16_t trip[NUM_TRIPLES];
-    if (ap26h_triples(trip) != NUM_TRIPLES) return AP26_E_ARG;
-    PrimeParam params[NPRIMES];
-    for (int g = 0; g < NPRIMES; g++) params[g] = make_param(g);
-    if (cudaMemcpyToSymbol(c_triples, trip, sizeof(trip)) != cudaSuccess) return AP26_E_CUDA;
-    if (cudaMemcpyToSymbol(c_params, params, sizeof(params)) != cudaSuccess) return AP26_E_CUDA;
+    if (upload_constants() != cudaSuccess) return AP26_E_CUDA;
     if (cudaFuncSetAttribute(setup_jobs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)ORDER_SMEM) != cudaSuccess)
       return AP26_E_CUDA;

@@ -8,7 +8,10 @@
 //                       per-K sieve bitstrings (replaces clearok/setok/
 //                       setupokok/offset, src/opencl/kernels/*.cl)
 //   chunk_begin_kernel  resets per-chunk counters
-//   sieve_kernel        persistent, work-stealing over tiles of n53 starts;
+//   class_plan_*, class_sieve_kernel (ap26_class.cuh)
+//                       the sieve of a whole K, by residue classes
+//   sieve_kernel        the sieve of a part of a K's lattice: persistent,
+//                       work-stealing over tiles of n53 starts;
 //                       replaces setupn.cl + sieve.cl (the 1.1 GB n59 array
 //                       of the reference is never materialised: starts are
 //                       generated from a flat index)
