@@ -266,14 +266,15 @@ static cudaError_t upload_constants() {
   for (int g = 0; g < NPRIMES; g++) params[g] = make_param(g);
   for (int i = 0; i < NSINGLE; i++)
     single[i] = make_param_p(PRIMES[FIRST_SINGLE + i], single_off(i));
-  ResParam res[NDENSE + 1];
+  ResParam res[NDENSE + 2];
   int str[NDENSE], slot[NSLOTS];
   uint16_t task[NTASKS];
   int nt = 0;
-  for (int k = 0; k <= NDENSE; k++) {
-    const PrimeParam p = make_param_p(k < NDENSE ? DENSE_M[k] : CLASSES, 0);
+  for (int k = 0; k < NDENSE + 2; k++) {
+    const PrimeParam p =
+        make_param_p(k < NDENSE ? DENSE_M[k] : k == RES_CLASS ? CLASSES : SKIP, 0);
     res[k] = ResParam{p.p, p.A, p.B, p.C, p.k, p.M};
-    if (k == NDENSE) break;
+    if (k >= NDENSE) continue;
     str[k] = dense_str_off(k);
     for (int b = 0; b < (DENSE_M[k] + 31) / 32; b++)
       for (int w = 0; w < 4; w++) task[nt++] = (uint16_t)(k | b << 5 | w << 8);

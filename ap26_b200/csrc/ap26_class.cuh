@@ -20,27 +20,40 @@
 // bytes of shared memory for 32 candidates that already passed 61 and 67,
 // against 4.2 bytes and a funnel shift for 32 raw ones in the window sieve.
 //
+// 71 is not among them.  In a coordinate scaled by MOD * STEP^-1 it excludes
+// 24 consecutive residues (mod 71) of x + v + b + j, so the (b, j) are listed
+// in the order of their coordinate: the 128 bits of a quarter row then span
+// about 5.4 coordinates, and where x + v lies in one of about 19.6 (of 71) the
+// whole quarter is excluded.  With the v of a bucket sorted by coordinate, the
+// points a quarter is alive for are one (cyclic) range of the bucket, 72% of
+// it; each lane walks the range of its own quarter.  What is left of 71 is
+// tested with the tail products.
+//
 // The units' points are enumerated without a search: the v are sorted by
-// s(v) mod 4087 once per K, so for each x the class's v are one bucket of the
-// sorted order, about 108 consecutive records of precomputed residues.
+// s(v) mod 4087 and coordinate once per K, so for each x the class's v are one
+// bucket of the sorted order, about 108 consecutive records of residues.
 //
 // Why this split (one B200, K = 43241061, sieve time of the whole K): the
 // window sieve moves 17.5 shared-memory wavefronts per lattice value and takes
-// 331 ms; this one moves about 8 and takes 156 ms.  It is bound by shared
-// memory: 91% of the wavefront slots, two thirds of them the dense rows'.  Of
-// those 156 ms, measured by leaving parts out, building the rows takes 2.7,
-// reading them 98, the masks' queue and stage A 32, stages B to D 17, and the
-// ends of the five launches a K 5.  Sixteen warps with more registers took
-// 163 ms, twenty 159, 28 with fewer registers 164 (24: 156); 22 dense moduli,
-// which only fit with 20 warps, 156; four points a warp with a shuffle to
-// join the two moduli's halves 192; single bits instead of masks in the first
-// queue 188.
+// 331 ms.  Classes alone took 156 ms, with 71 skipped by quarters and the
+// masks queued in 64-bit halves 140 ms.  It is bound by shared memory and L1:
+// 91% of their wavefront slots (issue 66%), half of them the dense rows', 14%
+// the v records' (the four quarters read four parts of a bucket), the rest the
+// queues and the lookups of the tail, most of them in stage A.  In one launch
+// (135 ms) building the rows takes 3 ms, reading them 82, the masks' queue and
+// stage A 33, stages B to D 18.  Sixteen warps with more registers were slower
+// (143 ms), twenty about equal (136.5), 26 and 28 too (143); 22 dense moduli,
+// which only fit with 20 warps, 134.7; v records as one 256-bit load 140;
+// four points a warp with a shuffle to join the two moduli's halves, single
+// bits instead of masks in the first queue, and two or four products in stage
+// A (136.7, 136.1 against 135.3) were slower too.
 //
 // The class sieve takes every whole K.  A K that 61 or 67 divides has more
 // (b, j) per class (up to thirteen rows) and is still faster than by windows:
 // 266 against 389 ms for 61 | K, 388 against 463 for 61 * 67 | K, 583 against
-// 695 for 61 * 67 * 71 * 73 | K, the densest.  Parts of a K (sieve_range) stay
-// with the window sieve: a class's points are spread over the whole lattice.
+// 695 for 61 * 67 * 71 * 73 | K, the densest (with classes alone).  Parts of a
+// K (sieve_range) stay with the window sieve: a class's points are spread over
+// the whole lattice.
 //
 // Bits that survive the dense rows become single candidates, tested against
 // the other moduli (primes 7..23 included) in full batches of 32 lanes that
@@ -56,19 +69,22 @@ constexpr int CLASSES = PAIR1_P;               // 4087
 constexpr int ROW_BITS = 512;
 constexpr int ROWS_PER_CLASS = 4;              // units per class
 constexpr int UNITS_PER_K = CLASSES * ROWS_PER_CLASS;
+constexpr int SKIP = 71;                       // the prime whole quarters of a row skip by
+constexpr int NBINS = CLASSES * SKIP;          // v buckets
 constexpr int MAX_WRAPS = 2;
 constexpr int J_COUNT = 64 * WORDS + MAX_WRAPS;   // 642 values of j
 
-// Dense moduli: 7 * 11 and the primes 71..163, in pairs (slots).  Four lanes
+// Dense moduli: 7 * 11 and the primes 73..167, in pairs (slots).  Four lanes
 // hold one point's row, 128 bits each.  A slot's rows alternate in shared
 // memory, 64 bytes each, and of the two points in one 8-lane phase of a
 // 128-bit load the first reads its row of the slot's first modulus and the
 // second its row of the other, then the other way round: the two rows lie in
-// the two halves of the 32 banks, so every load is conflict-free whatever the
-// rows.
+// the two halves of the 32 banks, and the four lanes in different 16-byte
+// columns of a half, so every load is conflict-free whatever the rows, also
+// where the four lanes' points differ.
 constexpr int NDENSE = 20;
-constexpr int DENSE_M[NDENSE] = {71,  73,  77,  79,  83,  89,  97,  101, 103, 107, 109,
-                                 113, 127, 131, 137, 139, 149, 151, 157, 163};
+constexpr int DENSE_M[NDENSE] = {73,  77,  79,  83,  89,  97,  101, 103, 107, 109,
+                                 113, 127, 131, 137, 139, 149, 151, 157, 163, 167};
 constexpr int NSLOTS = NDENSE / 2;
 static_assert(NSLOTS == 10, "records hold 16 + 4 residue bytes");
 static_assert(DENSE_M[NDENSE - 1] < 256, "residues fit a byte");
@@ -100,13 +116,13 @@ constexpr int build_tasks() {
 }
 constexpr int NTASKS = build_tasks();
 
-// Tail moduli: products of two or three primes, one lookup each, then the
-// remaining primes singly.
+// Tail moduli: products of two or three primes, one lookup each (about 3.4
+// wavefronts at 32 random bits), then the remaining primes singly.
 struct TailMod { int m, p, q, r; };
 constexpr int NTAIL = 6;
 constexpr TailMod TAIL_M[NTAIL] = {
-    {167 * 173, 167, 173, 1}, {179 * 181, 179, 181, 1}, {191 * 193, 191, 193, 1},
-    {13 * 17 * 19, 13, 17, 19}, {197 * 199, 197, 199, 1}, {23 * 211, 23, 211, 1}};
+    {173 * 179, 173, 179, 1}, {181 * 191, 181, 191, 1}, {193 * 197, 193, 197, 1},
+    {13 * 17 * 23, 13, 17, 23}, {71 * 199, 71, 199, 1}, {19 * 211, 19, 211, 1}};
 constexpr int STAGE_A = 3;                     // tail moduli of stage A; B takes the rest
 constexpr int FIRST_SINGLE = 30;               // PRIMES[30] = 223
 static_assert(PRIMES[FIRST_SINGLE] == 223, "single tail primes follow the products");
@@ -149,9 +165,10 @@ constexpr bool tail_mods_ok() {
 }
 static_assert(tail_mods_ok(), "tail moduli stay in the exact range of the reduction");
 
-// Residues of x, v and b: dense moduli, then the class modulus.
+// Residues of x, v and b: dense moduli, the class modulus, 71.
 struct ResParam { int p, A, B, C, k; uint32_t M; };
-__constant__ ResParam c_res[NDENSE + 1];
+constexpr int RES_CLASS = NDENSE, RES_SKIP = NDENSE + 1;
+__constant__ ResParam c_res[NDENSE + 2];
 __constant__ PrimeParam c_single[NSINGLE];     // off: word of the tail strings
 __constant__ uint16_t c_task[NTASKS];          // modulus | row block << 5 | 128-bit word << 8
 __constant__ int c_dense_str[NDENSE];          // word offset of a modulus's string
@@ -160,16 +177,22 @@ __constant__ int c_slot_base[NSLOTS];
 // One K's enumeration tables and bitstrings (device memory, one per context;
 // K-jobs are sieved one after the other).
 struct ClassPlan {
-  uint4 va[NV];                   // residue bytes of v: dense moduli 0..15
-  uint32_t vb[NV];                // ... 16..19
-  uint64_t vc[NV];                // v
+  // v records in bucket order; the padding is only read, for lanes past a
+  // bucket's end
+  uint4 va[NV + 16];              // residue bytes of v: dense moduli 0..15
+  uint32_t vb[NV + 16];           // ... 16..19
+  uint64_t vc[NV + 16];           // v
   alignas(16) uint32_t xu[NUM_TRIPLES][12];   // a slot's two residues * 128, 16 bits each
   int64_t xval[NUM_TRIPLES];
   int64_t bval[NB];
   int32_t xcls[NUM_TRIPLES];      // s(x) mod 4087
+  int32_t xskip[NUM_TRIPLES];     // skip coordinate of x
   int32_t bres[NDENSE + 1][NB];   // s(b)
-  uint32_t vstart[CLASSES + 1];   // sorted v: bucket starts
-  uint32_t vfill[CLASSES];
+  int32_t bskip[NB];              // s(b) - 2 + SHIFT mod 71
+  uint32_t vstart[NBINS + 1];     // v buckets: (s(v) mod 4087) * 71 + skip coordinate
+  uint32_t vfill[NBINS];
+  int32_t skip_mul, skip_inv;     // skip coordinate of residue r mod 71: r * mul; its inverse
+  int32_t skip_bad, skip_len;     // 71 excludes coordinates [bad, bad + len) mod 71
   uint32_t dense_str[DENSE_STR_WORDS];
   uint32_t tail_str[TAIL_WORDS];
 };
@@ -255,11 +278,28 @@ __device__ __forceinline__ int64_t v_value(const KJob &J, int i) {
                                    (uint64_t)j59 * (uint64_t)J.S59));
 }
 
-// Per K, first step: class sizes of v (vfill zeroed before), the x and b
+// 71's coordinate: OK_71 of the residue r = s(x) + s(v) + s(b) + j - 2 of a
+// candidate is that tt = (r + SHIFT) * MOD * STEP^-1 is neither 0 nor 48..70
+// (mod 71), 24 consecutive values; where 71 divides K, that r + SHIFT is not 0.
+struct SkipCoord { int mul, bad, len; };
+__device__ __forceinline__ SkipCoord skip_coord(int K) {
+  const int st = (int)(((int64_t)(K % SKIP) * (int)(PRIM23 % SKIP)) % SKIP);
+  if (!st) return SkipCoord{1, 0, 1};
+  int inv = 1;
+  while (inv * st % SKIP != 1) inv++;
+  return SkipCoord{(int)(MOD % SKIP) * inv % SKIP, SKIP - 23, 24};
+}
+
+__device__ __forceinline__ int v_bucket(int64_t v, const SkipCoord &c) {
+  return res_mod(v, c_res[RES_CLASS]) * SKIP + res_mod(v, c_res[RES_SKIP]) * c.mul % SKIP;
+}
+
+// Per K, first step: bucket sizes of v (vfill zeroed before), the x and b
 // tables and the bitstrings.  Grid-stride over all of them.
 __global__ void class_plan_count_kernel(const KJob *job, ClassPlan *P) {
   const KJob &J = *job;
   const int K = J.K, shift = J.shift;
+  const SkipCoord sc = skip_coord(K);
   const int stride = gridDim.x * blockDim.x;
   // strings first: their threads have the longest work
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < DENSE_STR_WORDS + TAIL_WORDS;
@@ -284,14 +324,15 @@ __global__ void class_plan_count_kernel(const KJob *job, ClassPlan *P) {
     }
   }
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < NV; i += stride)
-    atomicAdd(&P->vfill[res_mod(v_value(J, i), c_res[NDENSE])], 1u);
+    atomicAdd(&P->vfill[v_bucket(v_value(J, i), sc)], 1u);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < NUM_TRIPLES; i += stride) {
     const uint32_t tr = c_triples[i];
     const int i31 = tr & 31, i37 = (tr >> 5) & 31, i41 = (tr >> 10) & 31;
     const int64_t x = mod_MOD((uint64_t)J.n0 + (uint64_t)i31 * (uint64_t)J.S31 +
                               (uint64_t)i37 * (uint64_t)J.S37 + (uint64_t)i41 * (uint64_t)J.S41);
     P->xval[i] = x;
-    P->xcls[i] = res_mod(x, c_res[NDENSE]);
+    P->xcls[i] = res_mod(x, c_res[RES_CLASS]);
+    P->xskip[i] = res_mod(x, c_res[RES_SKIP]) * sc.mul % SKIP;
     for (int k = 0; k < NSLOTS; k++)
       P->xu[i][k] = (uint32_t)res_mod(x, c_res[2 * k]) * ROW_STRIDE |
                     (uint32_t)res_mod(x, c_res[2 * k + 1]) * ROW_STRIDE << 16;
@@ -301,19 +342,28 @@ __global__ void class_plan_count_kernel(const KJob *job, ClassPlan *P) {
     const int64_t x = mod_MOD((uint64_t)(b >> 2) * (uint64_t)S3 + (uint64_t)(b & 3) * (uint64_t)S5);
     P->bval[b] = x;
     for (int k = 0; k <= NDENSE; k++) P->bres[k][b] = res_mod(x, c_res[k]);
+    P->bskip[b] = (res_mod(x, c_res[RES_SKIP]) + shift + SKIP - MAX_WRAPS) % SKIP;
+    if (b == 0) {
+      int inv = 1;
+      while (inv * sc.mul % SKIP != 1) inv++;
+      P->skip_mul = sc.mul;
+      P->skip_inv = inv;
+      P->skip_bad = sc.bad;
+      P->skip_len = sc.len;
+    }
   }
 }
 
-// Second step (one block of 1024): class sizes to bucket starts.
+// Second step (one block of 1024): bucket sizes to bucket starts, 284
+// consecutive buckets a thread.
+constexpr int SCAN_EACH = 284;
+static_assert(SCAN_EACH % 4 == 0 && 1024 * SCAN_EACH >= NBINS, "one pass of the scan");
 __global__ void __launch_bounds__(1024) class_plan_scan_kernel(ClassPlan *P) {
   __shared__ uint32_t sums[32];
-  const int t = threadIdx.x, lane = t & 31;
-  uint32_t c[4], tot = 0;
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    c[i] = 4 * t + i < CLASSES ? P->vfill[4 * t + i] : 0u;
-    tot += c[i];
-  }
+  const int t = threadIdx.x, lane = t & 31, b0 = t * SCAN_EACH, b1 = min(b0 + SCAN_EACH, NBINS);
+  uint32_t tot = 0;
+#pragma unroll 8
+  for (int i = b0; i < b1; i++) tot += P->vfill[i];
   uint32_t x = tot;
   for (int o = 1; o < 32; o <<= 1) {
     const uint32_t y = __shfl_up_sync(FULL, x, o);
@@ -331,23 +381,23 @@ __global__ void __launch_bounds__(1024) class_plan_scan_kernel(ClassPlan *P) {
   }
   __syncthreads();
   uint32_t at = x - tot + (t >= 32 ? sums[(t >> 5) - 1] : 0u);
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    if (4 * t + i < CLASSES) {
-      P->vstart[4 * t + i] = at;
-      P->vfill[4 * t + i] = at;
-    }
-    at += c[i];
+#pragma unroll 8
+  for (int i = b0; i < b1; i++) {
+    const uint32_t c = P->vfill[i];
+    P->vstart[i] = at;
+    P->vfill[i] = at;
+    at += c;
   }
-  if (t == 1023) P->vstart[CLASSES] = at;
+  if (t == 1023) P->vstart[NBINS] = at;
 }
 
 // Third step: the v records in bucket order (any order inside a bucket).
 __global__ void class_plan_scatter_kernel(const KJob *job, ClassPlan *P) {
   const KJob &J = *job;
+  const SkipCoord sc = skip_coord(J.K);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < NV; i += gridDim.x * blockDim.x) {
     const int64_t v = v_value(J, i);
-    const uint32_t at = atomicAdd(&P->vfill[res_mod(v, c_res[NDENSE])], 1u);
+    const uint32_t at = atomicAdd(&P->vfill[v_bucket(v, sc)], 1u);
     uint32_t w[(NDENSE + 3) / 4] = {};
 #pragma unroll
     for (int k = 0; k < NDENSE; k++) w[k / 4] |= (uint32_t)res_mod(v, c_res[k]) << (8 * (k & 3));
@@ -374,12 +424,12 @@ struct ClassArgs {
 };
 
 constexpr int CLASS_WARPS = 24;
-// Per-warp stacks in shared memory: masks waiting for stage A (16 + 8 bytes),
-// candidates for B, C and D (8 bytes).  A stage takes 32 entries; it runs when
+// Per-warp stacks in shared memory: 64-bit masks with their x + v waiting for
+// stage A (16 bytes), candidates for B, C and D (8 bytes).  A stage takes 32 entries; it runs when
 // the entries about to be pushed would not fit, so its batches are full but
 // for the densest K.
-constexpr int QCAP = 48;
-constexpr int WARP_BYTES = QCAP * (24 + 3 * 8);
+constexpr int ACAP = 64, QCAP = 46;
+constexpr int WARP_BYTES = ACAP * 16 + QCAP * 3 * 8;
 constexpr int CLASS_SMEM = DENSE_BYTES + CLASS_WARPS * WARP_BYTES + 8 * ROW_BITS + 4 * TAIL_WORDS;
 static_assert(CLASS_SMEM <= 226 * 1024, "class sieve shared memory");
 
@@ -455,8 +505,7 @@ struct ClassShared {
 };
 
 struct ClassWarp {               // one warp's stacks and counts
-  uint4 *mask;                   // stage A: masks, their x + v and quarter << 52
-  uint2 *qa;
+  uint4 *qa;                     // 64 bits of a mask, x + v and which 64 bits << 52
   uint2 *qb, *qc, *qd;
   int na, nb, nc, nd;
   unsigned kept;
@@ -573,34 +622,21 @@ __device__ __forceinline__ void stage_a(const ClassArgs &A, const ClassShared &C
   const int n = min(W.na, 32);
   W.na -= n;
   bool alive = lane < n;
-  uint4 m = make_uint4(0, 0, 0, 0);
-  uint2 it = make_uint2(0, 0);
-  if (alive) {
-    m = W.mask[W.na + lane];
-    it = W.qa[W.na + lane];
-  }
+  uint4 it = make_uint4(0, 0, 0, 0);
+  if (alive) it = W.qa[W.na + lane];
   __syncwarp();
-  // the mask's first bit: half h, word z of the half
-  const bool h = (m.x | m.y) == 0u;
-  const uint32_t lo = h ? m.z : m.x, hi = h ? m.w : m.y;
-  const bool z = lo == 0u;
-  const uint32_t w = z ? hi : lo;
-  const uint32_t e = (it.y >> 20) * 128 + (h ? 64 : 0) + (z ? 32 : 0) + (uint32_t)(__ffs(w) - 1);
-  const uint32_t c = w & (w - 1);
-  m.x = !h && !z ? c : m.x;
-  m.y = !h && z ? c : m.y;
-  m.z = h && !z ? c : m.z;
-  m.w = h && z ? c : m.w;
-  const bool more = (m.x | m.y | m.z | m.w) != 0u;
+  // the mask's first bit
+  const bool z = it.x == 0u;
+  const uint32_t w = z ? it.y : it.x, c = w & (w - 1);
+  const uint32_t e = (it.w >> 20) * 64 + (z ? 32 : 0) + (uint32_t)(__ffs(w) - 1);
+  it.x = z ? 0u : c;
+  it.y = z ? c : it.y;
+  const bool more = (it.x | it.y) != 0u;
   const unsigned mb = __ballot_sync(FULL, more);
-  if (more) {
-    const int at = W.na + __popc(mb & ((1u << lane) - 1u));
-    W.mask[at] = m;
-    W.qa[at] = it;
-  }
+  if (more) W.qa[W.na + __popc(mb & ((1u << lane) - 1u))] = it;
   W.na += __popc(mb);
   const uint64_t v = C.ev[e & (ROW_BITS - 1)];
-  const uint64_t t = ((uint64_t)it.x | (uint64_t)(it.y & 0xfffffu) << 32) + v;
+  const uint64_t t = ((uint64_t)it.z | (uint64_t)(it.w & 0xfffffu) << 32) + v;
   const uint2 cd = make_uint2((uint32_t)t, (uint32_t)(t >> 32) & 0x0fffffffu);   // b drops out
   alive = alive && tail_test<0>(C.ts, cd.x, cd.y, std::make_integer_sequence<int, STAGE_A>{});
   const unsigned bal = __ballot_sync(FULL, alive);
@@ -621,20 +657,20 @@ __global__ void __launch_bounds__(CLASS_WARPS * 32, 1) class_sieve_kernel(ClassA
   extern __shared__ __align__(16) unsigned char smem_raw[];
   unsigned char *rows = smem_raw;
   uint4 *masks = reinterpret_cast<uint4 *>(rows + DENSE_BYTES);
-  uint2 *queues = reinterpret_cast<uint2 *>(masks + QCAP * CLASS_WARPS);
-  uint64_t *ev = reinterpret_cast<uint64_t *>(queues + 4 * QCAP * CLASS_WARPS);
+  uint2 *queues = reinterpret_cast<uint2 *>(masks + ACAP * CLASS_WARPS);
+  uint64_t *ev = reinterpret_cast<uint64_t *>(queues + 3 * QCAP * CLASS_WARPS);
   uint32_t *ts = reinterpret_cast<uint32_t *>(ev + ROW_BITS);
   __shared__ unsigned long long s_unit;
-  __shared__ int s_cnt[NB], s_x;
+  __shared__ int s_cnt[CLASS_WARPS], s_x;
+  __shared__ int s_o0[4], s_o1[4];      // first and last skip coordinate of the row's quarters
   __shared__ unsigned long long s_kept[CLASS_WARPS], s_late[CLASS_WARPS];
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const ClassPlan &P = *A.plan;
   const uint32_t *table = A.tables + (size_t)A.jobs[A.job].table * JOB_TABLE_WORDS;
   ClassWarp W;
-  W.mask = masks + warp * QCAP;
-  W.qa = queues + warp * 4 * QCAP;
-  W.qb = W.qa + QCAP;
+  W.qa = masks + warp * ACAP;
+  W.qb = queues + warp * 3 * QCAP;
   W.qc = W.qb + QCAP;
   W.qd = W.qc + QCAP;
   W.na = W.nb = W.nc = W.nd = 0;
@@ -662,44 +698,52 @@ __global__ void __launch_bounds__(CLASS_WARPS * 32, 1) class_sieve_kernel(ClassA
     // row h of the class, then h + 4, ... while the class has more (b, j)
     // than four rows hold
     for (int h = local % ROWS_PER_CLASS;; h += ROWS_PER_CLASS) {
-      // the (b, j) that pass 61 and 67: warp b lists b's
-      uint32_t word = 0;
-      int before = 0, cnt = 0;
-      if (warp < NB) {
-        int pos = cls + P.bres[NDENSE][warp] - MAX_WRAPS;
-        pos += pos < 0 ? CLASSES : 0;
-        pos -= pos >= CLASSES ? CLASSES : 0;
-        if (lane < 21) {
-          const int at = pos + 32 * lane;
-          word = __funnelshift_r(table[at >> 5], table[(at >> 5) + 1], at & 31);
-          if (lane == 20) word &= (1u << (J_COUNT - 640)) - 1u;
+      // the (b, j) that pass 61 and 67, in the order of their coordinate
+      // mod 71: LIST slots (coordinate, b, one of its j), EACH a thread
+      constexpr int JS = (J_COUNT + SKIP - 1) / SKIP;       // j of one coordinate, 10
+      constexpr int LIST = SKIP * NB * JS;
+      constexpr int EACH = (LIST + CLASS_WARPS * 32 - 1) / (CLASS_WARPS * 32);
+      uint32_t mine = 0;
+#pragma unroll
+      for (int u = 0; u < EACH; u++) {
+        const int slot = (int)threadIdx.x * EACH + u;
+        if (slot < LIST) {
+          const int o = slot / (NB * JS), b = slot / JS % NB;
+          const int j = (o * P.skip_inv + SKIP - P.bskip[b]) % SKIP + slot % JS * SKIP;
+          int at = cls + P.bres[RES_CLASS][b] + j - MAX_WRAPS;
+          at += at < 0 ? CLASSES : 0;
+          at -= at >= CLASSES ? CLASSES : 0;
+          at -= at >= CLASSES ? CLASSES : 0;
+          if (j < J_COUNT && (table[at >> 5] >> (at & 31) & 1u)) mine |= 1u << u;
         }
-        cnt = __popc(word);
-        int x = cnt;
-        for (int o = 1; o < 32; o <<= 1) {
-          const int y = __shfl_up_sync(FULL, x, o);
-          if (lane >= o) x += y;
-        }
-        before = x - cnt;
-        if (lane == 31) s_cnt[warp] = x;
       }
+      int before = __popc(mine);
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(FULL, before, o);
+        if (lane >= o) before += y;
+      }
+      if (lane == 31) s_cnt[warp] = before;
+      before -= __popc(mine);
+      if (threadIdx.x < 4) s_o0[threadIdx.x] = -1;
+      if (threadIdx.x == 0) s_x = 0;
       __syncthreads();
       int total = 0;
-      for (int b = 0; b < NB; b++) total += s_cnt[b];
+      for (int w = 0; w < CLASS_WARPS; w++) {
+        before += w < warp ? s_cnt[w] : 0;
+        total += s_cnt[w];
+      }
       const int e0 = h * ROW_BITS;
       if (e0 >= total) break;                  // uniform over the CTA
       const int ne = min(ROW_BITS, total - e0);
-      if (warp < NB) {
-        for (int b = 0; b < warp; b++) before += s_cnt[b];
-        const uint64_t bv = (uint64_t)P.bval[warp] | (uint64_t)warp << (J_BIT + 10);
-        while (word) {
-          const int j = lane * 32 + __ffs(word) - 1;
-          word &= word - 1;
-          const int e = before++ - e0;
-          if (e >= 0 && e < ROW_BITS) ev[e] = bv | (uint64_t)j << J_BIT;
-        }
+      for (; mine; mine &= mine - 1) {
+        const int slot = (int)threadIdx.x * EACH + __ffs(mine) - 1, e = before++ - e0;
+        if (e < 0 || e >= ROW_BITS) continue;
+        const int o = slot / (NB * JS), b = slot / JS % NB;
+        const int j = (o * P.skip_inv + SKIP - P.bskip[b]) % SKIP + slot % JS * SKIP;
+        ev[e] = (uint64_t)P.bval[b] | (uint64_t)j << J_BIT | (uint64_t)b << (J_BIT + 10);
+        if ((e & 127) == 0) s_o0[e >> 7] = o;
+        if ((e & 127) == 127 || e == ne - 1) s_o1[e >> 7] = o;
       }
-      if (threadIdx.x == 0) s_x = 0;
       __syncthreads();
 
       // rows of every dense modulus: 32 rows x 128 bits a task
@@ -728,6 +772,15 @@ __global__ void __launch_bounds__(CLASS_WARPS * 32, 1) class_sieve_kernel(ClassA
       }
       __syncthreads();
 
+      // A quarter's bits are all excluded by 71 where x + v lies in a range of
+      // the skip coordinate; this lane's points are the others, alive_n
+      // coordinates from alive_0 on.
+      int alive_0, alive_n;
+      {
+        const int o = s_o0[q], dead = max(0, P.skip_len - (s_o1[q] - o));
+        alive_n = o < 0 ? 0 : SKIP - dead;
+        alive_0 = ((P.skip_bad - o + dead) % SKIP + SKIP) % SKIP;
+      }
       // every point of the class: warps take the x in turn
       for (;;) {
         int xi = 0;
@@ -736,8 +789,18 @@ __global__ void __launch_bounds__(CLASS_WARPS * 32, 1) class_sieve_kernel(ClassA
         if (xi >= NUM_TRIPLES) break;
         int r = cls - P.xcls[xi];
         r += r < 0 ? CLASSES : 0;
-        const int p0 = (int)P.vstart[r], p1 = (int)P.vstart[r + 1];
-        if (p0 >= p1) continue;
+        // the class's v of this x are bucket positions p0..p1-1, sorted by skip
+        // coordinate; this lane's are n of them, cyclically from `at` on
+        const uint32_t *start = P.vstart + r * SKIP;
+        const int p0 = (int)start[0], p1 = (int)start[SKIP];
+        int t0 = alive_0 - P.xskip[xi];
+        t0 += t0 < 0 ? SKIP : 0;
+        const int t1 = t0 + alive_n;
+        int at = (int)start[t0];
+        int n = (int)start[t1 > SKIP ? t1 - SKIP : t1] - at + (t1 > SKIP ? p1 - p0 : 0);
+        const int most = __reduce_max_sync(FULL, n);
+        if (!most) continue;
+        n -= p;                                   // this lane's points left
         uint32_t u[NSLOTS];
         {
           const uint4 u0 = *reinterpret_cast<const uint4 *>(&P.xu[xi][0]);
@@ -748,36 +811,41 @@ __global__ void __launch_bounds__(CLASS_WARPS * 32, 1) class_sieve_kernel(ClassA
 #pragma unroll
           for (int k = 0; k < NSLOTS; k++) u[k] = w[k] + lane_pack;
         }
-        const uint64_t xv = (uint64_t)P.xval[xi] + ((uint64_t)q << 52);
-        int pt = min(p0 + p, p1 - 1);
-        uint4 va = P.va[pt];
-        uint32_t vb = P.vb[pt];
-        uint64_t vc = P.vc[pt];
-        for (int base = p0; base < p1; base += 8) {
+        const uint64_t xv = (uint64_t)P.xval[xi] + ((uint64_t)q << 53);
+        at += p;
+        at -= at >= p1 ? p1 - p0 : 0;
+        uint4 va = P.va[at];
+        uint32_t vb = P.vb[at];
+        uint64_t vc = P.vc[at];
+        for (int i = 0; i < most; i += 8, n -= 8) {
           uint4 m = make_uint4(FULL, FULL, FULL, FULL);
           const uint4 va0 = va;
           const uint32_t vb0 = vb;
           const uint64_t vc0 = vc;
-          pt = min(base + 8 + p, p1 - 1);        // the next eight points' records
-          va = P.va[pt];
-          vb = P.vb[pt];
-          vc = P.vc[pt];
+          at += 8;                                // the next points' records
+          at -= at >= p1 ? p1 - p0 : 0;
+          va = P.va[at];
+          vb = P.vb[at];
+          vc = P.vc[at];
           dense_rows(rows, va0, vb0, u, sel0, sel1, m,
                      std::make_integer_sequence<int, NSLOTS>{});
           const uint64_t xt = xv + vc0;
-          const bool mine = base + p < p1 && (m.x | m.y | m.z | m.w) != 0u;
-          const unsigned bal = __ballot_sync(FULL, mine);
-          while (W.na + __popc(bal) > QCAP) stage_a(A, C, W, lane);
-          if (mine) {
-            const int at = W.na + __popc(bal & ((1u << lane) - 1u));
-            W.mask[at] = m;
-            W.qa[at] = make_uint2((uint32_t)xt, (uint32_t)(xt >> 32));
-          }
-          W.na += __popc(bal);
+          const bool l0 = n > 0 && (m.x | m.y) != 0u, l1 = n > 0 && (m.z | m.w) != 0u;
+          const unsigned bal0 = __ballot_sync(FULL, l0), bal1 = __ballot_sync(FULL, l1);
+          const int c0 = __popc(bal0), c1 = __popc(bal1);
+          while (W.na + c0 + c1 > ACAP) stage_a(A, C, W, lane);
+          const unsigned below = (1u << lane) - 1u;
+          if (l0)
+            W.qa[W.na + __popc(bal0 & below)] =
+                make_uint4(m.x, m.y, (uint32_t)xt, (uint32_t)(xt >> 32));
+          W.na += c0;
+          if (l1)
+            W.qa[W.na + __popc(bal1 & below)] =
+                make_uint4(m.z, m.w, (uint32_t)xt, (uint32_t)(xt >> 32) + (1u << 20));
+          W.na += c1;
         }
       }
       // the masks refer to this row's (b, j) list: none is left over
-      // entries refer to this row's (b, j) list: none is left over
       ClassArgs A1 = A;            // copies: what flush takes by reference lives in
       ClassShared C1 = C;          // local memory
       ClassWarp W1 = W;
