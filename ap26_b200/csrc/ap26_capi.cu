@@ -165,9 +165,9 @@ __global__ void chunk_begin_kernel(DevState *st, int ring) {
   st->chain_next[ring] = 0;
 }
 
-// The same for a class-sieve launch over units [begin, ...) of the run.
-__global__ void class_begin_kernel(DevState *st, int ring, unsigned long long begin) {
-  st->tile_next = begin;
+// The same for a class-sieve launch, which counts its own pieces.
+__global__ void class_begin_kernel(DevState *st, int ring) {
+  st->tile_next = 0;
   st->cand_count[ring] = 0;
   st->chain_next[ring] = 0;
 }
@@ -292,9 +292,14 @@ static cudaError_t upload_constants() {
 
 // Argument blocks are only built through these, so no field can be left
 // value-initialised (a null counter pointer would fault on the device).
+// Units [begin, begin + units) of a job on `blocks` CTAs.  The last unit of
+// each CTA (a unit takes about 1.2 ms) is split in four ranges of x: the five
+// launches of a K took 140.3 ms with whole units only, 137.2 with four parts
+// and 137.8 with eight, each of which builds its unit's rows again (135.3 in
+// one launch).  A launch of fewer units splits them in more.
 static ClassArgs class_args(const KJob *jobs, int job, const ClassPlan *plan,
-                            const uint32_t *tables, DevState *st, unsigned long long unit_base,
-                            unsigned long long unit_end, Cand *cand, long long cand_cap,
+                            const uint32_t *tables, DevState *st, int begin, int units,
+                            int blocks, Cand *cand, long long cand_cap,
                             unsigned long long *cand_count, unsigned long long *job_counts,
                             int count_only) {
   ClassArgs a;
@@ -303,8 +308,10 @@ static ClassArgs class_args(const KJob *jobs, int job, const ClassPlan *plan,
   a.plan = plan;
   a.tables = tables;
   a.st = st;
-  a.unit_end = unit_end;
-  a.unit_base = unit_base;
+  a.unit_begin = begin;
+  a.units = units;
+  a.split_units = std::min(units, blocks);
+  a.parts = std::min(64, std::max(4, 2 * blocks / units));
   a.cand = cand;
   a.cand_cap = cand_cap;
   a.cand_count = cand_count;
@@ -960,20 +967,19 @@ static cudaError_t emit_run(ap26_ctx *ctx, JobSet &S, const uint32_t *tables, in
     if (two_streams && c >= 2) EM(cudaStreamWaitEvent(s, ctx->chain_done[r], 0));
     if (S.by_class) {
       const int per_job = class_chunks(S.chunk_units), j = (int)(c / per_job);
-      const unsigned long long base = (unsigned long long)j * UNITS_PER_K,
-                               begin = base + (c % per_job) * S.chunk_units,
-                               end = std::min(begin + S.chunk_units, base + UNITS_PER_K);
-      if (begin == base) {   // the job's plan, over the previous job's
+      const int begin = (int)(c % per_job) * S.chunk_units;
+      const int units = std::min(S.chunk_units, UNITS_PER_K - begin);
+      if (begin == 0) {   // the job's plan, over the previous job's
         EM(cudaMemsetAsync(ctx->d_plan->vfill, 0, sizeof(ctx->d_plan->vfill), s));
         class_plan_count_kernel<<<ctx->num_sms * 4, 256, 0, s>>>(S.d_jobs + j, ctx->d_plan);
         class_plan_scan_kernel<<<1, 1024, 0, s>>>(ctx->d_plan);
         class_plan_scatter_kernel<<<ctx->num_sms * 8, 256, 0, s>>>(S.d_jobs + j, ctx->d_plan);
       }
-      class_begin_kernel<<<1, 1, 0, s>>>(S.d_st, r, begin);
+      class_begin_kernel<<<1, 1, 0, s>>>(S.d_st, r);
       if (c < S.nprof) EM(cudaEventRecordWithFlags(ctx->prof_events[2 * c], s, flag));
       class_sieve_kernel<<<ctx->num_sms, CLASS_WARPS * 32, CLASS_SMEM, s>>>(
-          class_args(S.d_jobs, j, ctx->d_plan, tables, S.d_st, base, end, ctx->d_cand[r],
-                     ctx->cand_cap, &S.d_st->cand_count[r], S.d_job_counts,
+          class_args(S.d_jobs, j, ctx->d_plan, tables, S.d_st, begin, units, ctx->num_sms,
+                     ctx->d_cand[r], ctx->cand_cap, &S.d_st->cand_count[r], S.d_job_counts,
                      S.count_only ? 1 : 0));
     } else {
       chunk_begin_kernel<<<1, 1, 0, s>>>(S.d_st, r);

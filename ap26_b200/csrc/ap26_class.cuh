@@ -413,9 +413,11 @@ struct ClassArgs {
   int job;                       // the K-job sieved
   const ClassPlan *plan;         // its plan
   const uint32_t *tables;        // job blocks of bitstrings (the 61 * 67 pair's first)
-  DevState *st;                  // tile_next counts units here
-  unsigned long long unit_end;   // units [DevState::tile_next, unit_end) of this launch
-  unsigned long long unit_base;  // the job's first unit
+  DevState *st;                  // tile_next counts pieces of this launch here
+  // Pieces: whole units from unit_begin on, then each of the last split_units
+  // in `parts` ranges of x, so the CTAs of a launch end within a part of a
+  // unit of each other.
+  int unit_begin, units, split_units, parts;
   Cand *cand;
   long long cand_cap;
   unsigned long long *cand_count;
@@ -691,13 +693,21 @@ __global__ void __launch_bounds__(CLASS_WARPS * 32, 1) class_sieve_kernel(ClassA
   for (;;) {
     if (threadIdx.x == 0) s_unit = atomicAdd(&A.st->tile_next, 1ull);
     __syncthreads();
-    const unsigned long long unit = s_unit;
-    if (unit >= A.unit_end) break;
-    const int local = (int)(unit - A.unit_base);
-    const int cls = local / ROWS_PER_CLASS;
+    const unsigned long long piece = s_unit;
+    const int whole = A.units - A.split_units;
+    if (piece >= (unsigned long long)(whole + A.split_units * A.parts)) break;
+    int unit = (int)piece, x_begin = 0, x_end = NUM_TRIPLES;
+    if (unit >= whole) {
+      const int part = (unit - whole) % A.parts;
+      unit = whole + (unit - whole) / A.parts;
+      x_begin = part * NUM_TRIPLES / A.parts;
+      x_end = (part + 1) * NUM_TRIPLES / A.parts;
+    }
+    unit += A.unit_begin;
+    const int cls = unit / ROWS_PER_CLASS;
     // row h of the class, then h + 4, ... while the class has more (b, j)
     // than four rows hold
-    for (int h = local % ROWS_PER_CLASS;; h += ROWS_PER_CLASS) {
+    for (int h = unit % ROWS_PER_CLASS;; h += ROWS_PER_CLASS) {
       // the (b, j) that pass 61 and 67, in the order of their coordinate
       // mod 71: LIST slots (coordinate, b, one of its j), EACH a thread
       constexpr int JS = (J_COUNT + SKIP - 1) / SKIP;       // j of one coordinate, 10
@@ -725,7 +735,7 @@ __global__ void __launch_bounds__(CLASS_WARPS * 32, 1) class_sieve_kernel(ClassA
       if (lane == 31) s_cnt[warp] = before;
       before -= __popc(mine);
       if (threadIdx.x < 4) s_o0[threadIdx.x] = -1;
-      if (threadIdx.x == 0) s_x = 0;
+      if (threadIdx.x == 0) s_x = x_begin;
       __syncthreads();
       int total = 0;
       for (int w = 0; w < CLASS_WARPS; w++) {
@@ -786,7 +796,7 @@ __global__ void __launch_bounds__(CLASS_WARPS * 32, 1) class_sieve_kernel(ClassA
         int xi = 0;
         if (lane == 0) xi = atomicAdd(&s_x, 1);
         xi = __shfl_sync(FULL, xi, 0);
-        if (xi >= NUM_TRIPLES) break;
+        if (xi >= x_end) break;
         int r = cls - P.xcls[xi];
         r += r < 0 ? CLASSES : 0;
         // the class's v of this x are bucket positions p0..p1-1, sorted by skip
