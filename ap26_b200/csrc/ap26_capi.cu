@@ -79,60 +79,9 @@ __device__ void build_table(int K, int shift, uint32_t *tab) {
   }
 }
 
-// The sorted lattice order of K, built by all threads of a block with
-// ORDER_SMEM bytes of dynamic shared memory: the 12673 n53 starts of an n43
-// value, index i = j43*667 + j47*29 + j53, ordered by (k1 / ORDER_BUCKET,
-// k2, i) with k1 = (j43*d43 + j47*d47 + j53*d53) mod 4087 and k2 the same
-// mod 5183 (d = S * MOD^-1 mod the pair's period): a bitonic sort of
-// 16384 packed keys (18 key bits, 14 index bits; padding sorts last).
-constexpr int ORDER_N = 16384;
-constexpr size_t ORDER_SMEM = sizeof(uint32_t) * ORDER_N;
-static_assert((PAIR1_P / ORDER_BUCKET + 1) * PAIR2_P < (1 << 18), "sort key fits 18 bits");
-
-__device__ void build_order(int K, uint16_t *perm) {
-  extern __shared__ uint32_t sk[];
-  __shared__ int d[6];
-  if (threadIdx.x == 0) {
-    int64_t S[3];
-    kmul_mod(PRES5, K, &S[0]);
-    kmul_mod(PRES6, K, &S[1]);
-    kmul_mod(PRES7, K, &S[2]);
-    for (int x = 0; x < 3; x++) {
-      d[x] = (int)(S[x] % PAIR1_P) * PAIR1_PARAM.A % PAIR1_P;
-      d[3 + x] = (int)(S[x] % PAIR2_P) * PAIR2_PARAM.A % PAIR2_P;
-    }
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < ORDER_N; i += blockDim.x) {
-    uint32_t v = 0xffffffffu;
-    if (i < N53_PER_N43) {
-      const int j43 = i / 667, j47 = (i - j43 * 667) / 29, j53 = i - j43 * 667 - j47 * 29;
-      const int k1 = (j43 * d[0] + j47 * d[1] + j53 * d[2]) % PAIR1_P;
-      const int k2 = (j43 * d[3] + j47 * d[4] + j53 * d[5]) % PAIR2_P;
-      v = ((uint32_t)((k1 / ORDER_BUCKET) * PAIR2_P + k2) << 14) | (uint32_t)i;
-    }
-    sk[i] = v;
-  }
-  __syncthreads();
-  for (int k = 2; k <= ORDER_N; k <<= 1)
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      for (int i = threadIdx.x; i < ORDER_N; i += blockDim.x) {
-        const int ixj = i ^ j;
-        if (ixj > i) {
-          const uint32_t a = sk[i], b = sk[ixj];
-          if ((a > b) == ((i & k) == 0)) { sk[i] = b; sk[ixj] = a; }
-        }
-      }
-      __syncthreads();
-    }
-  for (int i = threadIdx.x; i < N53_PER_N43; i += blockDim.x) perm[i] = (uint16_t)(sk[i] & 0x3fffu);
-  __syncthreads();
-}
-
-// Block j: job j (256 threads, ORDER_SMEM dynamic shared memory).  Thread 0
-// sets the reference's per-K constants; the block builds the job's
-// bitstrings and lattice order in its block at KJob::table unless
-// build_tables is 0 (a serving unit builds them once, at admission).
+// Block j: job j.  Thread 0 sets the reference's per-K constants; the block
+// builds the job's bitstrings in its block at KJob::table unless build_tables
+// is 0 (a serving unit builds them once, at admission).
 __global__ void setup_jobs_kernel(KJob *jobs, int njobs, uint32_t *tables, int build_tables) {
   const int j = blockIdx.x;
   if (j >= njobs) return;
@@ -149,11 +98,7 @@ __global__ void setup_jobs_kernel(KJob *jobs, int njobs, uint32_t *tables, int b
     kmul_mod(PRES7, K, &J.S53);
     kmul_mod(PRES8, K, &J.S59);
   }
-  if (build_tables) {
-    uint32_t *blk = tables + (size_t)J.table * JOB_TABLE_WORDS;
-    build_table(K, J.shift, blk);
-    build_order(K, reinterpret_cast<uint16_t *>(blk + TABLE_WORDS));
-  }
+  if (build_tables) build_table(K, J.shift, tables + (size_t)J.table * TABLE_WORDS);
 }
 
 // Chunk bookkeeping; `ring` selects the candidate ring this chunk fills.
@@ -464,9 +409,7 @@ static_assert(sizeof(AdmitArgs) <= 4000, "kernel parameters stay below 4 KB");
 __global__ void admit_unit_kernel(const AdmitArgs a, UnitState *units, uint32_t *pool) {
   if (a.write_init && blockIdx.x == 0 && threadIdx.x == 0) units[a.slot] = a.init;
   if ((int)blockIdx.x < a.n) {
-    uint32_t *blk = pool + (size_t)a.table[blockIdx.x] * JOB_TABLE_WORDS;
-    build_table(a.K[blockIdx.x], a.shift, blk);
-    build_order(a.K[blockIdx.x], reinterpret_cast<uint16_t *>(blk + TABLE_WORDS));
+    build_table(a.K[blockIdx.x], a.shift, pool + (size_t)a.table[blockIdx.x] * TABLE_WORDS);
   }
 }
 
@@ -699,7 +642,7 @@ static int jobset_ensure(ap26_ctx *ctx, JobSet &S, int njobs) {
     drop_graphs(ctx);   // graphs hold the old buffers' addresses
   }
   CK(cudaMalloc(&S.d_jobs, sizeof(KJob) * cap));
-  if (S.own_tables) CK(cudaMalloc(&S.d_tables, sizeof(uint32_t) * JOB_TABLE_WORDS * (size_t)cap));
+  if (S.own_tables) CK(cudaMalloc(&S.d_tables, sizeof(uint32_t) * TABLE_WORDS * (size_t)cap));
   CK(cudaMalloc(&S.d_job_counts, sizeof(unsigned long long) * cap));
   CK(cudaMalloc(&S.d_job_hash, sizeof(unsigned long long) * WORDS * cap));
   CK(cudaMalloc(&S.d_st, sizeof(DevState)));
@@ -769,11 +712,6 @@ extern "C" int ap26_create(int device, const ap26_opts *opts, ap26_ctx **out) {
     CKC(cudaFuncSetAttribute(class_sieve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              CLASS_SMEM));
     CKC(cudaMalloc(&ctx->d_plan, sizeof(ClassPlan)));
-    // the set-up kernels sort each K's lattice order in 64 KB of shared memory
-    CKC(cudaFuncSetAttribute(setup_jobs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)ORDER_SMEM));
-    CKC(cudaFuncSetAttribute(admit_unit_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)ORDER_SMEM));
     // buffers
     if (ctx->opts.cand_ring_log2 < 12 || ctx->opts.cand_ring_log2 > 27 ||
         ctx->opts.batch_wave > kMaxBatchWave) {
@@ -919,6 +857,16 @@ static int ensure_prof_events(ap26_ctx *ctx, unsigned long long n) {
   return AP26_OK;
 }
 
+// Enqueues one K-job's plan.
+static cudaError_t emit_plan(const KJob *job, ClassPlan *plan, int num_sms, cudaStream_t s) {
+  cudaError_t e = cudaMemsetAsync(plan->vfill, 0, sizeof(plan->vfill), s);
+  if (e != cudaSuccess) return e;
+  class_plan_count_kernel<<<num_sms * 4, 256, 0, s>>>(job, plan);
+  class_plan_scan_kernel<<<1, 1024, 0, s>>>(plan);
+  class_plan_scatter_kernel<<<num_sms * 8, 256, 0, s>>>(job, plan);
+  return cudaGetLastError();
+}
+
 // Class-sieve units per launch for chunks of chunk_tiles tiles of tile_n53
 // starts (at least one unit), made equal over a K's launches.
 static int class_chunk_units(int chunk_tiles, int64_t tile_n53) {
@@ -948,7 +896,7 @@ static cudaError_t emit_run(ap26_ctx *ctx, JobSet &S, const uint32_t *tables, in
   EM(cudaMemcpyAsync(S.d_st, S.h_st, sizeof(DevState), cudaMemcpyHostToDevice, s));
   EM(cudaMemsetAsync(S.d_job_counts, 0, sizeof(unsigned long long) * njobs, s));
   EM(cudaMemsetAsync(S.d_job_hash, 0, sizeof(unsigned long long) * WORDS * njobs, s));
-  setup_jobs_kernel<<<njobs, 256, ORDER_SMEM, s>>>(S.d_jobs, njobs, const_cast<uint32_t *>(tables),
+  setup_jobs_kernel<<<njobs, 256, 0, s>>>(S.d_jobs, njobs, const_cast<uint32_t *>(tables),
                                           build_tables);
   EM(cudaGetLastError());
   // ring r: candidate buffer d_cand[r] and its fill count DevState::cand_count[r]
@@ -969,12 +917,8 @@ static cudaError_t emit_run(ap26_ctx *ctx, JobSet &S, const uint32_t *tables, in
       const int per_job = class_chunks(S.chunk_units), j = (int)(c / per_job);
       const int begin = (int)(c % per_job) * S.chunk_units;
       const int units = std::min(S.chunk_units, UNITS_PER_K - begin);
-      if (begin == 0) {   // the job's plan, over the previous job's
-        EM(cudaMemsetAsync(ctx->d_plan->vfill, 0, sizeof(ctx->d_plan->vfill), s));
-        class_plan_count_kernel<<<ctx->num_sms * 4, 256, 0, s>>>(S.d_jobs + j, ctx->d_plan);
-        class_plan_scan_kernel<<<1, 1024, 0, s>>>(ctx->d_plan);
-        class_plan_scatter_kernel<<<ctx->num_sms * 8, 256, 0, s>>>(S.d_jobs + j, ctx->d_plan);
-      }
+      // the job's plan, over the previous job's
+      if (begin == 0) EM(emit_plan(S.d_jobs + j, ctx->d_plan, ctx->num_sms, s));
       class_begin_kernel<<<1, 1, 0, s>>>(S.d_st, r);
       if (c < S.nprof) EM(cudaEventRecordWithFlags(ctx->prof_events[2 * c], s, flag));
       class_sieve_kernel<<<ctx->num_sms, CLASS_WARPS * 32, CLASS_SMEM, s>>>(
@@ -1221,7 +1165,6 @@ static void fill_job(KJob &J, int K, int shift, int item, int64_t q0, int64_t q1
   J.q_begin = q0;
   J.q_end = q1;
   J.word_begin = word_begin;
-  J.flags = JOB_SORTED;
 }
 
 // Runs jobs, retrying with smaller chunks on a candidate-buffer overflow.
@@ -1477,7 +1420,7 @@ static int serve_chunk_tiles(const ap26_ctx *ctx) {
   const int64_t bound = ctx->cand_cap * 256 / (kMaxSurvivorsPer256Tile * tile_n53);
   return (int)std::max<int64_t>(64, std::min<int64_t>(ctx->opts.chunk_tiles, bound));
 }
-constexpr int64_t kTableBytes = (int64_t)JOB_TABLE_WORDS * 4;   // bitstrings + lattice order
+constexpr int64_t kTableBytes = (int64_t)TABLE_WORDS * 4;
 
 static int64_t slice_set_bytes() {
   const int64_t jobs = 64;   // jobset_ensure's minimum capacity
@@ -1568,7 +1511,7 @@ static int serve_admit(ap26_ctx *ctx, const ap26_item *item, int K_start, int it
       a.K[b] = u.ks[i + b];
       a.table[b] = u.tables[i + b];
     }
-    admit_unit_kernel<<<std::max(1, a.n), 256, ORDER_SMEM, ctx->stream>>>(a, ctx->d_units,
+    admit_unit_kernel<<<std::max(1, a.n), 256, 0, ctx->stream>>>(a, ctx->d_units,
                                                                           ctx->d_pool);
     CK(cudaGetLastError());
     i += (size_t)a.n;
@@ -1801,7 +1744,6 @@ extern "C" int ap26_sieve_range(ap26_ctx *ctx, int K, int shift, int64_t q_begin
   J.ntiles = (int32_t)tiles;
   J.tile_begin = 0;
   J.table = 0;
-  J.flags = 0;   // natural lattice order: [q_begin, q_end) are the reference's positions
   memset(S.h_st, 0, sizeof(DevState));
   S.h_st->chunk_size = (unsigned long long)std::max<int64_t>(1, tiles);
   S.h_st->total_tiles = (unsigned long long)tiles;
@@ -1811,7 +1753,7 @@ extern "C" int ap26_sieve_range(ap26_ctx *ctx, int K, int shift, int64_t q_begin
   CK(cudaMemcpyAsync(S.d_jobs, S.h_jobs, sizeof(KJob), cudaMemcpyHostToDevice, s));
   CK(cudaMemcpyAsync(S.d_st, S.h_st, sizeof(DevState), cudaMemcpyHostToDevice, s));
   CK(cudaMemsetAsync(S.d_job_counts, 0, sizeof(unsigned long long), s));
-  setup_jobs_kernel<<<1, 256, ORDER_SMEM, s>>>(S.d_jobs, 1, S.d_tables, 1);
+  setup_jobs_kernel<<<1, 256, 0, s>>>(S.d_jobs, 1, S.d_tables, 1);
   chunk_begin_kernel<<<1, 1, 0, s>>>(S.d_st, 0);
   const SieveArgs sa = sieve_args(S.d_jobs, 1, S.d_tables, S.d_st, ctx->d_cand[0],
                                   ctx->cand_cap, S.d_job_counts, 0, &S.d_st->cand_count[0]);
@@ -1997,7 +1939,7 @@ extern "C" int ap26_chain_batch(ap26_ctx *ctx, int K, const int64_t *n, int64_t 
   memset(S.h_st, 0, sizeof(DevState));
   CK(cudaMemcpyAsync(S.d_jobs, S.h_jobs, sizeof(KJob), cudaMemcpyHostToDevice, s));
   CK(cudaMemcpyAsync(S.d_st, S.h_st, sizeof(DevState), cudaMemcpyHostToDevice, s));
-  setup_jobs_kernel<<<1, 256, ORDER_SMEM, s>>>(S.d_jobs, 1, S.d_tables, 0);
+  setup_jobs_kernel<<<1, 256, 0, s>>>(S.d_jobs, 1, S.d_tables, 0);
   CK(cudaMemcpyAsync(dn.p, n, sizeof(int64_t) * count, cudaMemcpyHostToDevice, s));
   CK(cudaEventRecord(ctx->ev0, s));
   chain_explicit_kernel<<<ctx->num_sms * 8, 128, 0, s>>>(S.d_jobs, dn.p, count, dk.p, df.p,
@@ -2120,7 +2062,8 @@ struct NoallocScratch {
   DevState st;
   KJob jobs[AP26_NOALLOC_MAX_K];
   unsigned long long counts[AP26_NOALLOC_MAX_K];
-  uint32_t tables[AP26_NOALLOC_MAX_K][JOB_TABLE_WORDS];
+  uint32_t tables[AP26_NOALLOC_MAX_K][TABLE_WORDS];
+  ClassPlan plan;                // of the K being sieved
 };
 static_assert(sizeof(NoallocScratch) == AP26_NOALLOC_SCRATCH_BYTES,
               "the scratch size stated in ap26.h");
@@ -2128,14 +2071,10 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[sizeof(NoallocS
 
 // Fills the job descriptors and zeroes the counters and state left behind by
 // the previous call (the array keeps the last call's contents).  A K outside
-// [1, AP26_KMAX_SAFE] gets an empty lattice range, no tiles and a count of
-// -1, so it costs the sieve nothing; the tile prefix skips it (find_job takes
-// the last job whose first tile is <= the tile, which is never an empty one).
-__global__ void noalloc_init_kernel(NoallocScratch *s, const int32_t *Ks, int nK, int shift,
-                                    int tile_n53) {
-  __shared__ int32_t s_tiles[AP26_NOALLOC_MAX_K];
+// [1, AP26_KMAX_SAFE] gets an empty lattice range and a count of -1, and the
+// class kernels pass it over, so it costs the sieve nothing.
+__global__ void noalloc_init_kernel(NoallocScratch *s, const int32_t *Ks, int nK, int shift) {
   const int j = threadIdx.x;
-  const int64_t ntiles = (N53_PER_K + tile_n53 - 1) / tile_n53;
   if (j < nK) {
     KJob &J = s->jobs[j];
     const int K = Ks[j];
@@ -2144,27 +2083,11 @@ __global__ void noalloc_init_kernel(NoallocScratch *s, const int32_t *Ks, int nK
     J.K = ok ? K : 1;
     J.shift = shift;
     J.item = ok ? 0 : -1;
-    J.q_begin = 0;
     J.q_end = ok ? N53_PER_K : 0;
-    J.ntiles = ok ? (int32_t)ntiles : 0;
     J.table = j;
-    J.flags = JOB_SORTED;
-    s_tiles[j] = J.ntiles;
     s->counts[j] = 0;
   }
-  __syncthreads();
-  if (j < nK) {
-    int64_t begin = 0;
-    for (int i = 0; i < j; i++) begin += s_tiles[i];
-    s->jobs[j].tile_begin = begin;
-  }
-  if (j == 0) {
-    int64_t total = 0;
-    for (int i = 0; i < nK; i++) total += s_tiles[i];
-    memset(&s->st, 0, sizeof(DevState));
-    s->st.chunk_size = (unsigned long long)total;
-    s->st.total_tiles = (unsigned long long)total;
-  }
+  if (j == 0) memset(&s->st, 0, sizeof(DevState));
 }
 
 __global__ void noalloc_finish_kernel(const NoallocScratch *s, int nK, int64_t *out) {
@@ -2174,7 +2097,7 @@ __global__ void noalloc_finish_kernel(const NoallocScratch *s, int nK, int64_t *
 
 struct NoallocDevice {
   NoallocScratch *ptr = nullptr;
-  int sieve_blocks = 0;
+  int num_sms = 0;
   bool ready = false;
 };
 static NoallocDevice g_noalloc_dev[64];
@@ -2182,7 +2105,7 @@ static std::mutex g_noalloc_mu;
 
 // Once per device, with that device current: the scratch array's device
 // address (its host-side name is only a stand-in), the constant tables, and
-// the launch shape of the default sieve variant.  Synchronous calls, so the
+// the kernels' shared memory.  Synchronous calls, so the
 // first call on a device must come before any stream capture.
 static int noalloc_setup(int device, NoallocDevice **out) {
   std::lock_guard<std::mutex> lock(g_noalloc_mu);
@@ -2191,20 +2114,14 @@ static int noalloc_setup(int device, NoallocDevice **out) {
     void *p = nullptr;
     if (cudaGetSymbolAddress(&p, g_noalloc_scratch) != cudaSuccess) return AP26_E_CUDA;
     if (upload_constants() != cudaSuccess) return AP26_E_CUDA;
-    if (cudaFuncSetAttribute(setup_jobs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)ORDER_SMEM) != cudaSuccess)
+    if (cudaFuncSetAttribute(class_sieve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             CLASS_SMEM) != cudaSuccess)
       return AP26_E_CUDA;
-    const SieveVariant &V = kVariants[0];
-    if (cudaFuncSetAttribute(V.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)V.smem()) != cudaSuccess)
-      return AP26_E_CUDA;
-    int per_sm = 0, sms = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, V.kernel, V.WARPS * 32,
-                                                      V.smem()) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
       return AP26_E_CUDA;
     d.ptr = static_cast<NoallocScratch *>(p);
-    d.sieve_blocks = sms * (per_sm > 0 ? per_sm : 1);
+    d.num_sms = sms;
     d.ready = true;
   }
   *out = &d;
@@ -2235,19 +2152,24 @@ extern "C" int ap26_sieve_count_noalloc(int device, const int32_t *d_Ks, int nK,
   int rc = noalloc_setup(device, &d);
   if (rc == AP26_OK) {
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const SieveVariant &V = kVariants[0];
     NoallocScratch *S = d->ptr;
     do {
-      noalloc_init_kernel<<<1, AP26_NOALLOC_MAX_K, 0, s>>>(S, d_Ks, nK, shift, V.WARPS * 32);
+      noalloc_init_kernel<<<1, AP26_NOALLOC_MAX_K, 0, s>>>(S, d_Ks, nK, shift);
       if (noalloc_launch_failed()) { rc = AP26_E_CUDA; break; }
-      setup_jobs_kernel<<<nK, 256, ORDER_SMEM, s>>>(S->jobs, nK, &S->tables[0][0], 1);
+      setup_jobs_kernel<<<nK, 256, 0, s>>>(S->jobs, nK, &S->tables[0][0], 1);
       if (noalloc_launch_failed()) { rc = AP26_E_CUDA; break; }
-      chunk_begin_kernel<<<1, 1, 0, s>>>(&S->st, 0);
-      if (noalloc_launch_failed()) { rc = AP26_E_CUDA; break; }
-      const SieveArgs sa = sieve_args(S->jobs, nK, &S->tables[0][0], &S->st, nullptr, 0,
-                                      S->counts, 1, &S->st.cand_count[0]);
-      V.kernel<<<d->sieve_blocks, V.WARPS * 32, V.smem(), s>>>(sa);
-      if (noalloc_launch_failed()) { rc = AP26_E_CUDA; break; }
+      for (int j = 0; j < nK && rc == AP26_OK; j++) {
+        if (emit_plan(S->jobs + j, &S->plan, d->num_sms, s) != cudaSuccess) {
+          rc = AP26_E_CUDA;
+          break;
+        }
+        class_begin_kernel<<<1, 1, 0, s>>>(&S->st, 0);
+        class_sieve_kernel<<<d->num_sms, CLASS_WARPS * 32, CLASS_SMEM, s>>>(
+            class_args(S->jobs, j, &S->plan, &S->tables[0][0], &S->st, 0, UNITS_PER_K, d->num_sms,
+                       nullptr, 0, &S->st.cand_count[0], S->counts, 1));
+        if (noalloc_launch_failed()) rc = AP26_E_CUDA;
+      }
+      if (rc != AP26_OK) break;
       noalloc_finish_kernel<<<1, AP26_NOALLOC_MAX_K, 0, s>>>(S, nK, d_counts);
       if (noalloc_launch_failed()) { rc = AP26_E_CUDA; break; }
     } while (0);

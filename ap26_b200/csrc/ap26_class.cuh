@@ -298,6 +298,7 @@ __device__ __forceinline__ int v_bucket(int64_t v, const SkipCoord &c) {
 // tables and the bitstrings.  Grid-stride over all of them.
 __global__ void class_plan_count_kernel(const KJob *job, ClassPlan *P) {
   const KJob &J = *job;
+  if (J.q_end == 0) return;                     // an empty job: nothing is sieved
   const int K = J.K, shift = J.shift;
   const SkipCoord sc = skip_coord(K);
   const int stride = gridDim.x * blockDim.x;
@@ -394,6 +395,7 @@ __global__ void __launch_bounds__(1024) class_plan_scan_kernel(ClassPlan *P) {
 // Third step: the v records in bucket order (any order inside a bucket).
 __global__ void class_plan_scatter_kernel(const KJob *job, ClassPlan *P) {
   const KJob &J = *job;
+  if (J.q_end == 0) return;
   const SkipCoord sc = skip_coord(J.K);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < NV; i += gridDim.x * blockDim.x) {
     const int64_t v = v_value(J, i);
@@ -669,7 +671,8 @@ __global__ void __launch_bounds__(CLASS_WARPS * 32, 1) class_sieve_kernel(ClassA
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const ClassPlan &P = *A.plan;
-  const uint32_t *table = A.tables + (size_t)A.jobs[A.job].table * JOB_TABLE_WORDS;
+  if (A.jobs[A.job].q_end == 0) return;
+  const uint32_t *table = A.tables + (size_t)A.jobs[A.job].table * TABLE_WORDS;
   ClassWarp W;
   W.qa = masks + warp * ACAP;
   W.qb = queues + warp * 3 * QCAP;

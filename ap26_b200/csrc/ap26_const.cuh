@@ -59,23 +59,7 @@ constexpr int word_offset(int g) {                   // g >= PAIR_PRIMES
   for (int i = PAIR_PRIMES; i < g; i++) o += nwords(PRIMES[i]);
   return o;
 }
-constexpr int TABLE_WORDS = word_offset(NPRIMES);   // 2806 words, 11224 bytes
-
-// Lattice order.  The 12673 n53 starts of one n43 value (index j43*667 +
-// j47*29 + j53) are visited sorted by their window starts in the pair
-// bitstrings: the start in the 61*67 string is k1 = (j43*d43 + j47*d47 +
-// j53*d53) mod 4087 (d = S * MOD^-1 mod 4087) up to the reductions mod MOD
-// (at most 3), and k2 likewise mod 5183.  Starts are ordered by k1 in
-// buckets of ORDER_BUCKET values, and by k2 inside a bucket (about 320
-// starts each).  The 32 starts of a warp then lie within about 230 bits of
-// each other in the first string and 870 bits in the second, and the 8
-// starts of a quarter warp (one phase of a 128-bit load) nearly always
-// within 8 consecutive quad entries: a CPU model of the order counts no
-// extra wavefronts for the first string and 1-3% for the second.  The
-// order is one 16-bit index per start, built with the tables.
-constexpr int ORDER_BUCKET = 103;
-constexpr int PERM_WORDS = (N53_PER_N43 + 1) / 2;   // 6337 words
-constexpr int JOB_TABLE_WORDS = TABLE_WORDS + PERM_WORDS;   // per K-job, 36,572 bytes
+constexpr int TABLE_WORDS = word_offset(NPRIMES);   // per K-job, 2806 words, 11224 bytes
 
 constexpr int64_t mod_pos(int64_t a, int64_t m) { return ((a % m) + m) % m; }
 constexpr int inv_mod(int a, int p) {                // a^-1 mod p, a coprime to p

@@ -38,9 +38,8 @@
 // that differ by at most (p-1)/32 < 17, within one 32-bank row.
 // Primes 61 and 67 share one string of period 4087 (bit j = B_61[j] &
 // B_67[j], window start n59 * MOD^-1 mod 4087), and 71 and 73 one of
-// period 5183; their windows are read conflict-free because the starts of
-// an n43 value are visited sorted by those window starts (ap26_const.cuh),
-// so a warp's 32 starts lie close together in both strings.
+// period 5183: one window each instead of two, at the price of bank
+// conflicts, since a warp's starts lie anywhere in the string.
 //
 //   dense phase  the first G primes for all 10 words of every n59: G-2
 //                windows (the two pairs, primes 4..G-1), each five 128-bit
@@ -67,11 +66,7 @@ struct KJob {
   int32_t K, shift, item, ntiles;
   int32_t word_begin;         // first shift word reported (the reference's ITER)
   int32_t table;              // index of this job's block in SieveArgs::tables
-  int32_t flags;              // JOB_SORTED: n53 starts in the sorted lattice order
-  int32_t pad;
 };
-
-enum : int32_t { JOB_SORTED = 1 };
 
 struct Cand {
   int64_t n;
@@ -109,8 +104,7 @@ enum : unsigned int {
 struct SieveArgs {
   const KJob *jobs;
   int njobs;
-  const uint32_t *tables;       // [*][JOB_TABLE_WORDS] (bitstrings, lattice order),
-                                // job j's at KJob::table
+  const uint32_t *tables;       // [*][TABLE_WORDS] bitstrings, job j's at KJob::table
   DevState *st;
   Cand *cand;
   long long cand_cap;
@@ -365,12 +359,9 @@ __device__ __forceinline__ int front_drain(const SieveArgs &A, const uint32_t *t
 // n43 = (n0 + i3*S3 + i5*S5 + i31*S31 + i37*S37 + i41*S41) mod MOD
 // (AP26.h:134) and n53 = n43 + j43*S43 + j47*S47 + j53*S53 mod MOD, the
 // value the reference's nested increments reach (setupn.cl:31-53).
-// With the sorted lattice order (perm != null) the q-th start of an n43
-// value is the perm[q mod 12673]-th of its natural order.
-__device__ __forceinline__ int64_t n53_at(const KJob &J, int64_t q, const uint16_t *perm) {
+__device__ __forceinline__ int64_t n53_at(const KJob &J, int64_t q) {
   int n43i = (int)(q / N53_PER_N43);
   int rem = (int)(q - (int64_t)n43i * N53_PER_N43);
-  if (perm) rem = perm[rem];
   int j43 = rem / 667;
   rem -= j43 * 667;
   int j47 = rem / 29;
@@ -430,7 +421,6 @@ sieve_kernel(SieveArgs A) {
   static_assert(QCAP >= 32 * WORDS, "queue too small for one dense batch");
 
   int cur_job = -1, cur_shift = 0;
-  const uint16_t *cur_perm = nullptr;
   int cnt = 0, lcnt = 0;
   unsigned long long kept_acc = 0, late_acc = 0;
 
@@ -461,9 +451,7 @@ sieve_kernel(SieveArgs A) {
         }
       }
       if (job < 0) break;
-      const uint32_t *src = A.tables + (size_t)A.jobs[job].table * JOB_TABLE_WORDS;
-      cur_perm = (A.jobs[job].flags & JOB_SORTED)
-                     ? reinterpret_cast<const uint16_t *>(src + TABLE_WORDS) : nullptr;
+      const uint32_t *src = A.tables + (size_t)A.jobs[job].table * TABLE_WORDS;
       for (int i = threadIdx.x; i < D; i += blockDim.x)   // D + 3 <= TABLE_WORDS
         reinterpret_cast<uint4 *>(tab)[i] = make_uint4(src[i], src[i + 1], src[i + 2], src[i + 3]);
       for (int i = D + threadIdx.x; i < TABLE_WORDS; i += blockDim.x) ptab[i] = src[i];
@@ -477,7 +465,7 @@ sieve_kernel(SieveArgs A) {
                        (int64_t)(tile - (unsigned long long)J.tile_begin) * (WARPS * 32) +
                        warp * 32 + lane;
     const bool valid = qi < J.q_end;
-    int64_t n59 = valid ? n53_at(J, qi, cur_perm) : 0;
+    int64_t n59 = valid ? n53_at(J, qi) : 0;
 
     for (int j = 0; j < J59; j++) {
       uint32_t acc[20];
