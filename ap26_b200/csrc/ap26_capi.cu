@@ -32,62 +32,35 @@ __device__ int kmul_mod(int64_t c, int K, int64_t *out) {
   return 0;
 }
 
-// Bit j of prime p's bitstring, B_p[j] = OK_p[((j + SHIFT) * MOD) mod p], with
-// OK_p[r] = 0 iff r = (jj * (STEP mod p)) mod p for some jj in [p-23, p]
-// (MAKE_OK, src/cpu/cpusse2.cpp:32-36; setok.cl:79-81).  stinv = (STEP mod
-// p)^-1 mod p, or 0 when p divides STEP.
-__device__ __forceinline__ bool bstr_bit(int p, int stinv, int cm, int sh, int j) {
-  const int r = (j + sh) % p * cm % p;
-  if (!stinv) return r != 0;
-  const int tt = r * stinv % p;
-  return tt != 0 && tt < p - 23;
-}
-
-__device__ int step_inv(int K, int p) {     // (K * 23# mod p)^(p-2) mod p, or 0
-  const int st = (int)(((int64_t)(K % p) * (int)(PRIM23 % p)) % p);
-  if (!st) return 0;
-  int e = p - 2, base = st, r = 1;
-  while (e) { if (e & 1) r = r * base % p; base = base * base % p; e >>= 1; }
-  return r;
-}
-
-// The sieve bitstrings of one (K, SHIFT), built by all threads of a block:
-// the two pair bitstrings (bit j = B_61[j] & B_67[j], then B_71[j] &
-// B_73[j]) and one bitstring per prime 4..82 at c_params[g].off.
-__device__ void build_table(int K, int shift, uint32_t *tab) {
-  for (int t = threadIdx.x; t < TABLE_WORDS; t += blockDim.x) {
-    uint32_t word = 0;
-    if (t < PAIR1_WORDS + PAIR2_WORDS) {
-      const bool first = t < PAIR1_WORDS;
-      const int p = first ? 61 : 71, q = first ? 67 : 73;
-      const int ip = step_inv(K, p), iq = step_inv(K, q);
-      const int cp = (int)(MOD % p), cq = (int)(MOD % q);
-      const int j0 = (first ? t : t - PAIR1_WORDS) * 32;
-      for (int u = 0; u < 32; u++)
-        if (bstr_bit(p, ip, cp, shift % p, j0 + u) && bstr_bit(q, iq, cq, shift % q, j0 + u))
-          word |= 1u << u;
+// Words first, first + stride, ... below `words` of the sieve bitstrings of
+// one (K, SHIFT): B_p[j] = OK_p[((j + SHIFT) * MOD) mod p] (MAKE_OK,
+// src/cpu/cpusse2.cpp:32-36; setok.cl:79-81), as the two pair bitstrings (bit
+// j = B_61[j] & B_67[j], then B_71[j] & B_73[j]) and one bitstring per prime
+// 4..82 at c_params[g].off.
+__device__ void build_table(int K, int shift, uint32_t *tab, int first, int stride, int words) {
+  for (int t = first; t < words; t += stride) {
+    if (t < PAIR1_WORDS) {
+      tab[t] = string_word(K, shift, 61, 67, 1, t * 32);
+    } else if (t < PAIR1_WORDS + PAIR2_WORDS) {
+      tab[t] = string_word(K, shift, 71, 73, 1, (t - PAIR1_WORDS) * 32);
     } else {
       int g = PAIR_PRIMES;
       while (g + 1 < NPRIMES && c_params[g + 1].off <= t) g++;
-      const int p = c_params[g].p;
-      const int stinv = step_inv(K, p), cm = (int)(MOD % p), sh = shift % p;
-      const int j0 = (t - c_params[g].off) * 32;
-      for (int u = 0; u < 32; u++)
-        if (bstr_bit(p, stinv, cm, sh, j0 + u)) word |= 1u << u;
+      tab[t] = string_word(K, shift, c_params[g].p, 1, 1, (t - c_params[g].off) * 32);
     }
-    tab[t] = word;
   }
 }
 
-// Block j: job j.  Thread 0 sets the reference's per-K constants; the block
-// builds the job's bitstrings in its block at KJob::table unless build_tables
-// is 0 (a serving unit builds them once, at admission).
-__global__ void setup_jobs_kernel(KJob *jobs, int njobs, uint32_t *tables, int build_tables) {
-  const int j = blockIdx.x;
-  if (j >= njobs) return;
-  KJob &J = jobs[j];
+// Blocks (j, y): job j.  Thread 0 of y = 0 sets the reference's per-K
+// constants; the blocks share the first `words` words of the job's bitstrings
+// at KJob::table: all of them for the window sieve, the 61 * 67 pair's for
+// the class sieve, none where a serving unit built them at admission.  A word
+// is a chain of some 600 instructions, so one word a thread: a block of 256
+// that built eleven each (and sorted a lattice order) took 0.3 ms.
+__global__ void setup_jobs_kernel(KJob *jobs, uint32_t *tables, int words) {
+  KJob &J = jobs[blockIdx.x];
   const int K = J.K;
-  if (threadIdx.x == 0) {
+  if (threadIdx.x == 0 && blockIdx.y == 0) {
     J.STEP = (int64_t)K * PRIM23;
     J.n0 = (N0 * (K % 17835) + ((N0 * 17835) % MOD) * (K / 17835) + N30) % MOD;
     kmul_mod(PRES2, K, &J.S31);
@@ -98,7 +71,13 @@ __global__ void setup_jobs_kernel(KJob *jobs, int njobs, uint32_t *tables, int b
     kmul_mod(PRES7, K, &J.S53);
     kmul_mod(PRES8, K, &J.S59);
   }
-  if (build_tables) build_table(K, J.shift, tables + (size_t)J.table * TABLE_WORDS);
+  build_table(K, J.shift, tables + (size_t)J.table * TABLE_WORDS,
+              (int)(blockIdx.y * blockDim.x + threadIdx.x), (int)(gridDim.y * blockDim.x), words);
+}
+
+static void launch_setup(KJob *jobs, int njobs, uint32_t *tables, int words, cudaStream_t s) {
+  setup_jobs_kernel<<<dim3((unsigned)njobs, (unsigned)std::max(1, (words + 255) / 256)), 256, 0,
+                      s>>>(jobs, tables, words);
 }
 
 // Chunk bookkeeping; `ring` selects the candidate ring this chunk fills.
@@ -267,8 +246,9 @@ static ClassArgs class_args(const KJob *jobs, int job, const ClassPlan *plan,
 
 static SieveArgs sieve_args(const KJob *jobs, int njobs, const uint32_t *tables, DevState *st,
                             Cand *cand, long long cand_cap, unsigned long long *job_counts,
-                            int count_only, unsigned long long *cand_count) {
+                            int count_only, unsigned long long *cand_count, int parts = 1) {
   SieveArgs a;
+  a.parts = parts;
   a.jobs = jobs;
   a.njobs = njobs;
   a.tables = tables;
@@ -409,7 +389,8 @@ static_assert(sizeof(AdmitArgs) <= 4000, "kernel parameters stay below 4 KB");
 __global__ void admit_unit_kernel(const AdmitArgs a, UnitState *units, uint32_t *pool) {
   if (a.write_init && blockIdx.x == 0 && threadIdx.x == 0) units[a.slot] = a.init;
   if ((int)blockIdx.x < a.n) {
-    build_table(a.K[blockIdx.x], a.shift, pool + (size_t)a.table[blockIdx.x] * TABLE_WORDS);
+    build_table(a.K[blockIdx.x], a.shift, pool + (size_t)a.table[blockIdx.x] * TABLE_WORDS,
+                (int)threadIdx.x, (int)blockDim.x, TABLE_WORDS);
   }
 }
 
@@ -896,8 +877,8 @@ static cudaError_t emit_run(ap26_ctx *ctx, JobSet &S, const uint32_t *tables, in
   EM(cudaMemcpyAsync(S.d_st, S.h_st, sizeof(DevState), cudaMemcpyHostToDevice, s));
   EM(cudaMemsetAsync(S.d_job_counts, 0, sizeof(unsigned long long) * njobs, s));
   EM(cudaMemsetAsync(S.d_job_hash, 0, sizeof(unsigned long long) * WORDS * njobs, s));
-  setup_jobs_kernel<<<njobs, 256, 0, s>>>(S.d_jobs, njobs, const_cast<uint32_t *>(tables),
-                                          build_tables);
+  launch_setup(S.d_jobs, njobs, const_cast<uint32_t *>(tables),
+               !build_tables ? 0 : S.by_class ? PAIR1_WORDS : TABLE_WORDS, s);
   EM(cudaGetLastError());
   // ring r: candidate buffer d_cand[r] and its fill count DevState::cand_count[r]
   SieveArgs sa[2];
@@ -1726,6 +1707,17 @@ extern "C" int ap26_serve_memory(const ap26_ctx *ctx, int64_t *in_use, int64_t *
   return AP26_OK;
 }
 
+// j59 ranges a start's 35 n59 values are split in, so that a short range of
+// starts fills the GPU and a longer one ends evenly: the fewest (of the
+// divisors of 35) that give every resident CTA eight tiles.  Device time with
+// the set-up, at one part and now: 12673 starts 774 and 85 us, 120000 968 and
+// 477, 600011 2114 and 1695 (of which the set-up was 600 and is 40).
+static int range_parts(const ap26_ctx *ctx, int64_t blocks) {
+  for (int parts : {1, 5, 7})
+    if (blocks * parts >= 8 * (int64_t)ctx->sieve_blocks) return parts;
+  return J59;
+}
+
 // ---- kernel-level entry points ---------------------------------------------------------
 extern "C" int ap26_sieve_range(ap26_ctx *ctx, int K, int shift, int64_t q_begin, int64_t q_end,
                                 int64_t *cand, int64_t cap, int64_t *n_cand, ap26_stats *stats) {
@@ -1739,7 +1731,9 @@ extern "C" int ap26_sieve_range(ap26_ctx *ctx, int K, int shift, int64_t q_begin
   // set-up and sieve only, in one launch over the whole range, candidates kept
   fill_job(S.h_jobs[0], K, shift, 0, q_begin, q_end);
   const int64_t tile_n53 = (int64_t)kVariants[ctx->variant].WARPS * 32;
-  const int64_t tiles = (q_end - q_begin + tile_n53 - 1) / tile_n53;
+  const int64_t blocks = (q_end - q_begin + tile_n53 - 1) / tile_n53;
+  const int parts = range_parts(ctx, blocks);
+  const int64_t tiles = blocks * parts;
   KJob &J = S.h_jobs[0];
   J.ntiles = (int32_t)tiles;
   J.tile_begin = 0;
@@ -1753,10 +1747,10 @@ extern "C" int ap26_sieve_range(ap26_ctx *ctx, int K, int shift, int64_t q_begin
   CK(cudaMemcpyAsync(S.d_jobs, S.h_jobs, sizeof(KJob), cudaMemcpyHostToDevice, s));
   CK(cudaMemcpyAsync(S.d_st, S.h_st, sizeof(DevState), cudaMemcpyHostToDevice, s));
   CK(cudaMemsetAsync(S.d_job_counts, 0, sizeof(unsigned long long), s));
-  setup_jobs_kernel<<<1, 256, 0, s>>>(S.d_jobs, 1, S.d_tables, 1);
+  launch_setup(S.d_jobs, 1, S.d_tables, TABLE_WORDS, s);
   chunk_begin_kernel<<<1, 1, 0, s>>>(S.d_st, 0);
   const SieveArgs sa = sieve_args(S.d_jobs, 1, S.d_tables, S.d_st, ctx->d_cand[0],
-                                  ctx->cand_cap, S.d_job_counts, 0, &S.d_st->cand_count[0]);
+                                  ctx->cand_cap, S.d_job_counts, 0, &S.d_st->cand_count[0], parts);
   V.kernel<<<ctx->sieve_blocks, V.WARPS * 32, V.smem(), s>>>(sa);
   CK(cudaGetLastError());
   CK(cudaMemcpyAsync(S.h_st, S.d_st, sizeof(DevState), cudaMemcpyDeviceToHost, s));
@@ -1939,7 +1933,7 @@ extern "C" int ap26_chain_batch(ap26_ctx *ctx, int K, const int64_t *n, int64_t 
   memset(S.h_st, 0, sizeof(DevState));
   CK(cudaMemcpyAsync(S.d_jobs, S.h_jobs, sizeof(KJob), cudaMemcpyHostToDevice, s));
   CK(cudaMemcpyAsync(S.d_st, S.h_st, sizeof(DevState), cudaMemcpyHostToDevice, s));
-  setup_jobs_kernel<<<1, 256, 0, s>>>(S.d_jobs, 1, S.d_tables, 0);
+  launch_setup(S.d_jobs, 1, S.d_tables, 0, s);
   CK(cudaMemcpyAsync(dn.p, n, sizeof(int64_t) * count, cudaMemcpyHostToDevice, s));
   CK(cudaEventRecord(ctx->ev0, s));
   chain_explicit_kernel<<<ctx->num_sms * 8, 128, 0, s>>>(S.d_jobs, dn.p, count, dk.p, df.p,
@@ -2156,7 +2150,7 @@ extern "C" int ap26_sieve_count_noalloc(int device, const int32_t *d_Ks, int nK,
     do {
       noalloc_init_kernel<<<1, AP26_NOALLOC_MAX_K, 0, s>>>(S, d_Ks, nK, shift);
       if (noalloc_launch_failed()) { rc = AP26_E_CUDA; break; }
-      setup_jobs_kernel<<<nK, 256, 0, s>>>(S->jobs, nK, &S->tables[0][0], 1);
+      launch_setup(S->jobs, nK, &S->tables[0][0], PAIR1_WORDS, s);
       if (noalloc_launch_failed()) { rc = AP26_E_CUDA; break; }
       for (int j = 0; j < nK && rc == AP26_OK; j++) {
         if (emit_plan(S->jobs + j, &S->plan, d->num_sms, s) != cudaSuccess) {

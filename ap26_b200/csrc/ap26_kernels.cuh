@@ -111,6 +111,7 @@ struct SieveArgs {
   unsigned long long *job_counts;  // per-job survivor counts
   int count_only;               // 1: count survivors, emit no candidates
   unsigned long long *cand_count;  // fill count of `cand` (DevState::cand_count[ring])
+  int parts;                    // tiles per block of starts, each 35 / parts of its j59
 };
 
 struct ChainArgs {
@@ -394,8 +395,8 @@ __device__ __forceinline__ int find_job(const KJob *jobs, int njobs, unsigned lo
 }
 
 // ---- the sieve kernel -----------------------------------------------------------
-// Persistent: each CTA grabs tiles (one n53 start per thread) from
-// DevState::tile_next until the chunk window ends; 35 n59 per start.  The
+// Persistent: each CTA grabs tiles (one n53 start per thread and 35 / parts
+// of its n59) from DevState::tile_next until the chunk window ends.  The
 // per-warp queues carry over from tile to tile and are flushed only when the
 // CTA moves to another K-job (the shared table changes) or runs out of work.
 template <int G, int R, int SL, int QCAP, int LCAP, int WARPS>
@@ -461,13 +462,14 @@ sieve_kernel(SieveArgs A) {
     }
     const KJob &J = A.jobs[job];
     const int64_t S59 = J.S59;
-    const int64_t qi = J.q_begin +
-                       (int64_t)(tile - (unsigned long long)J.tile_begin) * (WARPS * 32) +
-                       warp * 32 + lane;
+    const uint32_t local = (uint32_t)(tile - (unsigned long long)J.tile_begin);
+    const int steps = J59 / A.parts;
+    const int64_t qi = J.q_begin + (int64_t)(local / A.parts) * (WARPS * 32) + warp * 32 + lane;
     const bool valid = qi < J.q_end;
     int64_t n59 = valid ? n53_at(J, qi) : 0;
+    n59 = mod_MOD((uint64_t)n59 + (uint64_t)(local % A.parts * steps) * (uint64_t)S59);
 
-    for (int j = 0; j < J59; j++) {
+    for (int j = 0; j < steps; j++) {
       uint32_t acc[20];
 #pragma unroll
       for (int i = 0; i < 20; i++) acc[i] = valid ? FULL : 0u;
