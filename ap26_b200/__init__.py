@@ -224,8 +224,15 @@ def list_variants():
              "tail_group": o.tail_group} for o in arr]
 
 
+# Reports as the library writes them (struct AP).  Output arrays are left
+# uninitialised: the library fills what it counts, and zeroing room for 2^20
+# reports takes longer than reading them back.
+_AP = np.dtype([("k", np.int32), ("K", np.int32), ("first", np.int64), ("n", np.int64)])
+assert _AP.itemsize == ctypes.sizeof(AP)
+
+
 def _aps_to_list(arr, n):
-    return [(arr[i].k, arr[i].K, arr[i].first, arr[i].n) for i in range(n)]
+    return arr[:n].tolist()
 
 
 # ---- device context ---------------------------------------------------------------
@@ -277,10 +284,10 @@ class Context:
 
     def search_k(self, K, shift=0, cap=1 << 16):
         """Raw reports [(k, K, first, n)] of one K, AVX2 order, and stats."""
-        out = (AP * cap)()
+        out = np.empty(cap, _AP)
         n = ctypes.c_int(0)
         st = Stats()
-        self._check(lib.ap26_search_k(self.h, int(K), int(shift), out, cap, ctypes.byref(n),
+        self._check(lib.ap26_search_k(self.h, int(K), int(shift), _ptr(out), cap, ctypes.byref(n),
                                       ctypes.byref(st)), "ap26_search_k")
         return _aps_to_list(out, n.value), st
 
@@ -317,11 +324,12 @@ class Context:
         """Device-side ReportSolution of raw reports [(k, K, first[, n])]:
         returns (rc, [Final], new result_hash or None).  rc is the first
         non-OK status (the per-report statuses are in the Finals)."""
-        arr = (AP * max(1, len(aps)))(*[AP(int(a[0]), int(a[1]), int(a[2]),
-                                           int(a[3]) if len(a) > 3 else 0) for a in aps])
+        arr = np.zeros(max(1, len(aps)), _AP)
+        arr[:len(aps)] = [(int(a[0]), int(a[1]), int(a[2]), int(a[3]) if len(a) > 3 else 0)
+                          for a in aps]
         fin = (Final * max(1, len(aps)))()
         h = ctypes.c_int32(result_hash or 0)
-        rc = lib.ap26_report_batch(self.h, arr, len(aps), fin,
+        rc = lib.ap26_report_batch(self.h, _ptr(arr), len(aps), fin,
                                    ctypes.byref(h) if result_hash is not None else None, None)
         if rc in (E_CUDA, E_NODEV):
             raise AP26Error(rc, "ap26_report_batch")
@@ -330,7 +338,7 @@ class Context:
     def sprp_bases(self, N, a):
         N = np.ascontiguousarray(N, dtype=np.uint64)
         a = np.ascontiguousarray(a, dtype=np.uint32)
-        v = np.zeros(len(N), np.uint8)
+        v = np.empty(len(N), np.uint8)
         st = Stats()
         self._check(lib.ap26_sprp_bases(self.h, _ptr(N), _ptr(a), len(N), _ptr(v),
                                         ctypes.byref(st)), "ap26_sprp_bases")
@@ -340,19 +348,17 @@ class Context:
         """items: [(id, kmin, kmax, shift)] -> (per-item list of reports, results, stats)."""
         its = (Item * len(items))(*[Item(int(a), int(b), int(c), int(d), 0) for a, b, c, d in items])
         res = (ItemResult * len(items))()
-        aps = (AP * ap_cap)()
+        aps = np.empty(ap_cap, _AP)
         n = ctypes.c_int64(0)
         st = Stats()
-        self._check(lib.ap26_search_batch(self.h, its, len(items), aps, ap_cap, ctypes.byref(n),
-                                          res, ctypes.byref(st)), "ap26_search_batch")
-        per = []
-        for r in res:
-            per.append([(aps[i].k, aps[i].K, aps[i].first, aps[i].n)
-                        for i in range(r.first_ap, r.first_ap + r.n_aps)])
+        self._check(lib.ap26_search_batch(self.h, its, len(items), _ptr(aps), ap_cap,
+                                          ctypes.byref(n), res, ctypes.byref(st)),
+                    "ap26_search_batch")
+        per = [_aps_to_list(aps[r.first_ap:], r.n_aps) for r in res]
         return per, list(res), st
 
     def sieve_range(self, K, shift, q0, q1, cap=1 << 22):
-        cand = np.zeros(cap, np.int64)
+        cand = np.empty(cap, np.int64)
         n = ctypes.c_int64(0)
         st = Stats()
         self._check(lib.ap26_sieve_range(self.h, int(K), int(shift), int(q0), int(q1), _ptr(cand),
@@ -370,7 +376,7 @@ class Context:
 
     def sprp_batch(self, N):
         N = np.ascontiguousarray(N, dtype=np.uint64)
-        v = np.zeros(len(N), np.uint8)
+        v = np.empty(len(N), np.uint8)
         st = Stats()
         self._check(lib.ap26_sprp_batch(self.h, _ptr(N), len(N), _ptr(v), ctypes.byref(st)),
                     "ap26_sprp_batch")
@@ -378,8 +384,8 @@ class Context:
 
     def chain_batch(self, K, n):
         n = np.ascontiguousarray(n, dtype=np.int64)
-        k = np.zeros(len(n), np.int32)
-        f = np.zeros(len(n), np.int64)
+        k = np.empty(len(n), np.int32)
+        f = np.empty(len(n), np.int64)
         st = Stats()
         self._check(lib.ap26_chain_batch(self.h, int(K), _ptr(n), len(n), _ptr(k), _ptr(f),
                                          ctypes.byref(st)), "ap26_chain_batch")
@@ -438,9 +444,9 @@ class Context:
 
     def serve_poll(self, ap_cap=1 << 16):
         res = ItemResult()
-        aps = (AP * ap_cap)()
+        aps = np.empty(ap_cap, _AP)
         n = ctypes.c_int64(0)
-        rc = lib.ap26_serve_poll(self.h, ctypes.byref(res), aps, ap_cap, ctypes.byref(n))
+        rc = lib.ap26_serve_poll(self.h, ctypes.byref(res), _ptr(aps), ap_cap, ctypes.byref(n))
         if rc < 0:
             raise AP26Error(rc, "ap26_serve_poll")
         if rc == 0:

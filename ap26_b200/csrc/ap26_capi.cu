@@ -7,14 +7,19 @@
 // stream (optionally replayed from a CUDA graph), one D2H of the raw reports.
 #include <cuda_runtime.h>
 #include <algorithm>
+#include <atomic>
 #include <chrono>
+#include <condition_variable>
 #include <cstddef>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
 #include <deque>
+#include <functional>
+#include <initializer_list>
 #include <string>
 #include <mutex>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -136,8 +141,9 @@ __global__ void int_probe_kernel(int iters, unsigned *sink) {
 }
 
 // ---- PRP microbenchmark kernel: verdicts of sprp2 over an array ----------------
+// The squarings go to squarings[warp of the grid], or added to *squarings.
 __global__ void sprp_batch_kernel(const uint64_t *N, long long count, uint8_t *verdict,
-                                  unsigned long long *squarings) {
+                                  unsigned long long *squarings, int per_warp) {
   unsigned sq = 0;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < count;
        i += (long long)gridDim.x * blockDim.x) {
@@ -146,7 +152,10 @@ __global__ void sprp_batch_kernel(const uint64_t *N, long long count, uint8_t *v
   }
   unsigned v = sq;
   for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
-  if ((threadIdx.x & 31) == 0 && v) atomicAdd(squarings, (unsigned long long)v);
+  if ((threadIdx.x & 31) == 0) {
+    if (per_warp) squarings[(blockIdx.x * blockDim.x + threadIdx.x) >> 5] = v;
+    else if (v) atomicAdd(squarings, (unsigned long long)v);
+  }
 }
 
 // strong_prp(a, N) for explicit (N, a) pairs, a in [2, 31].
@@ -164,10 +173,9 @@ __global__ void sprp_bases_kernel(const uint64_t *N, const uint32_t *a, long lon
 }
 
 // Chain walk for explicit candidates (kernel-level parity entry point).
-__global__ void chain_explicit_kernel(const KJob *job, const int64_t *n, long long count,
+__global__ void chain_explicit_kernel(int64_t S, const int64_t *n, long long count,
                                       int32_t *k_out, int64_t *first_out, DevState *st) {
   unsigned tests = 0, sq = 0;
-  const int64_t S = job->STEP;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < count;
        i += (long long)gridDim.x * blockDim.x) {
     int k = 0;
@@ -212,6 +220,26 @@ static cudaError_t upload_constants() {
   if ((e = cudaMemcpyToSymbol(c_task, task, sizeof(task))) != cudaSuccess) return e;
   if ((e = cudaMemcpyToSymbol(c_dense_str, str, sizeof(str))) != cudaSuccess) return e;
   return cudaMemcpyToSymbol(c_slot_base, slot, sizeof(slot));
+}
+
+// ap26_sieve_range: one job's descriptor and a fresh run state, in one launch.
+__global__ void range_init_kernel(KJob job, KJob *jobs, DevState *st, unsigned long long tiles,
+                                  unsigned long long *job_counts) {
+  jobs[0] = job;
+  memset(st, 0, sizeof(*st));
+  st->tile_end = tiles;
+  job_counts[0] = 0;
+}
+
+// Candidates [begin, begin + most) of the ring as plain n, and the run state.
+__global__ void range_pack_kernel(const Cand *cand, const DevState *st, long long cand_cap,
+                                  long long begin, long long most, int64_t *out,
+                                  DevState *st_out) {
+  const long long n = min((long long)st->cand_count[0], cand_cap) - begin;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < min(n, most);
+       i += (long long)gridDim.x * blockDim.x)
+    out[i] = cand[begin + i].n;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *st_out = *st;
 }
 
 // Argument blocks are only built through these, so no field can be left
@@ -452,6 +480,97 @@ struct Slice {
   int rc = AP26_OK;
 };
 
+// Staging of the kernel-level entry points: sets of pinned host buffers with
+// their device counterparts, used in turn by a call's slices, and a copy
+// stream for each of a call's host threads.  Allocated with the context (the
+// first set) or with the first call that needs them, freed with the context.
+constexpr int kSets = 3;
+constexpr int kTeam = 8;                        // host threads of a call, at most
+constexpr int64_t kSetBytes = 8 << 20;          // in, and out, per set
+constexpr int64_t kZeroCopyBytes = 1 << 20;     // up to here kernels use the pinned buffers
+constexpr int64_t kThreadBytes = 512 << 10;     // a thread copies at least this much
+struct StageSet {
+  char *h_in = nullptr, *h_out = nullptr, *d_in = nullptr, *d_out = nullptr;
+  cudaEvent_t k0 = nullptr, k1 = nullptr, back = nullptr;   // kernel, results copied back
+  cudaEvent_t in[kTeam] = {};                               // each thread's part copied
+};
+
+// One array of a call: an element of it per value.
+struct Column {
+  char *p;
+  int64_t size;
+};
+
+// The host threads of staged calls: started with the first call that wants
+// them (starting one takes 20-30 us, as long as a short call), asleep between
+// calls, ended with the context.  One call at a time uses them.
+class Team {
+ public:
+  ~Team() {
+    {
+      std::lock_guard<std::mutex> lock(mu_);
+      stop_ = true;
+    }
+    wake_.notify_all();
+    for (std::thread &t : threads_) t.join();
+  }
+  // Threads a call can have, itself included: `wanted`, or fewer where no more start.
+  int size(int wanted) {
+    try {
+      while ((int)threads_.size() + 1 < wanted) {
+        const int i = (int)threads_.size() + 1;
+        threads_.emplace_back([this, i] { loop(i); });
+      }
+    } catch (const std::system_error &) {
+    } catch (const std::bad_alloc &) {
+    }
+    return std::min(wanted, (int)threads_.size() + 1);
+  }
+  // f(0) here and f(1) .. f(n - 1) in the other threads, n <= size().
+  void run(int n, const std::function<void(int)> &f) {
+    if (n > 1) {
+      std::lock_guard<std::mutex> lock(mu_);
+      job_ = &f;
+      n_ = n;
+      left_ = n - 1;
+      call_++;
+      wake_.notify_all();
+    }
+    f(0);
+    if (n > 1) {
+      std::unique_lock<std::mutex> lock(mu_);
+      done_.wait(lock, [this] { return left_ == 0; });
+      job_ = nullptr;
+    }
+  }
+
+ private:
+  void loop(int i) {
+    unsigned long long seen = 0;
+    for (;;) {
+      const std::function<void(int)> *f = nullptr;
+      {
+        std::unique_lock<std::mutex> lock(mu_);
+        wake_.wait(lock, [&] { return stop_ || call_ != seen; });
+        if (stop_) return;
+        seen = call_;
+        if (i >= n_ || !job_) continue;
+        f = job_;
+      }
+      (*f)(i);
+      std::lock_guard<std::mutex> lock(mu_);
+      if (--left_ == 0) done_.notify_one();
+    }
+  }
+  std::vector<std::thread> threads_;
+  std::mutex mu_;
+  std::condition_variable wake_, done_;
+  const std::function<void(int)> *job_ = nullptr;
+  int n_ = 0, left_ = 0;
+  unsigned long long call_ = 0;
+  bool stop_ = false;
+};
+
 struct ap26_ctx {
   int device = 0;
   ap26_opts opts{};
@@ -482,6 +601,11 @@ struct ap26_ctx {
   int64_t serve_budget = 0;                    // pool + fixed serving buffers
   UnitState *d_units = nullptr;                // kUnitSlots serving-unit states
   std::vector<int> free_slots;
+  StageSet sets[kSets];
+  Team team;
+  cudaStream_t copy_in[kTeam] = {};            // one thread's copies each
+  cudaStream_t back_stream = nullptr;          // results
+  unsigned long long *d_tally = nullptr;       // squarings of an ap26_sprp_batch call
   std::string last_error;
   bool pending = false;        // a call timed out with its work still queued
 };
@@ -508,19 +632,168 @@ static int cuda_fail(ap26_ctx *ctx, cudaError_t e, const char *what) {
 
 constexpr int kChainThreads = 256;   // chain_kernel block size
 
-// Device buffer owned by one call of a kernel-level entry point: freed on
-// every return path, the early CUDA-error returns of CK included.
-template <typename T>
-struct DevBuf {
-  T *p = nullptr;
-  DevBuf() = default;
-  DevBuf(const DevBuf &) = delete;
-  DevBuf &operator=(const DevBuf &) = delete;
-  ~DevBuf() {
-    if (p) cudaFree(p);
+static cudaError_t stage_ensure(ap26_ctx *ctx, int sets, int team) {
+  cudaError_t e = cudaSuccess;
+  const auto event = [&](cudaEvent_t &v, unsigned flags) {
+    if (e == cudaSuccess && !v) e = cudaEventCreateWithFlags(&v, flags);
+  };
+  const auto stream = [&](cudaStream_t &v) {
+    if (e == cudaSuccess && !v) e = cudaStreamCreateWithFlags(&v, cudaStreamNonBlocking);
+  };
+  for (int i = 0; i < sets; i++) {
+    StageSet &G = ctx->sets[i];
+    event(G.k0, cudaEventDefault);
+    event(G.k1, cudaEventDefault);
+    event(G.back, cudaEventDisableTiming);
+    for (int t = 0; t < kTeam; t++) event(G.in[t], cudaEventDisableTiming);
+    if (e == cudaSuccess && !G.h_in) e = cudaMallocHost(&G.h_in, kSetBytes);
+    if (e == cudaSuccess && !G.h_out) e = cudaMallocHost(&G.h_out, kSetBytes);
+    if (e == cudaSuccess && !G.d_in) e = cudaMalloc(&G.d_in, kSetBytes);
+    if (e == cudaSuccess && !G.d_out) e = cudaMalloc(&G.d_out, kSetBytes);
   }
-  cudaError_t alloc(size_t n) { return cudaMalloc(&p, sizeof(T) * n); }
-};
+  for (int t = 0; t < team; t++) stream(ctx->copy_in[t]);
+  stream(ctx->back_stream);
+  return e;
+}
+
+static void stage_free(ap26_ctx *ctx) {
+  for (cudaStream_t v : ctx->copy_in)
+    if (v) cudaStreamSynchronize(v);
+  if (ctx->back_stream) cudaStreamSynchronize(ctx->back_stream);
+  for (StageSet &G : ctx->sets) {
+    cudaFree(G.d_in);
+    cudaFree(G.d_out);
+    cudaFreeHost(G.h_in);
+    cudaFreeHost(G.h_out);
+    for (cudaEvent_t v : {G.k0, G.k1, G.back})
+      if (v) cudaEventDestroy(v);
+    for (cudaEvent_t v : G.in)
+      if (v) cudaEventDestroy(v);
+  }
+  for (cudaStream_t v : ctx->copy_in)
+    if (v) cudaStreamDestroy(v);
+  if (ctx->back_stream) cudaStreamDestroy(ctx->back_stream);
+}
+
+// Runs `count` values, given in the arrays `in`, through a kernel that fills
+// the arrays `out`.  launch(n, in, out, stream) starts it on n values, whose
+// arrays lie one after the other in its buffers.  Kernels run in ctx->stream,
+// behind whatever is queued there; *ms is the sum of their times.  Returns
+// once all is done.
+//
+// The time of a long call is its copies: ap26_sprp_batch of 2^24 values spent
+// 16 of 18.4 ms in one thread's pageable copies and in allocations.  Here its
+// slices go through kSets sets of buffers, each slice filled and emptied by
+// up to kTeam threads, so that copies, transfers both ways and kernels
+// overlap.  The time of a short call is its number of driver calls: it has
+// one launch and one wait, and the kernel reaches the pinned buffers itself
+// (61 values 62 us, now 32).
+template <class Launch>
+static int staged(ap26_ctx *ctx, int64_t count, std::initializer_list<Column> in,
+                  std::initializer_list<Column> out, double *ms, const Launch &launch) {
+  int64_t in_per = 0, out_per = 0;
+  for (const Column &c : in) in_per += c.size;
+  for (const Column &c : out) out_per += c.size;
+  const int64_t per = std::max(in_per, out_per);
+  *ms = 0;
+  // part [from, to) of a slice of n values that starts with value `first`
+  const auto fill = [&](char *buf, int64_t first, int64_t n, int64_t from, int64_t to) {
+    for (const Column &c : in) {
+      memcpy(buf + from * c.size, c.p + (first + from) * c.size, (size_t)((to - from) * c.size));
+      buf += n * c.size;
+    }
+  };
+  const auto empty = [&](const char *buf, int64_t first, int64_t n, int64_t from, int64_t to) {
+    for (const Column &c : out) {
+      memcpy(c.p + (first + from) * c.size, buf + from * c.size, (size_t)((to - from) * c.size));
+      buf += n * c.size;
+    }
+  };
+  if (count * per <= kZeroCopyBytes) {
+    StageSet &G = ctx->sets[0];
+    fill(G.h_in, 0, count, 0, count);
+    CK(cudaEventRecord(G.k0, ctx->stream));
+    CK(launch(count, G.h_in, G.h_out, ctx->stream));
+    CK(cudaEventRecord(G.k1, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    float t = 0;
+    cudaEventElapsedTime(&t, G.k0, G.k1);
+    *ms = t;
+    empty(G.h_out, 0, count, 0, count);
+    return AP26_OK;
+  }
+  const int64_t slice = kSetBytes / per, slices = (count + slice - 1) / slice;
+  const int team = ctx->team.size((int)std::max<int64_t>(
+      1, std::min<int64_t>({(int64_t)kTeam, (int64_t)std::thread::hardware_concurrency(),
+                            count * (in_per + out_per) / kThreadBytes})));
+  CK(stage_ensure(ctx, (int)std::min<int64_t>(slices, kSets), team));
+  std::vector<std::atomic<int>> filled((size_t)slices);   // threads done with a slice's copies
+  std::atomic<int> failed{0};
+  double total = 0;
+  const auto work = [&](int t) {
+    cudaError_t e = cudaSetDevice(ctx->device);
+    const auto ok = [&](cudaError_t r) {
+      if (e == cudaSuccess) e = r;
+      return e == cudaSuccess;
+    };
+    const auto part = [&](int64_t n, int k) { return n * k / team; };
+    // slice i's results, this thread's part
+    const auto take = [&](int64_t i) {
+      StageSet &G = ctx->sets[i % kSets];
+      // its kernel is launched by whoever fills it last
+      while (filled[(size_t)i].load() < team + 1)
+        if (failed.load()) return;
+      if (!ok(cudaEventSynchronize(G.back))) return;
+      if (t == 0) {
+        float ms1 = 0;
+        cudaEventElapsedTime(&ms1, G.k0, G.k1);
+        total += ms1;
+      }
+      const int64_t first = i * slice, n = std::min(slice, count - first);
+      empty(G.h_out, first, n, part(n, t), part(n, t + 1));
+    };
+    for (int64_t i = 0; i < slices && e == cudaSuccess && !failed.load(); i++) {
+      StageSet &G = ctx->sets[i % kSets];
+      if (i >= kSets) take(i - kSets);
+      if (e != cudaSuccess || failed.load()) break;
+      const int64_t first = i * slice, n = std::min(slice, count - first);
+      const int64_t from = part(n, t), to = part(n, t + 1);
+      fill(G.h_in, first, n, from, to);
+      int64_t at = 0;
+      for (const Column &c : in) {
+        ok(cudaMemcpyAsync(G.d_in + at + from * c.size, G.h_in + at + from * c.size,
+                           (size_t)((to - from) * c.size), cudaMemcpyHostToDevice, ctx->copy_in[t]));
+        at += n * c.size;
+      }
+      ok(cudaEventRecord(G.in[t], ctx->copy_in[t]));
+      if (e != cudaSuccess) break;
+      if (filled[(size_t)i].fetch_add(1) != team - 1) continue;
+      // the last thread to fill the slice starts its kernel
+      for (int k = 0; k < team; k++) ok(cudaStreamWaitEvent(ctx->stream, G.in[k], 0));
+      ok(cudaEventRecord(G.k0, ctx->stream));
+      if (e == cudaSuccess) ok(launch(n, G.d_in, G.d_out, ctx->stream));
+      ok(cudaEventRecord(G.k1, ctx->stream));
+      ok(cudaStreamWaitEvent(ctx->back_stream, G.k1, 0));
+      ok(cudaMemcpyAsync(G.h_out, G.d_out, (size_t)(n * out_per), cudaMemcpyDeviceToHost,
+                         ctx->back_stream));
+      ok(cudaEventRecord(G.back, ctx->back_stream));
+      if (e == cudaSuccess) filled[(size_t)i].fetch_add(1);
+    }
+    for (int64_t i = std::max<int64_t>(0, slices - kSets);
+         i < slices && e == cudaSuccess && !failed.load(); i++)
+      take(i);
+    if (e != cudaSuccess) failed.store((int)e);
+  };
+  ctx->team.run(team, work);
+  *ms = total;
+  if (failed.load()) {
+    // nothing may still write the buffers when the next call reuses them
+    cudaStreamSynchronize(ctx->stream);
+    cudaStreamSynchronize(ctx->back_stream);
+    return cuda_fail(ctx, (cudaError_t)failed.load(), "staged call");
+  }
+  return AP26_OK;
+}
 
 extern "C" int ap26_version(void) { return 10100; }
 
@@ -693,6 +966,8 @@ extern "C" int ap26_create(int device, const ap26_opts *opts, ap26_ctx **out) {
     CKC(cudaFuncSetAttribute(class_sieve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              CLASS_SMEM));
     CKC(cudaMalloc(&ctx->d_plan, sizeof(ClassPlan)));
+    CKC(cudaMalloc(&ctx->d_tally, sizeof(unsigned long long)));
+    CKC(stage_ensure(ctx, 1, 1));
     // buffers
     if (ctx->opts.cand_ring_log2 < 12 || ctx->opts.cand_ring_log2 > 27 ||
         ctx->opts.batch_wave > kMaxBatchWave) {
@@ -736,6 +1011,8 @@ extern "C" void ap26_destroy(ap26_ctx *ctx) {
   cudaFree(ctx->d_units);
   cudaFree(ctx->d_pool);
   cudaFree(ctx->d_plan);
+  cudaFree(ctx->d_tally);
+  stage_free(ctx);
   cudaFree(ctx->d_cand[0]); cudaFree(ctx->d_cand[1]);
   for (int r = 0; r < 2; r++) {
     if (ctx->sieve_done[r]) cudaEventDestroy(ctx->sieve_done[r]);
@@ -812,7 +1089,8 @@ static bool k_in_domain(int K, int shift) {
   return K >= 1 && K <= AP26_KMAX_SAFE && shift >= 0 && shift <= AP26_SHIFT_MAX;
 }
 
-// Bounded host wait on an event: polls it, gives up after timeout_s.
+// Bounded host wait on an event: polls it, without sleeping for the first
+// millisecond (a sleep takes at least 50 us), and gives up after timeout_s.
 static int wait_event(ap26_ctx *ctx, cudaEvent_t e, double timeout_s) {
   auto t0 = std::chrono::steady_clock::now();
   for (;;) {
@@ -825,7 +1103,8 @@ static int wait_event(ap26_ctx *ctx, cudaEvent_t e, double timeout_s) {
       ctx->pending = true;
       return AP26_E_TIMEOUT;
     }
-    std::this_thread::sleep_for(std::chrono::microseconds(el < 0.01 ? 20 : 200));
+    if (el > 0.001)
+      std::this_thread::sleep_for(std::chrono::microseconds(el < 0.01 ? 20 : 200));
   }
 }
 
@@ -1738,22 +2017,20 @@ extern "C" int ap26_sieve_range(ap26_ctx *ctx, int K, int shift, int64_t q_begin
   J.ntiles = (int32_t)tiles;
   J.tile_begin = 0;
   J.table = 0;
-  memset(S.h_st, 0, sizeof(DevState));
-  S.h_st->chunk_size = (unsigned long long)std::max<int64_t>(1, tiles);
-  S.h_st->total_tiles = (unsigned long long)tiles;
   cudaStream_t s = ctx->stream;
   const SieveVariant &V = kVariants[ctx->variant];
+  StageSet &G = ctx->sets[0];
+  const long long most = kSetBytes / (long long)sizeof(int64_t);
   CK(cudaEventRecord(ctx->ev0, s));
-  CK(cudaMemcpyAsync(S.d_jobs, S.h_jobs, sizeof(KJob), cudaMemcpyHostToDevice, s));
-  CK(cudaMemcpyAsync(S.d_st, S.h_st, sizeof(DevState), cudaMemcpyHostToDevice, s));
-  CK(cudaMemsetAsync(S.d_job_counts, 0, sizeof(unsigned long long), s));
+  range_init_kernel<<<1, 1, 0, s>>>(J, S.d_jobs, S.d_st, (unsigned long long)tiles, S.d_job_counts);
   launch_setup(S.d_jobs, 1, S.d_tables, TABLE_WORDS, s);
-  chunk_begin_kernel<<<1, 1, 0, s>>>(S.d_st, 0);
   const SieveArgs sa = sieve_args(S.d_jobs, 1, S.d_tables, S.d_st, ctx->d_cand[0],
                                   ctx->cand_cap, S.d_job_counts, 0, &S.d_st->cand_count[0], parts);
   V.kernel<<<ctx->sieve_blocks, V.WARPS * 32, V.smem(), s>>>(sa);
+  // the candidates go straight to pinned memory, a buffer of them at a time
+  range_pack_kernel<<<ctx->num_sms, 256, 0, s>>>(ctx->d_cand[0], S.d_st, ctx->cand_cap, 0, most,
+                                                 (int64_t *)G.h_out, S.h_st);
   CK(cudaGetLastError());
-  CK(cudaMemcpyAsync(S.h_st, S.d_st, sizeof(DevState), cudaMemcpyDeviceToHost, s));
   CK(cudaEventRecord(ctx->ev1, s));
   rc = wait_event(ctx, ctx->ev1, ctx->opts.wait_timeout_s);
   if (rc != AP26_OK) return rc;
@@ -1761,10 +2038,15 @@ extern "C" int ap26_sieve_range(ap26_ctx *ctx, int K, int shift, int64_t q_begin
   *n_cand = nc;
   if (nc > ctx->cand_cap) return AP26_E_OVERFLOW;
   if (nc > cap) return AP26_E_CAPACITY;
-  if (nc > 0) {
-    std::vector<Cand> tmp(nc);
-    CK(cudaMemcpy(tmp.data(), ctx->d_cand[0], sizeof(Cand) * nc, cudaMemcpyDeviceToHost));
-    for (long long i = 0; i < nc; i++) cand[i] = tmp[i].n;
+  for (long long at = 0; at < nc; at += most) {
+    const long long n = std::min(most, nc - at);
+    if (at > 0) {
+      range_pack_kernel<<<ctx->num_sms, 256, 0, s>>>(ctx->d_cand[0], S.d_st, ctx->cand_cap, at,
+                                                     most, (int64_t *)G.h_out, S.h_st);
+      CK(cudaGetLastError());
+      CK(cudaStreamSynchronize(s));
+    }
+    memcpy(cand + at, G.h_out, sizeof(int64_t) * n);
   }
   if (stats) {
     float ms = 0;
@@ -1774,7 +2056,7 @@ extern "C" int ap26_sieve_range(ap26_ctx *ctx, int K, int shift, int64_t q_begin
     stats->late_items = (int64_t)S.h_st->late_items;
     stats->device_ms = ms;
     stats->error_flags = (int32_t)S.h_st->err_flags;
-    stats->launches = 3;
+    stats->launches = 4;
   }
   return AP26_OK;
 }
@@ -1806,26 +2088,30 @@ extern "C" int ap26_sprp_batch(ap26_ctx *ctx, const uint64_t *N, int64_t count, 
                                ap26_stats *stats) {
   if (!ctx || !N || !verdict || count < 0) return AP26_E_ARG;
   CK(cudaSetDevice(ctx->device));
+  drain(ctx);
   if (count == 0) return AP26_OK;
-  DevBuf<uint64_t> dN;
-  DevBuf<uint8_t> dV;
-  DevBuf<unsigned long long> dsq;
+  // a short call's warps leave their counts behind the verdicts
+  const bool small = count * (int64_t)sizeof(uint64_t) <= kZeroCopyBytes;
+  const int64_t warps = std::min<int64_t>((count + 63) / 64, ctx->num_sms * 16) * 2;
+  unsigned long long *const tally =
+      small ? (unsigned long long *)(ctx->sets[0].h_out + kZeroCopyBytes) : ctx->d_tally;
+  if (!small) CK(cudaMemsetAsync(ctx->d_tally, 0, sizeof(*ctx->d_tally), ctx->stream));
+  double ms = 0;
+  int rc = staged(
+      ctx, count, {{(char *)N, sizeof(uint64_t)}}, {{(char *)verdict, 1}}, &ms,
+      [&](int64_t n, const char *in, char *out, cudaStream_t s) {
+        const int block = small ? 64 : 256;
+        const int64_t blocks = std::min<int64_t>((n + block - 1) / block, ctx->num_sms * 16);
+        sprp_batch_kernel<<<(int)blocks, block, 0, s>>>((const uint64_t *)in, n, (uint8_t *)out,
+                                                        tally, small);
+        return cudaGetLastError();
+      });
+  if (rc != AP26_OK) return rc;
   unsigned long long hsq = 0;
-  CK(dN.alloc(count));
-  CK(dV.alloc(count));
-  CK(dsq.alloc(1));
-  cudaStream_t s = ctx->stream;
-  CK(cudaMemsetAsync(dsq.p, 0, sizeof(unsigned long long), s));
-  CK(cudaMemcpyAsync(dN.p, N, sizeof(uint64_t) * count, cudaMemcpyHostToDevice, s));
-  CK(cudaEventRecord(ctx->ev0, s));
-  sprp_batch_kernel<<<ctx->num_sms * 16, 256, 0, s>>>(dN.p, count, dV.p, dsq.p);
-  CK(cudaGetLastError());
-  CK(cudaEventRecord(ctx->ev1, s));
-  CK(cudaMemcpyAsync(verdict, dV.p, count, cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(&hsq, dsq.p, sizeof(hsq), cudaMemcpyDeviceToHost, s));
-  CK(cudaStreamSynchronize(s));
-  float ms = 0;
-  cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
+  if (small)
+    for (int64_t w = 0; w < warps; w++) hsq += tally[w];
+  else
+    CK(cudaMemcpy(&hsq, ctx->d_tally, sizeof(hsq), cudaMemcpyDeviceToHost));
   if (stats) {
     memset(stats, 0, sizeof(*stats));
     stats->prp_tests = count;
@@ -1839,27 +2125,24 @@ extern "C" int ap26_sprp_batch(ap26_ctx *ctx, const uint64_t *N, int64_t count, 
 extern "C" int ap26_sprp_bases(ap26_ctx *ctx, const uint64_t *N, const uint32_t *a,
                                int64_t count, uint8_t *verdict, ap26_stats *stats) {
   if (!ctx || count < 0 || (count > 0 && (!N || !a || !verdict))) return AP26_E_ARG;
-  for (int64_t i = 0; i < count; i++)
-    if (a[i] < 2 || a[i] > 31) return AP26_E_ARG;
+  uint32_t outside = 0;
+  for (int64_t i = 0; i < count; i++) outside |= (uint32_t)(a[i] - 2u > 29u);
+  if (outside) return AP26_E_ARG;
   CK(cudaSetDevice(ctx->device));
   if (count == 0) return AP26_OK;
-  DevBuf<uint64_t> dN;
-  DevBuf<uint32_t> dA;
-  DevBuf<uint8_t> dV;
-  CK(dN.alloc(count));
-  CK(dA.alloc(count));
-  CK(dV.alloc(count));
-  cudaStream_t s = ctx->stream;
-  CK(cudaMemcpyAsync(dN.p, N, sizeof(uint64_t) * count, cudaMemcpyHostToDevice, s));
-  CK(cudaMemcpyAsync(dA.p, a, sizeof(uint32_t) * count, cudaMemcpyHostToDevice, s));
-  CK(cudaEventRecord(ctx->ev0, s));
-  sprp_bases_kernel<<<ctx->num_sms * 16, 256, 0, s>>>(dN.p, dA.p, count, dV.p);
-  CK(cudaGetLastError());
-  CK(cudaEventRecord(ctx->ev1, s));
-  CK(cudaMemcpyAsync(verdict, dV.p, count, cudaMemcpyDeviceToHost, s));
-  CK(cudaStreamSynchronize(s));
-  float ms = 0;
-  cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
+  drain(ctx);
+  double ms = 0;
+  int rc = staged(
+      ctx, count, {{(char *)N, sizeof(uint64_t)}, {(char *)a, sizeof(uint32_t)}},
+      {{(char *)verdict, 1}}, &ms,
+      [&](int64_t n, const char *in, char *out, cudaStream_t s) {
+        const int64_t blocks = std::min<int64_t>((n + 63) / 64, ctx->num_sms * 32);
+        sprp_bases_kernel<<<(int)blocks, 64, 0, s>>>(
+            (const uint64_t *)in, (const uint32_t *)(in + sizeof(uint64_t) * n), n,
+            (uint8_t *)out);
+        return cudaGetLastError();
+      });
+  if (rc != AP26_OK) return rc;
   if (stats) {
     memset(stats, 0, sizeof(*stats));
     stats->prp_tests = count;
@@ -1876,29 +2159,25 @@ extern "C" int ap26_report_batch(ap26_ctx *ctx, const ap26_ap *raw, int64_t n, a
   CK(cudaSetDevice(ctx->device));
   if (stats) memset(stats, 0, sizeof(*stats));
   if (n == 0) return AP26_OK;
-  DevBuf<APRec> dR;
-  DevBuf<FinRec> dF;
-  CK(dR.alloc(n));
-  CK(dF.alloc(n));
-  cudaStream_t s = ctx->stream;
-  // ap26_ap and APRec share a layout; with jobs == null the job field is K
-  CK(cudaMemcpyAsync(dR.p, raw, sizeof(APRec) * n, cudaMemcpyHostToDevice, s));
-  CK(cudaEventRecord(ctx->ev0, s));
-  ReportArgs ra;
-  ra.aps = dR.p;
-  ra.count = nullptr;
-  ra.n = n;
-  ra.jobs = nullptr;
-  ra.fin = dF.p;
-  ra.job_hash = nullptr;
-  const long long want = (n + REPORT_WARPS - 1) / REPORT_WARPS;
-  report_kernel<<<(int)std::min<long long>(want, ctx->num_sms * 8), REPORT_WARPS * 32, 0, s>>>(ra);
-  CK(cudaGetLastError());
-  CK(cudaEventRecord(ctx->ev1, s));
-  CK(cudaMemcpyAsync(out, dF.p, sizeof(FinRec) * n, cudaMemcpyDeviceToHost, s));
-  CK(cudaStreamSynchronize(s));
-  float ms = 0;
-  cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
+  drain(ctx);
+  double ms = 0;
+  int rc = staged(
+      ctx, n, {{(char *)raw, sizeof(APRec)}}, {{(char *)out, sizeof(FinRec)}}, &ms,
+      [&](int64_t m, const char *in, char *fin, cudaStream_t s) {
+        // ap26_ap and APRec share a layout; with jobs == null the job field is K
+        ReportArgs ra;
+        ra.aps = (const APRec *)in;
+        ra.count = nullptr;
+        ra.n = m;
+        ra.jobs = nullptr;
+        ra.fin = (FinRec *)fin;
+        ra.job_hash = nullptr;
+        const int64_t want = (m + REPORT_WARPS - 1) / REPORT_WARPS;
+        report_kernel<<<(int)std::min<int64_t>(want, ctx->num_sms * 8), REPORT_WARPS * 32, 0, s>>>(
+            ra);
+        return cudaGetLastError();
+      });
+  if (rc != AP26_OK) return rc;
   if (stats) {
     stats->aps = n;
     stats->device_ms = ms;
@@ -1921,36 +2200,24 @@ extern "C" int ap26_chain_batch(ap26_ctx *ctx, int K, const int64_t *n, int64_t 
   drain(ctx);
   if (count == 0) return AP26_OK;
   JobSet &S = ctx->main;
-  int rc;
-  if ((rc = jobset_ensure(ctx, S, 1)) != AP26_OK) return rc;
-  fill_job(S.h_jobs[0], K, 0, 0, 0, 0);
-  DevBuf<int64_t> dn, df;
-  DevBuf<int32_t> dk;
-  CK(dn.alloc(count));
-  CK(df.alloc(count));
-  CK(dk.alloc(count));
-  cudaStream_t s = ctx->stream;
-  memset(S.h_st, 0, sizeof(DevState));
-  CK(cudaMemcpyAsync(S.d_jobs, S.h_jobs, sizeof(KJob), cudaMemcpyHostToDevice, s));
-  CK(cudaMemcpyAsync(S.d_st, S.h_st, sizeof(DevState), cudaMemcpyHostToDevice, s));
-  launch_setup(S.d_jobs, 1, S.d_tables, 0, s);
-  CK(cudaMemcpyAsync(dn.p, n, sizeof(int64_t) * count, cudaMemcpyHostToDevice, s));
-  CK(cudaEventRecord(ctx->ev0, s));
-  chain_explicit_kernel<<<ctx->num_sms * 8, 128, 0, s>>>(S.d_jobs, dn.p, count, dk.p, df.p,
-                                                         S.d_st);
-  CK(cudaGetLastError());
-  CK(cudaEventRecord(ctx->ev1, s));
-  CK(cudaMemcpyAsync(k_out, dk.p, sizeof(int32_t) * count, cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(first_out, df.p, sizeof(int64_t) * count, cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(S.h_st, S.d_st, sizeof(DevState), cudaMemcpyDeviceToHost, s));
-  CK(cudaStreamSynchronize(s));
-  float ms = 0;
-  cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
+  memset(S.h_st, 0, sizeof(DevState));     // pinned: the kernel sets its error flags there
+  double ms = 0;
+  int rc = staged(
+      ctx, count, {{(char *)n, sizeof(int64_t)}},
+      {{(char *)first_out, sizeof(int64_t)}, {(char *)k_out, sizeof(int32_t)}}, &ms,
+      [&](int64_t m, const char *in, char *out, cudaStream_t s) {
+        const int64_t blocks = std::min<int64_t>((m + 63) / 64, ctx->num_sms * 16);
+        chain_explicit_kernel<<<(int)blocks, 64, 0, s>>>(
+            (int64_t)K * PRIM23, (const int64_t *)in, m, (int32_t *)(out + sizeof(int64_t) * m),
+            (int64_t *)out, S.h_st);
+        return cudaGetLastError();
+      });
+  if (rc != AP26_OK) return rc;
   if (stats) {
     memset(stats, 0, sizeof(*stats));
     stats->device_ms = ms;
     stats->error_flags = (int32_t)S.h_st->err_flags;
-    stats->launches = 2;
+    stats->launches = 1;
   }
   return (S.h_st->err_flags & ERR_DOMAIN) ? AP26_E_DOMAIN : AP26_OK;
 }
@@ -1959,15 +2226,14 @@ extern "C" int ap26_probe_peaks(ap26_ctx *ctx, double *smem_gbs, double *int_top
   if (!ctx) return AP26_E_ARG;
   CK(cudaSetDevice(ctx->device));
   drain(ctx);
-  DevBuf<unsigned> sink;
-  CK(sink.alloc(1));
+  unsigned *const sink = (unsigned *)ctx->d_tally;
   cudaStream_t s = ctx->stream;
   const int blocks = ctx->num_sms * 4, threads = 256;
   const int siters = 4096, iiters = 4096;
   float ms = 0;
   for (int rep = 0; rep < 2; rep++) {
     CK(cudaEventRecord(ctx->ev0, s));
-    smem_probe_kernel<<<blocks, threads, 0, s>>>(siters, sink.p);
+    smem_probe_kernel<<<blocks, threads, 0, s>>>(siters, sink);
     CK(cudaGetLastError());
     CK(cudaEventRecord(ctx->ev1, s));
     CK(cudaEventSynchronize(ctx->ev1));
@@ -1976,7 +2242,7 @@ extern "C" int ap26_probe_peaks(ap26_ctx *ctx, double *smem_gbs, double *int_top
   if (smem_gbs) *smem_gbs = (double)blocks * threads * siters * 8 * 16 / (ms * 1e-3) / 1e9;
   for (int rep = 0; rep < 2; rep++) {
     CK(cudaEventRecord(ctx->ev0, s));
-    int_probe_kernel<<<blocks, threads, 0, s>>>(iiters, sink.p);
+    int_probe_kernel<<<blocks, threads, 0, s>>>(iiters, sink);
     CK(cudaGetLastError());
     CK(cudaEventRecord(ctx->ev1, s));
     CK(cudaEventSynchronize(ctx->ev1));

@@ -1,0 +1,63 @@
+"""The kernel-level calls at the sizes where their paths change: a call of up to 1 MB of values is one kernel on pinned memory, a longer
+one goes through sets of 8 MB in slices, by several host threads.  A long
+call's results are those of short calls on its pieces (which the other files
+check against the oracle and the reference's vectors).
+"""
+import numpy as np
+import pytest
+
+import ap26_b200 as A
+
+pytestmark = pytest.mark.gpu
+
+PIECE = 30_000          # one kernel on pinned memory for every call
+
+
+def _values(rng, n):
+    N = np.exp2(rng.uniform(2, 63, n)).astype(np.uint64)
+    N[:8] = [0, 1, 2, 3, 4, 9, (1 << 63) - 25, 1 << 63]
+    odd = rng.random(n) < 0.95
+    N[odd] |= np.uint64(1)
+    return rng.permutation(N)
+
+
+@pytest.mark.parametrize("n", [1, 31, 131_072, 131_073, 1_048_576, 1_048_577, 4_300_001])
+def test_long_sprp_batches_equal_their_pieces(ctx, n):
+    N = _values(np.random.default_rng(n), max(8, n))[:n]
+    got, st = ctx.sprp_batch(N)
+    parts = [ctx.sprp_batch(N[i:i + PIECE]) for i in range(0, n, PIECE)]
+    assert np.array_equal(got, np.concatenate([v for v, _ in parts]))
+    assert st.late_items == sum(s.late_items for _, s in parts)     # modular squarings
+    assert st.prp_tests == n
+
+
+@pytest.mark.parametrize("n", [87_382, 700_001])
+def test_long_base_batches_equal_their_pieces(ctx, n):
+    rng = np.random.default_rng(n)
+    N, a = _values(rng, n), rng.integers(2, 32, n, dtype=np.uint32)
+    got, _ = ctx.sprp_bases(N, a)
+    assert np.array_equal(got, np.concatenate(
+        [ctx.sprp_bases(N[i:i + PIECE], a[i:i + PIECE])[0] for i in range(0, n, PIECE)]))
+
+
+@pytest.mark.parametrize("n", [87_400, 750_003])
+def test_long_chain_batches_equal_their_pieces(ctx, n):
+    cand, _ = ctx.sieve_range(366384, 0, 0, 40 * 12673)
+    c = np.resize(np.sort(cand), n)
+    k, f, _ = ctx.chain_batch(366384, c)
+    parts = [ctx.chain_batch(366384, c[i:i + PIECE]) for i in range(0, n, PIECE)]
+    assert np.array_equal(k, np.concatenate([p[0] for p in parts]))
+    assert np.array_equal(f, np.concatenate([p[1] for p in parts]))
+
+
+@pytest.mark.parametrize("n", [18_725, 160_001])
+def test_long_report_batches_equal_their_pieces(ctx, n):
+    aps, _ = ctx.search_k(366384, 0)
+    reps = (aps * (n // len(aps) + 1))[:n]
+    rc, fin, h = ctx.report_batch(reps, result_hash=5)
+    one, onefin, _ = ctx.report_batch(aps, result_hash=0)
+    assert rc == one == 0
+    assert all(bytes(f) == bytes(onefin[i % len(aps)]) for i, f in enumerate(fin))
+    total = 5 + sum(onefin[i % len(aps)].hash_add for i in range(n))
+    assert h == (total - 1) % 2_000_000_000 + 1
+
