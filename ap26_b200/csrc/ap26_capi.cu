@@ -29,6 +29,8 @@
 
 namespace ap26 {
 
+constexpr int SPRP_BLOCK = 256;   // sprp_batch_kernel's largest block
+
 // ---- per-job set-up kernel ----------------------------------------------------
 // The reference's per-K constants (src/opencl/AP26.h:112-120, int64 split
 // multiplications).
@@ -141,19 +143,72 @@ __global__ void int_probe_kernel(int iters, unsigned *sink) {
 }
 
 // ---- PRP microbenchmark kernel: verdicts of sprp2 over an array ----------------
+// A block sorts its values: those of sprp2's small range and the others wait
+// in a queue each, and a queue is tested when a block's worth waits (the rest
+// at the end), so a warp runs only one form of the test.  With values spread
+// over the logarithm of [2^40, 2^63), of which 13% are not small, both forms
+// in most warps would cost twice the time.  A block takes `take` values at a
+// time; with take = half its threads, both queues' last tests run side by
+// side.
 // The squarings go to squarings[warp of the grid], or added to *squarings.
-__global__ void sprp_batch_kernel(const uint64_t *N, long long count, uint8_t *verdict,
-                                  unsigned long long *squarings, int per_warp) {
+__global__ void __launch_bounds__(SPRP_BLOCK)
+sprp_batch_kernel(const uint64_t *N, long long count, uint8_t *verdict,
+                  unsigned long long *squarings, int per_warp, int take) {
+  __shared__ uint64_t value[2][2 * SPRP_BLOCK];
+  __shared__ uint32_t index[2][2 * SPRP_BLOCK];
+  __shared__ int waiting[2];
+  const int tid = threadIdx.x, lane = tid & 31, block = blockDim.x;
+  if (tid < 2) waiting[tid] = 0;
+  __syncthreads();
   unsigned sq = 0;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < count;
-       i += (long long)gridDim.x * blockDim.x) {
-    const uint64_t n = N[i];
-    verdict[i] = (uint8_t)((n & 1) && n < (1ull << 63) ? sprp2(n, sq) : 0);
+  // takes n0 and n1 values off the queues, the second by whole other warps;
+  // called by all threads
+  auto test = [&](int n0, int n1) {
+    const int second = (n0 + 31) & ~31;
+    if (tid < n0) {
+      const int at = waiting[0] - n0 + tid;
+      verdict[index[0][at]] = (uint8_t)sprp2_as<true>(value[0][at], sq);
+    } else if (tid >= second && tid < second + n1) {
+      const int at = waiting[1] - n1 + tid - second;
+      verdict[index[1][at]] = (uint8_t)sprp2_as<false>(value[1][at], sq);
+    }
+    __syncthreads();
+    if (tid == 0) {
+      waiting[0] -= n0;
+      waiting[1] -= n1;
+    }
+    __syncthreads();
+  };
+  for (long long i0 = blockIdx.x * (long long)take; i0 < count;
+       i0 += (long long)gridDim.x * take) {
+    const long long i = i0 + tid;
+    const bool here = tid < take && i < count;
+    const uint64_t x = here ? N[i] : 0;
+    const bool valid = (x & 1) && x >= 3 && x < (1ull << 63);
+    if (here && !valid) verdict[i] = 0;
+    const bool small = valid && sprp2_small(x);
+#pragma unroll
+    for (int form = 0; form < 2; form++) {
+      const bool mine = form ? valid && !small : small;
+      const unsigned bal = __ballot_sync(FULL, mine);
+      int at = 0;
+      if (lane == 0 && bal) at = atomicAdd(&waiting[form], __popc(bal));
+      at = __shfl_sync(FULL, at, 0) + __popc(bal & ((1u << lane) - 1u));
+      if (mine) {
+        value[form][at] = x;
+        index[form][at] = (uint32_t)i;
+      }
+    }
+    __syncthreads();
+    if (waiting[0] >= block) test(block, 0);
+    if (waiting[1] >= block) test(0, block);
   }
+  if (((waiting[0] + 31) & ~31) + waiting[1] > block) test(waiting[0], 0);
+  test(waiting[0], waiting[1]);
   unsigned v = sq;
   for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
-  if ((threadIdx.x & 31) == 0) {
-    if (per_warp) squarings[(blockIdx.x * blockDim.x + threadIdx.x) >> 5] = v;
+  if (lane == 0) {
+    if (per_warp) squarings[(blockIdx.x * block + tid) >> 5] = v;
     else if (v) atomicAdd(squarings, (unsigned long long)v);
   }
 }
@@ -2092,7 +2147,7 @@ extern "C" int ap26_sprp_batch(ap26_ctx *ctx, const uint64_t *N, int64_t count, 
   if (count == 0) return AP26_OK;
   // a short call's warps leave their counts behind the verdicts
   const bool small = count * (int64_t)sizeof(uint64_t) <= kZeroCopyBytes;
-  const int64_t warps = std::min<int64_t>((count + 63) / 64, ctx->num_sms * 16) * 2;
+  const int64_t warps = std::min<int64_t>((count + 63) / 64, ctx->num_sms * 4) * 4;
   unsigned long long *const tally =
       small ? (unsigned long long *)(ctx->sets[0].h_out + kZeroCopyBytes) : ctx->d_tally;
   if (!small) CK(cudaMemsetAsync(ctx->d_tally, 0, sizeof(*ctx->d_tally), ctx->stream));
@@ -2100,10 +2155,10 @@ extern "C" int ap26_sprp_batch(ap26_ctx *ctx, const uint64_t *N, int64_t count, 
   int rc = staged(
       ctx, count, {{(char *)N, sizeof(uint64_t)}}, {{(char *)verdict, 1}}, &ms,
       [&](int64_t n, const char *in, char *out, cudaStream_t s) {
-        const int block = small ? 64 : 256;
-        const int64_t blocks = std::min<int64_t>((n + block - 1) / block, ctx->num_sms * 16);
+        const int block = small ? 128 : SPRP_BLOCK, take = small ? block / 2 : block;
+        const int64_t blocks = std::min<int64_t>((n + take - 1) / take, ctx->num_sms * 4);
         sprp_batch_kernel<<<(int)blocks, block, 0, s>>>((const uint64_t *)in, n, (uint8_t *)out,
-                                                        tally, small);
+                                                        tally, small, take);
         return cudaGetLastError();
       });
   if (rc != AP26_OK) return rc;

@@ -1,8 +1,16 @@
-"""The kernel-level calls at the sizes where their paths change: a call of up to 1 MB of values is one kernel on pinned memory, a longer
+"""The kernel-level calls at the sizes and values where their paths change.
+
+Sizes: a call of up to 1 MB of values is one kernel on pinned memory, a longer
 one goes through sets of 8 MB in slices, by several host threads.  A long
 call's results are those of short calls on its pieces (which the other files
 check against the oracle and the reference's vectors).
+
+Values: the base-2 test has a form for 2^33 <= N < 2^60 with an odd part of
+N - 1 of at least six bits, and one for every other odd N; both against the
+oracle at those limits.
 """
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -61,3 +69,21 @@ def test_long_report_batches_equal_their_pieces(ctx, n):
     total = 5 + sum(onefin[i % len(aps)].hash_add for i in range(n))
     assert h == (total - 1) % 2_000_000_000 + 1
 
+
+def test_sprp_forms_at_their_limits(ctx, oracle):
+    N = []
+    for e in (33, 34, 59, 60, 61, 62):
+        N += [(1 << e) + d for d in range(-301, 301, 2)]
+    N += list(range(3, 2000, 2)) + [(1 << 63) - d for d in range(1, 301, 2)]
+    for e in range(3, 63):                       # N - 1 with a small odd part
+        N += [m * (1 << e) + 1 for m in (1, 3, 5, 31, 33, 63, 65) if m << e < 1 << 62]
+    N = np.array(N, np.uint64)
+    got, _ = ctx.sprp_batch(N)
+    exp = np.array([oracle.ao_sprp(ctypes.c_int64(int(n)), ctypes.c_int64(2)) for n in N], np.uint8)
+    assert np.array_equal(got, exp)
+    for a in (2, 3, 23, 31):
+        M = N[N > a]
+        got, _ = ctx.sprp_bases(M, np.full(len(M), a, np.uint32))
+        exp = np.array([oracle.ao_sprp(ctypes.c_int64(int(n)), ctypes.c_int64(a)) for n in M],
+                       np.uint8)
+        assert np.array_equal(got, exp), a
