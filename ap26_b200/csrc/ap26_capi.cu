@@ -1271,7 +1271,7 @@ static cudaError_t emit_run(ap26_ctx *ctx, JobSet &S, const uint32_t *tables, in
     ra.jobs = S.d_jobs;
     ra.fin = S.d_fin;
     ra.job_hash = S.d_job_hash;
-    report_kernel<<<ctx->num_sms * 2, REPORT_WARPS * 32, 0, s>>>(ra);
+    report_kernel<<<ctx->num_sms * 8, REPORT_THREADS, 0, s>>>(ra);
     EM(cudaGetLastError());
   }
   EM(cudaMemcpyAsync(S.h_st, S.d_st, sizeof(DevState), cudaMemcpyDeviceToHost, s));
@@ -2227,9 +2227,7 @@ extern "C" int ap26_report_batch(ap26_ctx *ctx, const ap26_ap *raw, int64_t n, a
         ra.jobs = nullptr;
         ra.fin = (FinRec *)fin;
         ra.job_hash = nullptr;
-        const int64_t want = (m + REPORT_WARPS - 1) / REPORT_WARPS;
-        report_kernel<<<(int)std::min<int64_t>(want, ctx->num_sms * 8), REPORT_WARPS * 32, 0, s>>>(
-            ra);
+        report_kernel<<<(int)std::min<int64_t>(m, ctx->num_sms * 16), REPORT_THREADS, 0, s>>>(ra);
         return cudaGetLastError();
       });
   if (rc != AP26_OK) return rc;

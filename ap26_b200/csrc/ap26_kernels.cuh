@@ -840,24 +840,27 @@ __device__ __forceinline__ int report_word(int64_t n, int shift) {
   return min(max(t >> 6, 0), WORDS - 1);
 }
 
-constexpr int REPORT_WARPS = 4;
-enum : uint8_t { TERM_DOM = 1, TERM_P2 = 2, TERM_P9 = 4 };
+constexpr int REPORT_THREADS = 96;
+constexpr int REPORT_BASES = 9;      // 2 and validate_ap26's 3..23 (AP26.cpp:519)
+enum : uint32_t { TERM_P2 = 1, TERM_P9 = (1 << REPORT_BASES) - 1, TERM_DOM = 1 << REPORT_BASES };
 
-// One warp per report: lane j tests terms j, j+32, ... (domain 0 <= N <
-// 2^62 of the reference's mulmod, AP26.cpp:494/529; base 2; the 8 further
-// bases of validate_ap26, AP26.cpp:519), then lane 0 replays the recursion
-// of ReportSolution over the per-term verdicts: every call adds
-// first%1000 + len; a piece whose first 9-base failure is at i is checked
-// to base 2 as a whole (Computation error otherwise), its leading i terms
-// are one call (valid, reported at length >= 20) and its trailing
-// len-(i+1) terms the next piece.
-__global__ void __launch_bounds__(REPORT_WARPS * 32) report_kernel(ReportArgs A) {
-  __shared__ uint8_t flags[REPORT_WARPS][FIN_MAX_TERMS];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+// One block per report: a thread tests one term to one base (terms in the
+// domain 0 <= N < 2^62 of the reference's mulmod, AP26.cpp:494/529), then
+// thread 0 replays the recursion of ReportSolution over the per-term
+// verdicts: every call adds first%1000 + len; a piece whose first 9-base
+// failure is at i is checked to base 2 as a whole (Computation error
+// otherwise), its leading i terms are one call (valid, reported at length >=
+// 20) and its trailing len-(i+1) terms the next piece.
+//
+// A report has 10 to 26 terms, so 90 to 234 tests, each a chain of some 75
+// dependent modular products: the time of one K's 150 reports is that chain's
+// latency.  A warp per report with a lane per term ran nine of them one after
+// the other (274 us for 150 reports, ten of 32 lanes busy); 96 threads run
+// most reports' tests at once.
+__global__ void __launch_bounds__(REPORT_THREADS) report_kernel(ReportArgs A) {
+  __shared__ uint32_t fl[FIN_MAX_TERMS];
   const long long n = A.count ? min((long long)*A.count, A.n) : A.n;
-  uint8_t *fl = flags[warp];
-  for (long long r = (long long)blockIdx.x * REPORT_WARPS + warp; r < n;
-       r += (long long)gridDim.x * REPORT_WARPS) {
+  for (long long r = blockIdx.x; r < n; r += gridDim.x) {
     const APRec rec = A.aps[r];
     const int K = A.jobs ? A.jobs[rec.job].K : rec.job;
     const int k = rec.k;
@@ -872,27 +875,20 @@ __global__ void __launch_bounds__(REPORT_WARPS * 32) report_kernel(ReportArgs A)
     if (args_ok && k > FIN_MAX_TERMS) out.status = REP_OVERFLOW;
     else if (!args_ok) out.status = REP_ARG;
     if (out.status == REP_OK) {
+      for (int j = threadIdx.x; j < k; j += REPORT_THREADS) fl[j] = 0;
+      __syncthreads();
       const uint64_t D = (uint64_t)K * (uint64_t)PRIM23;     // < 2^57
-      for (int j = lane; j < k; j += 32) {
-        uint8_t f = 0;
+      const uint32_t bases[REPORT_BASES] = {2, 3, 5, 7, 11, 13, 17, 19, 23};
+      for (int t = threadIdx.x; t < k * REPORT_BASES; t += REPORT_THREADS) {
+        const int j = t / REPORT_BASES, b = t - j * REPORT_BASES;
         const uint64_t jd = (uint64_t)j * D;                   // < 2^64
         const uint64_t N = (uint64_t)first + jd;
-        if (jd < (1ull << 62) && N < (1ull << 62)) {
-          f = TERM_DOM;
-          unsigned sq = 0;
-          if ((N & 1) && sprp2(N, sq)) {
-            f |= TERM_P2;
-            bool all = true;
-            const uint32_t bases[8] = {3, 5, 7, 11, 13, 17, 19, 23};
-            for (int b = 0; b < 8 && all; b++) all = sprp_base(bases[b], N);
-            if (all) f |= TERM_P9;
-          }
-        }
-        fl[j] = f;
+        if (jd < (1ull << 62) && N < (1ull << 62))
+          atomicOr(&fl[j], TERM_DOM | ((N & 1) && sprp_base(bases[b], N) ? 1u << b : 0u));
       }
     }
-    __syncwarp();
-    if (lane == 0) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
       if (out.status == REP_OK) {
         const int64_t D = (int64_t)K * PRIM23;
         int s = 0;
@@ -907,7 +903,7 @@ __global__ void __launch_bounds__(REPORT_WARPS * 32) report_kernel(ReportArgs A)
           } else {
             for (int j = s; j < e; j++) {
               if (!(fl[j] & TERM_DOM)) { out.status = REP_DOMAIN; break; }
-              if (!(fl[j] & TERM_P9)) { i = j; break; }
+              if ((fl[j] & TERM_P9) != TERM_P9) { i = j; break; }
             }
           }
           if (out.status != REP_OK) break;
@@ -955,7 +951,7 @@ __global__ void __launch_bounds__(REPORT_WARPS * 32) report_kernel(ReportArgs A)
         atomicAdd(&A.job_hash[rec.job * WORDS + report_word(rec.n, A.jobs[rec.job].shift)],
                   (unsigned long long)out.hash_add);
     }
-    __syncwarp();
+    __syncthreads();
   }
 }
 
