@@ -1177,7 +1177,9 @@ static cudaError_t emit_plan(const KJob *job, ClassPlan *plan, int num_sms, cuda
   cudaError_t e = cudaMemsetAsync(plan->vfill, 0, sizeof(plan->vfill), s);
   if (e != cudaSuccess) return e;
   class_plan_count_kernel<<<num_sms * 4, 256, 0, s>>>(job, plan);
+  class_plan_sum_kernel<<<(CLASSES + 7) / 8, 256, 0, s>>>(plan);
   class_plan_scan_kernel<<<1, 1024, 0, s>>>(plan);
+  class_plan_start_kernel<<<(CLASSES + 7) / 8, 256, 0, s>>>(plan);
   class_plan_scatter_kernel<<<num_sms * 8, 256, 0, s>>>(job, plan);
   return cudaGetLastError();
 }
@@ -1342,7 +1344,7 @@ static int enqueue_jobs(ap26_ctx *ctx, JobSet &S, int njobs, bool count_only, bo
   S.nprof = (ctx->opts.profile && &S == &ctx->main) ? std::min(S.nchunks, kProfChunks) : 0;
   if ((rc = ensure_prof_events(ctx, S.nprof)) != AP26_OK) return rc;
   S.launches = 1 + (int)S.nchunks * (count_only ? 3 : 4) + (count_only ? 0 : 1) +
-               (S.by_class ? 3 * njobs : 0);
+               (S.by_class ? 5 * njobs : 0);
   CK(cudaEventRecord(S.t0, ctx->stream));
   bool launched = false;
   if (ctx->opts.use_graphs > 0) {

@@ -36,22 +36,24 @@
 // Why this split (one B200, K = 43241061, sieve time of the whole K): the
 // window sieve moves 17.5 shared-memory wavefronts per lattice value and takes
 // 331 ms.  Classes alone took 156 ms, with 71 skipped by quarters and the
-// masks queued in 64-bit halves 140 ms.  It is bound by shared memory and L1:
-// 91% of their wavefront slots (issue 66%), half of them the dense rows', 14%
-// the v records' (the four quarters read four parts of a bucket), the rest the
-// queues and the lookups of the tail, most of them in stage A.  In one launch
-// (135 ms) building the rows takes 3 ms, reading them 82, the masks' queue and
-// stage A 33, stages B to D 18.  Sixteen warps with more registers were slower
-// (143 ms), twenty about equal (136.5), 26 and 28 too (143); 22 dense moduli,
-// which only fit with 20 warps, 134.7; v records as one 256-bit load 140;
-// four points a warp with a shuffle to join the two moduli's halves, single
-// bits instead of masks in the first queue, and two or four products in stage
-// A (136.7, 136.1 against 135.3) were slower too.
+// masks queued in 64-bit halves 140 ms, with the last single primes in two
+// stages and every shared address a constant (80 registers, hardly a spill)
+// 130 in one launch, where that had taken 135.  It is bound by shared memory
+// and L1: 91% of their wavefront slots (issue 67%), half of them the dense
+// rows', 14% the v records' (the four quarters read four parts of a bucket),
+// the rest the queues and the lookups of the tail, most of them in stage A.
+// Of the 135 ms, building the rows took 3, reading them 82, the masks' queue
+// and stage A 33, the stages behind it 18.  Warps: 16 with more registers 143
+// ms, 20 132, 22 131, 24 130, 26 and 28 143.  22 dense moduli, which only fit
+// with 20 warps, gained 0.6 ms; v records as one 256-bit load lost 5, a branch
+// around the tail lookups of dead lanes 1, two or four products in stage A 1,
+// four points a warp with a shuffle to join the two moduli's halves 36, single
+// bits instead of masks in the first queue 32.
 //
 // The class sieve takes every whole K.  A K that 61 or 67 divides has more
 // (b, j) per class (up to thirteen rows) and is still faster than by windows:
-// 266 against 389 ms for 61 | K, 388 against 463 for 61 * 67 | K, 583 against
-// 695 for 61 * 67 * 71 * 73 | K, the densest (with classes alone).  Parts of a
+// 230 against 389 ms for 61 | K, 326 against 463 for 61 * 67 | K, 550 against
+// 695 for 61 * 67 * 71 * 73 | K, the densest.  Parts of a
 // K (sieve_range) stay with the window sieve: a class's points are spread over
 // the whole lattice.
 //
@@ -64,7 +66,9 @@
 namespace ap26 {
 
 constexpr int NV = 19 * 23 * 29 * J59;        // v values, 443555
-constexpr int NB = 8;                          // b values
+constexpr int NB = 8;                          // b values: i3 * S3 + i5 * S5, multiples of
+                                               // MOD / 15
+static_assert(S3 == MOD / 15 * 10 && S5 == MOD / 15 * 3, "S3 = 2/3 MOD, S5 = 1/5 MOD");
 constexpr int CLASSES = PAIR1_P;               // 4087
 constexpr int ROW_BITS = 512;
 constexpr int ROWS_PER_CLASS = 4;              // units per class
@@ -126,7 +130,7 @@ constexpr TailMod TAIL_M[NTAIL] = {
 constexpr int STAGE_A = 3;                     // tail moduli of stage A; B takes the rest
 constexpr int FIRST_SINGLE = 30;               // PRIMES[30] = 223
 static_assert(PRIMES[FIRST_SINGLE] == 223, "single tail primes follow the products");
-constexpr int STAGE_C = 11;                    // singles of stage C; D takes the rest
+constexpr int STAGE_C = 11, STAGE_D = 25;      // singles before stage D, and before stage E
 constexpr int NSINGLE = NPRIMES - FIRST_SINGLE;
 constexpr int tail_words(int m) { return (m + 31) / 32; }
 constexpr int tail_off(int k) {
@@ -184,13 +188,14 @@ struct ClassPlan {
   uint64_t vc[NV + 16];           // v
   alignas(16) uint32_t xu[NUM_TRIPLES][12];   // a slot's two residues * 128, 16 bits each
   int64_t xval[NUM_TRIPLES];
-  int64_t bval[NB];
+  int32_t bmul[NB];               // value of b / (MOD / 15)
   int32_t xcls[NUM_TRIPLES];      // s(x) mod 4087
   int32_t xskip[NUM_TRIPLES];     // skip coordinate of x
   int32_t bres[NDENSE + 1][NB];   // s(b)
   int32_t bskip[NB];              // s(b) - 2 + SHIFT mod 71
   uint32_t vstart[NBINS + 1];     // v buckets: (s(v) mod 4087) * 71 + skip coordinate
   uint32_t vfill[NBINS];
+  uint32_t vclass[CLASSES];
   int32_t skip_mul, skip_inv;     // skip coordinate of residue r mod 71: r * mul; its inverse
   int32_t skip_bad, skip_len;     // 71 excludes coordinates [bad, bad + len) mod 71
   uint32_t dense_str[DENSE_STR_WORDS];
@@ -341,7 +346,7 @@ __global__ void class_plan_count_kernel(const KJob *job, ClassPlan *P) {
   if (blockIdx.x == 0 && threadIdx.x < NB) {
     const int b = threadIdx.x;
     const int64_t x = mod_MOD((uint64_t)(b >> 2) * (uint64_t)S3 + (uint64_t)(b & 3) * (uint64_t)S5);
-    P->bval[b] = x;
+    P->bmul[b] = (int32_t)(x / (MOD / 15));
     for (int k = 0; k <= NDENSE; k++) P->bres[k][b] = res_mod(x, c_res[k]);
     P->bskip[b] = (res_mod(x, c_res[RES_SKIP]) + shift + SKIP - MAX_WRAPS) % SKIP;
     if (b == 0) {
@@ -355,41 +360,60 @@ __global__ void class_plan_count_kernel(const KJob *job, ClassPlan *P) {
   }
 }
 
-// Second step (one block of 1024): bucket sizes to bucket starts, 284
-// consecutive buckets a thread.
-constexpr int SCAN_EACH = 284;
-static_assert(SCAN_EACH % 4 == 0 && 1024 * SCAN_EACH >= NBINS, "one pass of the scan");
-__global__ void __launch_bounds__(1024) class_plan_scan_kernel(ClassPlan *P) {
-  __shared__ uint32_t sums[32];
-  const int t = threadIdx.x, lane = t & 31, b0 = t * SCAN_EACH, b1 = min(b0 + SCAN_EACH, NBINS);
-  uint32_t tot = 0;
-#pragma unroll 8
-  for (int i = b0; i < b1; i++) tot += P->vfill[i];
-  uint32_t x = tot;
+// Second step, bucket sizes to bucket starts: a warp per class adds its 71
+// buckets up, one block of 1024 scans the classes, a warp per class scans its
+// buckets.  (One block over all 290177 buckets took 0.45 ms.)
+__device__ __forceinline__ uint32_t warp_scan(uint32_t x, int lane) {   // inclusive
   for (int o = 1; o < 32; o <<= 1) {
     const uint32_t y = __shfl_up_sync(FULL, x, o);
     if (lane >= o) x += y;
   }
+  return x;
+}
+
+__global__ void class_plan_sum_kernel(ClassPlan *P) {
+  const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (r >= CLASSES) return;
+  uint32_t sum = 0;
+  for (int i = lane; i < SKIP; i += 32) sum += P->vfill[r * SKIP + i];
+  for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(FULL, sum, o);
+  if (lane == 0) P->vclass[r] = sum;
+}
+
+__global__ void __launch_bounds__(1024) class_plan_scan_kernel(ClassPlan *P) {
+  __shared__ uint32_t sums[32];
+  const int t = threadIdx.x, lane = t & 31;
+  uint32_t c[4], tot = 0;
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    c[i] = 4 * t + i < CLASSES ? P->vclass[4 * t + i] : 0u;
+    tot += c[i];
+  }
+  const uint32_t x = warp_scan(tot, lane);
   if (lane == 31) sums[t >> 5] = x;
   __syncthreads();
-  if (t < 32) {
-    uint32_t s = sums[t];
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(FULL, s, o);
-      if (lane >= o) s += y;
-    }
-    sums[t] = s;
-  }
+  if (t < 32) sums[t] = warp_scan(sums[t], lane);
   __syncthreads();
   uint32_t at = x - tot + (t >= 32 ? sums[(t >> 5) - 1] : 0u);
-#pragma unroll 8
-  for (int i = b0; i < b1; i++) {
-    const uint32_t c = P->vfill[i];
-    P->vstart[i] = at;
-    P->vfill[i] = at;
-    at += c;
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    if (4 * t + i < CLASSES) P->vclass[4 * t + i] = at;
+    at += c[i];
   }
   if (t == 1023) P->vstart[NBINS] = at;
+}
+
+__global__ void class_plan_start_kernel(ClassPlan *P) {
+  const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (r >= CLASSES) return;
+  uint32_t at = P->vclass[r];
+  for (int i0 = 0; i0 < SKIP; i0 += 32) {
+    const int i = i0 + lane;
+    const uint32_t c = i < SKIP ? P->vfill[r * SKIP + i] : 0u;
+    const uint32_t x = warp_scan(c, lane);
+    if (i < SKIP) P->vstart[r * SKIP + i] = P->vfill[r * SKIP + i] = at + x - c;
+    at += __shfl_sync(FULL, x, 31);
+  }
 }
 
 // Third step: the v records in bucket order (any order inside a bucket).
@@ -429,35 +453,50 @@ struct ClassArgs {
 
 constexpr int CLASS_WARPS = 24;
 // Per-warp stacks in shared memory: 64-bit masks with their x + v waiting for
-// stage A (16 bytes), candidates for B, C and D (8 bytes).  A stage takes 32 entries; it runs when
+// stage A (16 bytes), candidates for B to E (8 bytes).  A stage takes 32 entries; it runs when
 // the entries about to be pushed would not fit, so its batches are full but
 // for the densest K.
-constexpr int ACAP = 64, QCAP = 46;
-constexpr int WARP_BYTES = ACAP * 16 + QCAP * 3 * 8;
-constexpr int CLASS_SMEM = DENSE_BYTES + CLASS_WARPS * WARP_BYTES + 8 * ROW_BITS + 4 * TAIL_WORDS;
-static_assert(CLASS_SMEM <= 226 * 1024, "class sieve shared memory");
+constexpr int ACAP = 64, QCAP = 40, QUEUES = 4;
+static_assert(ACAP >= 64 && QCAP >= 32, "a push fits an empty queue");
+constexpr int WARP_BYTES = ACAP * 16 + QCAP * QUEUES * 8;
+// Dynamic shared memory: rows, each warp's stacks, tail strings, (b, j) list.
+constexpr int QUEUE_BASE = DENSE_BYTES;
+constexpr int TS_BASE = QUEUE_BASE + CLASS_WARPS * WARP_BYTES;
+constexpr int EV_BASE = TS_BASE + 4 * TAIL_WORDS;
+constexpr int CLASS_SMEM = EV_BASE + 2 * ROW_BITS;
+extern __shared__ __align__(16) unsigned char class_smem[];
+static_assert(CLASS_SMEM <= 227 * 1024 - 1536,   // static shared memory beside it
+               "class sieve shared memory");
 
 // x + v + b is below 3 * MOD < 2^50; a candidate holds it with j << 50.
 constexpr int J_BIT = 50;
 static_assert(3 * MOD < (1ll << J_BIT), "sums fit 50 bits");
 
+__device__ __forceinline__ uint32_t *tail_string() {
+  return reinterpret_cast<uint32_t *>(class_smem + TS_BASE);
+}
+// The row's (b, j): value of b / (MOD / 15) << 10 | j.
+__device__ __forceinline__ uint16_t *row_list() {
+  return reinterpret_cast<uint16_t *>(class_smem + EV_BASE);
+}
+
 template <int k>
-__device__ __forceinline__ uint32_t tail_bit(const uint32_t *ts, uint32_t l0, uint32_t l1,
+__device__ __forceinline__ uint32_t tail_bit(uint32_t l0, uint32_t l1,
                                              uint32_t l2, uint32_t l3, uint32_t i) {
   constexpr TailParam P = tail_param(k);
   const uint32_t x = l0 * P.A + l1 * P.B + l2 * P.C + l3 * P.D + i;
   const uint32_t s = x - (uint32_t)P.m * (__umulhi(x, P.M) >> P.k);
-  const uint32_t w = ts[P.off + (s >> 5)];
+  const uint32_t w = tail_string()[P.off + (s >> 5)];
   return __funnelshift_r(w, w, s);             // bit 0: the string's bit s
 }
 
 template <int k0, int... I>
-__device__ __forceinline__ bool tail_test(const uint32_t *ts, uint32_t x, uint32_t y,
+__device__ __forceinline__ bool tail_test(uint32_t x, uint32_t y,
                                           std::integer_sequence<int, I...>) {
   const uint32_t i = y >> (J_BIT - 32);
   const uint32_t l0 = x & 0xfffu, l1 = (x >> 12) & 0xfffu,
                  l2 = __funnelshift_r(x, y, 24) & 0xfffu, l3 = (y >> 4) & 0x3fffu;
-  return ((tail_bit<k0 + I>(ts, l0, l1, l2, l3, i) & ...) & 1u) != 0u;
+  return ((tail_bit<k0 + I>(l0, l1, l2, l3, i) & ...) & 1u) != 0u;
 }
 
 // Transposes the 32 x 32 bit matrix whose row r is lane r's word: lane s
@@ -501,81 +540,80 @@ __device__ __forceinline__ void dense_rows(const unsigned char *rows, const uint
   (dense_slot<K>(rows, w[K / 2], u[K], sel0, sel1, acc), ...);
 }
 
-// What the stages read, the same for a whole row of a class.
-struct ClassShared {
-  const uint32_t *ts;            // tail bitstrings
-  const uint64_t *ev;            // the row's (b, j): value of b | j << 50
-  int shift, word_begin;
-};
-
-struct ClassWarp {               // one warp's stacks and counts
-  uint4 *qa;                     // 64 bits of a mask, x + v and which 64 bits << 52
-  uint2 *qb, *qc, *qd;
-  int na, nb, nc, nd;
+// One warp's stacks and counts.  Stack 0 holds stage A's entries (64 bits of a
+// mask, x + v and which 64 bits << 52), stacks 1 to 4 the candidates of B to E.
+struct ClassWarp {
+  unsigned char *base;
+  int n[QUEUES + 1];
   unsigned kept;
   unsigned long long late;
+  __device__ __forceinline__ uint4 *masks() const { return reinterpret_cast<uint4 *>(base); }
+  template <int Q> __device__ __forceinline__ uint2 *queue() const {
+    return reinterpret_cast<uint2 *>(base + ACAP * 16 + (Q - 1) * QCAP * 8);
+  }
 };
 
 // Takes up to 32 entries off a candidate stack.
-__device__ __forceinline__ bool pop(const uint2 *q, int &n, int lane, uint2 &it) {
+template <int Q>
+__device__ __forceinline__ bool pop(ClassWarp &W, int lane, uint2 &it) {
   __syncwarp();
-  const int take = min(n, 32);
-  n -= take;
-  it = lane < take ? q[n + lane] : make_uint2(0, 0);
+  const int take = min(W.n[Q], 32);
+  W.n[Q] -= take;
+  it = lane < take ? W.queue<Q>()[W.n[Q] + lane] : make_uint2(0, 0);
   __syncwarp();
   return lane < take;
 }
 
-__device__ __forceinline__ void push(uint2 *q, int &n, unsigned bal, bool mine, int lane,
+template <int Q>
+__device__ __forceinline__ void push(ClassWarp &W, unsigned bal, bool mine, int lane,
                                      const uint2 &it) {
-  if (mine) q[n + __popc(bal & ((1u << lane) - 1u))] = it;
-  n += __popc(bal);
+  if (mine) W.queue<Q>()[W.n[Q] + __popc(bal & ((1u << lane) - 1u))] = it;
+  W.n[Q] += __popc(bal);
 }
 
 // Bit of one single prime's string, limbs of 16, 16 and 18 bits.
 template <int k>
-__device__ __forceinline__ uint32_t single_bit(const uint32_t *ts, uint32_t a, uint32_t b,
-                                               uint32_t c, uint32_t i) {
+__device__ __forceinline__ uint32_t single_bit(uint32_t a, uint32_t b, uint32_t c, uint32_t i) {
   constexpr PrimeParam P = make_param_p(PRIMES[FIRST_SINGLE + k], single_off(k));
   const uint32_t x = a * (uint32_t)P.A + b * (uint32_t)P.B + c * (uint32_t)P.C + i;
   const uint32_t s = x - (uint32_t)P.p * (__umulhi(x, P.M) >> P.k);
-  const uint32_t w = ts[P.off + (s >> 5)];
+  const uint32_t w = tail_string()[P.off + (s >> 5)];
   return __funnelshift_r(w, w, s);
 }
 
 template <int k0, int... I>
-__device__ __forceinline__ bool single_step(const uint32_t *ts, uint32_t a, uint32_t b, uint32_t c,
-                                            uint32_t i, std::integer_sequence<int, I...>) {
-  return ((single_bit<k0 + I>(ts, a, b, c, i) & ...) & 1u) != 0u;
+__device__ __forceinline__ bool single_step(uint32_t a, uint32_t b, uint32_t c, uint32_t i,
+                                            std::integer_sequence<int, I...>) {
+  return ((single_bit<k0 + I>(a, b, c, i) & ...) & 1u) != 0u;
 }
 
 // Single primes k0..k1-1, STEP at a time while any lane is alive.  Unrolled:
 // parameters read from constant memory at a running index made the last
 // stage take a fifth of the kernel's time.
 template <int k0, int k1, int STEP>
-__device__ __forceinline__ bool single_test(const uint32_t *ts, const uint2 &it, bool alive) {
+__device__ __forceinline__ bool single_test(const uint2 &it, bool alive) {
   const uint32_t a = it.x & 0xffffu, b = it.x >> 16, c = it.y & 0x3ffffu;
-  alive = alive && single_step<k0>(ts, a, b, c, it.y >> (J_BIT - 32),
+  alive = alive && single_step<k0>(a, b, c, it.y >> (J_BIT - 32),
                                    std::make_integer_sequence<int, (k1 - k0 < STEP ? k1 - k0 : STEP)>{});
   if constexpr (k0 + STEP < k1) {
-    if (__any_sync(FULL, alive)) alive = single_test<k0 + STEP, k1, STEP>(ts, it, alive);
+    if (__any_sync(FULL, alive)) alive = single_test<k0 + STEP, k1, STEP>(it, alive);
     else alive = false;
   }
   return alive;
 }
 
-// Stage D: the last single primes, then emission of the candidates whose i
+// Stage E: the last single primes, then emission of the candidates whose i
 // lies in the shift words searched.
-__device__ __forceinline__ void stage_d(const ClassArgs &A, const ClassShared &C, ClassWarp &W,
-                                        int lane) {
+__device__ __forceinline__ void stage_e(const ClassArgs &A, ClassWarp &W, int lane) {
   uint2 it;
-  bool alive = pop(W.qd, W.nd, lane, it);
-  alive = single_test<STAGE_C, NSINGLE, 7>(C.ts, it, alive);
+  bool alive = pop<4>(W, lane, it);
+  alive = single_test<STAGE_D, NSINGLE, 7>(it, alive);
   uint64_t t = (uint64_t)it.x | (uint64_t)(it.y & 0x3ffffu) << 32;
   int i = (int)(it.y >> (J_BIT - 32)) - MAX_WRAPS;
   if (t >= (uint64_t)MOD) { t -= (uint64_t)MOD; i++; }
   if (t >= (uint64_t)MOD) { t -= (uint64_t)MOD; i++; }
-  alive = alive && i >= 64 * C.word_begin && i < 64 * WORDS;
+  const KJob &J = A.jobs[A.job];
+  alive = alive && i >= 64 * J.word_begin && i < 64 * WORDS;
   const unsigned bal = __ballot_sync(FULL, alive);
   if (!bal) return;
   W.kept += alive;
@@ -586,7 +624,7 @@ __device__ __forceinline__ void stage_d(const ClassArgs &A, const ClassShared &C
   at = __shfl_sync(FULL, at, leader) + __popc(bal & ((1u << lane) - 1u));
   if (alive) {
     if ((long long)at < A.cand_cap) {
-      A.cand[at].n = (int64_t)t + (int64_t)(C.shift + i) * MOD;
+      A.cand[at].n = (int64_t)t + (int64_t)(J.shift + i) * MOD;
       A.cand[at].job = A.job;
     } else {
       atomicOr(&A.st->err_flags, ERR_CAND_OVERFLOW);
@@ -594,40 +632,47 @@ __device__ __forceinline__ void stage_d(const ClassArgs &A, const ClassShared &C
   }
 }
 
-// Stage C: the first single primes.
-__device__ __forceinline__ void stage_c(const ClassArgs &A, const ClassShared &C, ClassWarp &W,
-                                        int lane) {
+// Stage D: the next single primes.
+__device__ __forceinline__ void stage_d(const ClassArgs &A, ClassWarp &W, int lane) {
   uint2 it;
-  bool alive = pop(W.qc, W.nc, lane, it);
-  alive = single_test<0, STAGE_C, STAGE_C>(C.ts, it, alive);
+  bool alive = pop<3>(W, lane, it);
+  alive = single_test<STAGE_C, STAGE_D, 7>(it, alive);
+  const unsigned bal = __ballot_sync(FULL, alive);
+  while (W.n[4] + __popc(bal) > QCAP) stage_e(A, W, lane);
+  push<4>(W, bal, alive, lane, it);
+}
+
+// Stage C: the first single primes.
+__device__ __forceinline__ void stage_c(const ClassArgs &A, ClassWarp &W, int lane) {
+  uint2 it;
+  bool alive = pop<2>(W, lane, it);
+  alive = single_test<0, STAGE_C, STAGE_C>(it, alive);
   const unsigned bal = __ballot_sync(FULL, alive);
   W.late += __popc(bal);
-  while (W.nd + __popc(bal) > QCAP) stage_d(A, C, W, lane);
-  push(W.qd, W.nd, bal, alive, lane, it);
+  while (W.n[3] + __popc(bal) > QCAP) stage_d(A, W, lane);
+  push<3>(W, bal, alive, lane, it);
 }
 
 // Stage B: the other tail products.
-__device__ __forceinline__ void stage_b(const ClassArgs &A, const ClassShared &C, ClassWarp &W,
-                                        int lane) {
+__device__ __forceinline__ void stage_b(const ClassArgs &A, ClassWarp &W, int lane) {
   uint2 it;
-  bool alive = pop(W.qb, W.nb, lane, it);
-  alive = alive && tail_test<STAGE_A>(C.ts, it.x, it.y,
+  bool alive = pop<1>(W, lane, it);
+  alive &= tail_test<STAGE_A>(it.x, it.y,
                                       std::make_integer_sequence<int, NTAIL - STAGE_A>{});
   const unsigned bal = __ballot_sync(FULL, alive);
-  while (W.nc + __popc(bal) > QCAP) stage_c(A, C, W, lane);
-  push(W.qc, W.nc, bal, alive, lane, it);
+  while (W.n[2] + __popc(bal) > QCAP) stage_c(A, W, lane);
+  push<2>(W, bal, alive, lane, it);
 }
 
 // Stage A: one bit of each of up to 32 waiting masks becomes a candidate
 // (masks with more bits go back), tested against the first tail products.
-__device__ __forceinline__ void stage_a(const ClassArgs &A, const ClassShared &C, ClassWarp &W,
-                                        int lane) {
+__device__ __forceinline__ void stage_a(const ClassArgs &A, ClassWarp &W, int lane) {
   __syncwarp();
-  const int n = min(W.na, 32);
-  W.na -= n;
+  const int n = min(W.n[0], 32);
+  W.n[0] -= n;
   bool alive = lane < n;
   uint4 it = make_uint4(0, 0, 0, 0);
-  if (alive) it = W.qa[W.na + lane];
+  if (alive) it = W.masks()[W.n[0] + lane];
   __syncwarp();
   // the mask's first bit
   const bool z = it.x == 0u;
@@ -637,35 +682,34 @@ __device__ __forceinline__ void stage_a(const ClassArgs &A, const ClassShared &C
   it.y = z ? c : it.y;
   const bool more = (it.x | it.y) != 0u;
   const unsigned mb = __ballot_sync(FULL, more);
-  if (more) W.qa[W.na + __popc(mb & ((1u << lane) - 1u))] = it;
-  W.na += __popc(mb);
-  const uint64_t v = C.ev[e & (ROW_BITS - 1)];
-  const uint64_t t = ((uint64_t)it.z | (uint64_t)(it.w & 0xfffffu) << 32) + v;
-  const uint2 cd = make_uint2((uint32_t)t, (uint32_t)(t >> 32) & 0x0fffffffu);   // b drops out
-  alive = alive && tail_test<0>(C.ts, cd.x, cd.y, std::make_integer_sequence<int, STAGE_A>{});
+  if (more) W.masks()[W.n[0] + __popc(mb & ((1u << lane) - 1u))] = it;
+  W.n[0] += __popc(mb);
+  const uint32_t v = row_list()[e & (ROW_BITS - 1)];
+  const uint64_t t = ((uint64_t)it.z | (uint64_t)(it.w & 0xfffffu) << 32) +
+                     (uint64_t)(v >> 10) * (uint64_t)(MOD / 15);
+  const uint2 cd = make_uint2((uint32_t)t, (uint32_t)(t >> 32) | (v & 0x3ffu) << (J_BIT - 32));
+  alive &= tail_test<0>(cd.x, cd.y, std::make_integer_sequence<int, STAGE_A>{});
   const unsigned bal = __ballot_sync(FULL, alive);
-  while (W.nb + __popc(bal) > QCAP) stage_b(A, C, W, lane);
-  push(W.qb, W.nb, bal, alive, lane, cd);
+  while (W.n[1] + __popc(bal) > QCAP) stage_b(A, W, lane);
+  push<1>(W, bal, alive, lane, cd);
 }
 
 // Empties the stacks (the masks refer to one row's (b, j) list).
-__device__ __noinline__ void flush(const ClassArgs &A, const ClassShared &C, ClassWarp &W,
-                                   int lane) {
-  while (W.na > 0) stage_a(A, C, W, lane);
-  while (W.nb > 0) stage_b(A, C, W, lane);
-  while (W.nc > 0) stage_c(A, C, W, lane);
-  while (W.nd > 0) stage_d(A, C, W, lane);
+__device__ __noinline__ void flush(const ClassArgs &A, ClassWarp &W, int lane) {
+  while (W.n[0] > 0) stage_a(A, W, lane);
+  while (W.n[1] > 0) stage_b(A, W, lane);
+  while (W.n[2] > 0) stage_c(A, W, lane);
+  while (W.n[3] > 0) stage_d(A, W, lane);
+  while (W.n[4] > 0) stage_e(A, W, lane);
 }
 
 __global__ void __launch_bounds__(CLASS_WARPS * 32, 1) class_sieve_kernel(ClassArgs A) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  unsigned char *rows = smem_raw;
-  uint4 *masks = reinterpret_cast<uint4 *>(rows + DENSE_BYTES);
-  uint2 *queues = reinterpret_cast<uint2 *>(masks + ACAP * CLASS_WARPS);
-  uint64_t *ev = reinterpret_cast<uint64_t *>(queues + 3 * QCAP * CLASS_WARPS);
-  uint32_t *ts = reinterpret_cast<uint32_t *>(ev + ROW_BITS);
+  unsigned char *const rows = class_smem;
+  uint32_t *const ts = tail_string();
+  uint16_t *const ev = row_list();
   __shared__ unsigned long long s_unit;
   __shared__ int s_cnt[CLASS_WARPS], s_x;
+  __shared__ uint8_t eb[ROW_BITS];      // b of the row's (b, j)
   __shared__ int s_o0[4], s_o1[4];      // first and last skip coordinate of the row's quarters
   __shared__ unsigned long long s_kept[CLASS_WARPS], s_late[CLASS_WARPS];
 
@@ -674,18 +718,10 @@ __global__ void __launch_bounds__(CLASS_WARPS * 32, 1) class_sieve_kernel(ClassA
   if (A.jobs[A.job].q_end == 0) return;
   const uint32_t *table = A.tables + (size_t)A.jobs[A.job].table * TABLE_WORDS;
   ClassWarp W;
-  W.qa = masks + warp * ACAP;
-  W.qb = queues + warp * 3 * QCAP;
-  W.qc = W.qb + QCAP;
-  W.qd = W.qc + QCAP;
-  W.na = W.nb = W.nc = W.nd = 0;
+  W.base = class_smem + QUEUE_BASE + warp * WARP_BYTES;
+  for (int k = 0; k <= QUEUES; k++) W.n[k] = 0;
   W.kept = 0;
   W.late = 0;
-  ClassShared C;
-  C.ts = ts;
-  C.ev = ev;
-  C.shift = A.jobs[A.job].shift;
-  C.word_begin = A.jobs[A.job].word_begin;
   for (int i = threadIdx.x; i < TAIL_WORDS; i += blockDim.x) ts[i] = P.tail_str[i];
 
   // this lane's part: quarter q of the row of point lane / 4 of eight
@@ -753,7 +789,8 @@ __global__ void __launch_bounds__(CLASS_WARPS * 32, 1) class_sieve_kernel(ClassA
         if (e < 0 || e >= ROW_BITS) continue;
         const int o = slot / (NB * JS), b = slot / JS % NB;
         const int j = (o * P.skip_inv + SKIP - P.bskip[b]) % SKIP + slot % JS * SKIP;
-        ev[e] = (uint64_t)P.bval[b] | (uint64_t)j << J_BIT | (uint64_t)b << (J_BIT + 10);
+        ev[e] = (uint16_t)(P.bmul[b] << 10 | j);
+        eb[e] = (uint8_t)b;
         if ((e & 127) == 0) s_o0[e >> 7] = o;
         if ((e & 127) == 127 || e == ne - 1) s_o1[e >> 7] = o;
       }
@@ -771,8 +808,7 @@ __global__ void __launch_bounds__(CLASS_WARPS * 32, 1) class_sieve_kernel(ClassA
           const int e = wq * 128 + u * 32 + lane;
           uint32_t x = 0;
           if (e < ne) {
-            const uint32_t v = (uint32_t)(ev[e] >> J_BIT);   // b << 10 | j
-            const int b = (int)(v >> 10), j = (int)(v & 0x3ffu);
+            const int b = eb[e], j = ev[e] & 0x3ff;
             const int at = (P.bres[k][b] + j + m - MAX_WRAPS) % m + s0;
             x = __funnelshift_r(str[at >> 5], str[(at >> 5) + 1], at & 31);
           }
@@ -846,23 +882,22 @@ __global__ void __launch_bounds__(CLASS_WARPS * 32, 1) class_sieve_kernel(ClassA
           const bool l0 = n > 0 && (m.x | m.y) != 0u, l1 = n > 0 && (m.z | m.w) != 0u;
           const unsigned bal0 = __ballot_sync(FULL, l0), bal1 = __ballot_sync(FULL, l1);
           const int c0 = __popc(bal0), c1 = __popc(bal1);
-          while (W.na + c0 + c1 > ACAP) stage_a(A, C, W, lane);
+          while (W.n[0] + c0 + c1 > ACAP) stage_a(A, W, lane);
           const unsigned below = (1u << lane) - 1u;
           if (l0)
-            W.qa[W.na + __popc(bal0 & below)] =
+            W.masks()[W.n[0] + __popc(bal0 & below)] =
                 make_uint4(m.x, m.y, (uint32_t)xt, (uint32_t)(xt >> 32));
-          W.na += c0;
+          W.n[0] += c0;
           if (l1)
-            W.qa[W.na + __popc(bal1 & below)] =
+            W.masks()[W.n[0] + __popc(bal1 & below)] =
                 make_uint4(m.z, m.w, (uint32_t)xt, (uint32_t)(xt >> 32) + (1u << 20));
-          W.na += c1;
+          W.n[0] += c1;
         }
       }
       // the masks refer to this row's (b, j) list: none is left over
       ClassArgs A1 = A;            // copies: what flush takes by reference lives in
-      ClassShared C1 = C;          // local memory
-      ClassWarp W1 = W;
-      flush(A1, C1, W1, lane);
+      ClassWarp W1 = W;            // local memory
+      flush(A1, W1, lane);
       W = W1;
       __syncthreads();
     }

@@ -329,7 +329,7 @@ int ap26_chain_batch(ap26_ctx *ctx, int K, const int64_t *n, int64_t count,
  * valid once that stream reaches this point.
  * - Allocates nothing (no cudaMalloc/cudaFree, no context object): all
  *   scratch -- job descriptors, tables, counters -- lives in one
- *   file-scope device array of AP26_NOALLOC_SCRATCH_BYTES (15,574,880 bytes)
+ *   file-scope device array of AP26_NOALLOC_SCRATCH_BYTES (15,591,200 bytes)
  *   that every GPU loading the library keeps until process exit.  At most
  *   AP26_NOALLOC_MAX_K values of K per call; more returns AP26_E_CAPACITY.
  *   An invalid K costs no sieve time.
@@ -343,7 +343,7 @@ int ap26_chain_batch(ap26_ctx *ctx, int K, const int64_t *n, int64_t count,
  *   calls whose work overlaps on the GPU (other streams, other threads)
  *   race on it and must be serialised by the caller. */
 #define AP26_NOALLOC_MAX_K 64
-#define AP26_NOALLOC_SCRATCH_BYTES 15574880
+#define AP26_NOALLOC_SCRATCH_BYTES 15591200
 int ap26_sieve_count_noalloc(int device, const int32_t *d_Ks, int nK, int shift,
                              int64_t *d_counts, void *stream);
 
