@@ -227,21 +227,67 @@ __global__ void sprp_bases_kernel(const uint64_t *N, const uint32_t *a, long lon
   }
 }
 
-// Chain walk for explicit candidates (kernel-level parity entry point).
-__global__ void chain_explicit_kernel(int64_t S, const int64_t *n, long long count,
-                                      int32_t *k_out, int64_t *first_out, DevState *st) {
-  unsigned tests = 0, sq = 0;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < count;
-       i += (long long)gridDim.x * blockDim.x) {
+// Chain walk for explicit candidates (kernel-level parity entry point).  A warp
+// takes 32 candidates.  Their first terms are one test a lane; about one walk
+// in four goes on, and the lanes of those that ended test further terms of
+// the others ahead: with c walks left, 32 / c terms of each at once.  A term
+// past a walk's end changes nothing, also where it is outside the domain.
+// The time of a short call is its longest walk, ten tests one after the other
+// where every lane walked alone: 20011 candidates 44 us and now 30, a million
+// 589 and 294.
+constexpr int CHAIN_WARPS = 2;
+__global__ void __launch_bounds__(CHAIN_WARPS * 32)
+chain_explicit_kernel(int64_t S, const int64_t *n, long long count, int32_t *k_out,
+                      int64_t *first_out, DevState *st) {
+  __shared__ int owner[CHAIN_WARPS][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  unsigned sq = 0;
+  for (long long i0 = (blockIdx.x * (long long)CHAIN_WARPS + warp) * 32; i0 < count;
+       i0 += (long long)gridDim.x * CHAIN_WARPS * 32) {
+    const long long i = i0 + lane;
+    const int64_t start = i < count ? n[i] : 0;
+    int64_t m = start + S * 5, step = S;
     int k = 0;
-    int64_t m = n[i] + S * 5;
-    while (prp_term(st, m, tests, sq)) { k++; m += S; }
-    if (k >= 10) {
-      m = n[i] + S * 4;
-      while (m > 0 && prp_term(st, m, tests, sq)) { k++; m -= S; }
+    bool walking = i < count;
+    for (;;) {
+      const unsigned left = __ballot_sync(FULL, walking);
+      if (!left) break;
+      const int c = __popc(left), ahead = 32 / c, mine = __popc(left & ((1u << lane) - 1u));
+      if (walking) owner[warp][mine] = lane;
+      __syncwarp();
+      // this lane's test: term `t` ahead of walk w
+      const int w = lane / ahead, t = lane - w * ahead;
+      const int from = w < c ? owner[warp][w] : 0;
+      __syncwarp();
+      const int64_t dir = __shfl_sync(FULL, step, from);
+      const int64_t term = __shfl_sync(FULL, m, from) + dir * t;
+      const bool ok = w < c && (dir > 0 || term > 0) && (uint64_t)term < (1ull << 62) &&
+                      (term & 1) && sprp2((uint64_t)term, sq);
+      const unsigned hits = __ballot_sync(FULL, ok);
+      if (walking) {
+        const unsigned got = hits >> (mine * ahead);
+        const int run = min(ahead, ~got ? __ffs(~got) - 1 : 32);
+        k += run;
+        m += step * run;
+        if (run < ahead) {                      // the walk stops at m
+          if (step < 0 && m <= 0) {
+            walking = false;                    // below zero, untested
+          } else {
+            if ((uint64_t)m >= (1ull << 62)) atomicOr(&st->err_flags, ERR_DOMAIN);
+            if (step > 0 && k >= 10) {
+              step = -S;
+              m = start + S * 4;
+            } else {
+              walking = false;
+            }
+          }
+        }
+      }
     }
-    k_out[i] = k;
-    first_out[i] = m + S;
+    if (i < count) {
+      k_out[i] = k;
+      first_out[i] = m + S;
+    }
   }
 }
 
@@ -2262,7 +2308,7 @@ extern "C" int ap26_chain_batch(ap26_ctx *ctx, int K, const int64_t *n, int64_t 
       {{(char *)first_out, sizeof(int64_t)}, {(char *)k_out, sizeof(int32_t)}}, &ms,
       [&](int64_t m, const char *in, char *out, cudaStream_t s) {
         const int64_t blocks = std::min<int64_t>((m + 63) / 64, ctx->num_sms * 16);
-        chain_explicit_kernel<<<(int)blocks, 64, 0, s>>>(
+        chain_explicit_kernel<<<(int)blocks, CHAIN_WARPS * 32, 0, s>>>(
             (int64_t)K * PRIM23, (const int64_t *)in, m, (int32_t *)(out + sizeof(int64_t) * m),
             (int64_t *)out, S.h_st);
         return cudaGetLastError();

@@ -87,3 +87,18 @@ def test_sprp_forms_at_their_limits(ctx, oracle):
         exp = np.array([oracle.ao_sprp(ctypes.c_int64(int(n)), ctypes.c_int64(a)) for n in M],
                        np.uint8)
         assert np.array_equal(got, exp), a
+
+
+def test_chain_terms_past_the_end_of_a_walk_do_not_count(ctx):
+    """Terms are tested ahead of a walk: one at 2^62 or beyond is an error only
+    where the walk reaches it (2^62 is the domain of the reference's PrimeQ)."""
+    K = 50_000_001
+    S = K * A.PRIM23
+    top = (1 << 62) - 1
+    n = next(m for m in range(top, top - 12, -1) if m % 3 == 0 and m % 2) - 5 * S
+    k, f, _ = ctx.chain_batch(K, np.array([n], np.int64))
+    assert (k[0], f[0]) == (0, n + 6 * S)        # n + 5S composite, n + 6S beyond 2^62
+    for bad in (n + S, n + 4):
+        with pytest.raises(A.AP26Error) as e:
+            ctx.chain_batch(K, np.array([bad], np.int64))
+        assert e.value.code == A.E_DOMAIN
