@@ -213,17 +213,15 @@ sprp_batch_kernel(const uint64_t *N, long long count, uint8_t *verdict,
   }
 }
 
-// strong_prp(a, N) for explicit (N, a) pairs, a in [2, 31].
+// strong_prp(a, N) for explicit (N, a) pairs, a in [2, 31].  Base 2 takes the
+// general form too: sprp2's would be run beside it by nearly every warp.
 __global__ void sprp_bases_kernel(const uint64_t *N, const uint32_t *a, long long count,
                                   uint8_t *verdict) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < count;
        i += (long long)gridDim.x * blockDim.x) {
     const uint64_t n = N[i];
     const uint32_t b = a[i];
-    unsigned sq = 0;
-    bool v = false;
-    if ((n & 1) && n > b && n < (1ull << 63)) v = b == 2 ? sprp2(n, sq) : sprp_base(b, n);
-    verdict[i] = (uint8_t)v;
+    verdict[i] = (uint8_t)((n & 1) && n > b && n < (1ull << 63) && sprp_base(b, n));
   }
 }
 

@@ -792,11 +792,16 @@ __device__ __forceinline__ bool sprp_base(uint32_t a, uint64_t N) {
       if (am >= N) am -= N;
     }
   }
-  uint64_t x = am;
-  const int top = 63 - __clzll((long long)d);
-  for (int i = top - 1; i >= 0; i--) {
-    x = mont_sq(x, N, inv);
-    if ((d >> i) & 1) x = mont_mul(x, am, N, inv);
+  // two bits of d at a time, from a, a^2 and a^3: in a warp some lane has a
+  // bit set at every step, so one bit at a time is a product at every square
+  // (9600 reports 258 us, now 234)
+  const uint64_t am2 = mont_sq(am, N, inv), am3 = mont_mul(am2, am, N, inv);
+  const int top = (63 - __clzll((long long)d)) & ~1;
+  uint64_t x = (d >> top) == 1 ? am : (d >> top) == 2 ? am2 : am3;
+  for (int i = top - 2; i >= 0; i -= 2) {
+    x = mont_sq(mont_sq(x, N, inv), N, inv);
+    const int w = (int)(d >> i) & 3;
+    if (w) x = mont_mul(x, w == 1 ? am : w == 2 ? am2 : am3, N, inv);
   }
   if (x == one || x == mone) return true;
   for (int s = 1; s < t; s++) {
