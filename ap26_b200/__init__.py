@@ -231,6 +231,9 @@ _AP = np.dtype([("k", np.int32), ("K", np.int32), ("first", np.int64), ("n", np.
 assert _AP.itemsize == ctypes.sizeof(AP)
 
 
+_DENSITY_PRIMES = (61, 67, 71, 73, 79, 83, 89, 97, 101, 103, 107, 109, 113, 127, 131, 137, 139)
+
+
 def _aps_to_list(arr, n):
     return arr[:n].tolist()
 
@@ -358,12 +361,23 @@ class Context:
         return per, list(res), st
 
     def sieve_range(self, K, shift, q0, q1, cap=1 << 22):
-        cand = np.empty(cap, np.int64)
+        # room for the survivors expected of this K (a prime that divides it
+        # excludes one residue, not 24), the rest of cap only if they are more
+        room = 0.37 * max(0, int(q1) - int(q0))
+        for p in _DENSITY_PRIMES:
+            if int(K) % p == 0:
+                room *= (p - 1) / (p - 24)
+        room = min(int(cap), int(room) + 1024)
         n = ctypes.c_int64(0)
         st = Stats()
-        self._check(lib.ap26_sieve_range(self.h, int(K), int(shift), int(q0), int(q1), _ptr(cand),
-                                         cap, ctypes.byref(n), ctypes.byref(st)),
-                    "ap26_sieve_range")
+        while True:
+            cand = np.empty(room, np.int64)
+            rc = lib.ap26_sieve_range(self.h, int(K), int(shift), int(q0), int(q1), _ptr(cand),
+                                      room, ctypes.byref(n), ctypes.byref(st))
+            if rc != E_CAPACITY or not room < n.value <= cap:
+                break
+            room = n.value
+        self._check(rc, "ap26_sieve_range")
         return cand[:n.value].copy(), st
 
     def sieve_count(self, Ks, shift):

@@ -64,22 +64,40 @@ __device__ void build_table(int K, int shift, uint32_t *tab, int first, int stri
 // the class sieve, none where a serving unit built them at admission.  A word
 // is a chain of some 600 instructions, so one word a thread: a block of 256
 // that built eleven each (and sorted a lattice order) took 0.3 ms.
+__device__ void set_constants(KJob &J) {
+  const int K = J.K;
+  J.STEP = (int64_t)K * PRIM23;
+  J.n0 = (N0 * (K % 17835) + ((N0 * 17835) % MOD) * (K / 17835) + N30) % MOD;
+  kmul_mod(PRES2, K, &J.S31);
+  kmul_mod(PRES3, K, &J.S37);
+  kmul_mod(PRES4, K, &J.S41);
+  kmul_mod(PRES5, K, &J.S43);
+  kmul_mod(PRES6, K, &J.S47);
+  kmul_mod(PRES7, K, &J.S53);
+  kmul_mod(PRES8, K, &J.S59);
+}
+
 __global__ void setup_jobs_kernel(KJob *jobs, uint32_t *tables, int words) {
   KJob &J = jobs[blockIdx.x];
   const int K = J.K;
-  if (threadIdx.x == 0 && blockIdx.y == 0) {
-    J.STEP = (int64_t)K * PRIM23;
-    J.n0 = (N0 * (K % 17835) + ((N0 * 17835) % MOD) * (K / 17835) + N30) % MOD;
-    kmul_mod(PRES2, K, &J.S31);
-    kmul_mod(PRES3, K, &J.S37);
-    kmul_mod(PRES4, K, &J.S41);
-    kmul_mod(PRES5, K, &J.S43);
-    kmul_mod(PRES6, K, &J.S47);
-    kmul_mod(PRES7, K, &J.S53);
-    kmul_mod(PRES8, K, &J.S59);
-  }
+  if (threadIdx.x == 0 && blockIdx.y == 0) set_constants(J);
   build_table(K, J.shift, tables + (size_t)J.table * TABLE_WORDS,
               (int)(blockIdx.y * blockDim.x + threadIdx.x), (int)(gridDim.y * blockDim.x), words);
+}
+
+// The whole set-up of an ap26_sieve_range call in one launch: its job, a fresh
+// run state of `tiles` tiles and its bitstrings, one word a thread.
+__global__ void range_setup_kernel(KJob job, KJob *jobs, DevState *st, unsigned long long tiles,
+                                   unsigned long long *job_counts, uint32_t *tables) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    memset(st, 0, sizeof(*st));
+    st->tile_end = tiles;
+    job_counts[0] = 0;
+    set_constants(job);
+    jobs[0] = job;
+  }
+  build_table(job.K, job.shift, tables, (int)(blockIdx.x * blockDim.x + threadIdx.x),
+              (int)(gridDim.x * blockDim.x), TABLE_WORDS);
 }
 
 static void launch_setup(KJob *jobs, int njobs, uint32_t *tables, int words, cudaStream_t s) {
@@ -321,24 +339,13 @@ static cudaError_t upload_constants() {
   return cudaMemcpyToSymbol(c_slot_base, slot, sizeof(slot));
 }
 
-// ap26_sieve_range: one job's descriptor and a fresh run state, in one launch.
-__global__ void range_init_kernel(KJob job, KJob *jobs, DevState *st, unsigned long long tiles,
-                                  unsigned long long *job_counts) {
-  jobs[0] = job;
-  memset(st, 0, sizeof(*st));
-  st->tile_end = tiles;
-  job_counts[0] = 0;
-}
-
-// Candidates [begin, begin + most) of the ring as plain n, and the run state.
+// Candidates [begin, begin + most) of the ring as plain n.
 __global__ void range_pack_kernel(const Cand *cand, const DevState *st, long long cand_cap,
-                                  long long begin, long long most, int64_t *out,
-                                  DevState *st_out) {
+                                  long long begin, long long most, int64_t *out) {
   const long long n = min((long long)st->cand_count[0], cand_cap) - begin;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < min(n, most);
        i += (long long)gridDim.x * blockDim.x)
     out[i] = cand[begin + i].n;
-  if (blockIdx.x == 0 && threadIdx.x == 0) *st_out = *st;
 }
 
 // Argument blocks are only built through these, so no field can be left
@@ -373,9 +380,12 @@ static ClassArgs class_args(const KJob *jobs, int job, const ClassPlan *plan,
 
 static SieveArgs sieve_args(const KJob *jobs, int njobs, const uint32_t *tables, DevState *st,
                             Cand *cand, long long cand_cap, unsigned long long *job_counts,
-                            int count_only, unsigned long long *cand_count, int parts = 1) {
+                            int count_only, unsigned long long *cand_count, int parts = 1,
+                            int64_t *raw = nullptr, long long raw_cap = 0) {
   SieveArgs a;
   a.parts = parts;
+  a.raw = raw;
+  a.raw_cap = raw_cap;
   a.jobs = jobs;
   a.njobs = njobs;
   a.tables = tables;
@@ -2123,14 +2133,14 @@ extern "C" int ap26_sieve_range(ap26_ctx *ctx, int K, int shift, int64_t q_begin
   StageSet &G = ctx->sets[0];
   const long long most = kSetBytes / (long long)sizeof(int64_t);
   CK(cudaEventRecord(ctx->ev0, s));
-  range_init_kernel<<<1, 1, 0, s>>>(J, S.d_jobs, S.d_st, (unsigned long long)tiles, S.d_job_counts);
-  launch_setup(S.d_jobs, 1, S.d_tables, TABLE_WORDS, s);
+  range_setup_kernel<<<(TABLE_WORDS + 255) / 256, 256, 0, s>>>(
+      J, S.d_jobs, S.d_st, (unsigned long long)tiles, S.d_job_counts, S.d_tables);
+  // the first candidates go straight to pinned memory, the others to the ring
   const SieveArgs sa = sieve_args(S.d_jobs, 1, S.d_tables, S.d_st, ctx->d_cand[0],
-                                  ctx->cand_cap, S.d_job_counts, 0, &S.d_st->cand_count[0], parts);
+                                  ctx->cand_cap, S.d_job_counts, 0, &S.d_st->cand_count[0], parts,
+                                  (int64_t *)G.h_out, std::min<long long>(most, ctx->cand_cap));
   V.kernel<<<ctx->sieve_blocks, V.WARPS * 32, V.smem(), s>>>(sa);
-  // the candidates go straight to pinned memory, a buffer of them at a time
-  range_pack_kernel<<<ctx->num_sms, 256, 0, s>>>(ctx->d_cand[0], S.d_st, ctx->cand_cap, 0, most,
-                                                 (int64_t *)G.h_out, S.h_st);
+  CK(cudaMemcpyAsync(S.h_st, S.d_st, sizeof(DevState), cudaMemcpyDeviceToHost, s));
   CK(cudaGetLastError());
   CK(cudaEventRecord(ctx->ev1, s));
   rc = wait_event(ctx, ctx->ev1, ctx->opts.wait_timeout_s);
@@ -2143,7 +2153,7 @@ extern "C" int ap26_sieve_range(ap26_ctx *ctx, int K, int shift, int64_t q_begin
     const long long n = std::min(most, nc - at);
     if (at > 0) {
       range_pack_kernel<<<ctx->num_sms, 256, 0, s>>>(ctx->d_cand[0], S.d_st, ctx->cand_cap, at,
-                                                     most, (int64_t *)G.h_out, S.h_st);
+                                                     most, (int64_t *)G.h_out);
       CK(cudaGetLastError());
       CK(cudaStreamSynchronize(s));
     }
@@ -2157,7 +2167,7 @@ extern "C" int ap26_sieve_range(ap26_ctx *ctx, int K, int shift, int64_t q_begin
     stats->late_items = (int64_t)S.h_st->late_items;
     stats->device_ms = ms;
     stats->error_flags = (int32_t)S.h_st->err_flags;
-    stats->launches = 4;
+    stats->launches = 2;
   }
   return AP26_OK;
 }

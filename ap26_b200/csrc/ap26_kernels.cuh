@@ -112,6 +112,8 @@ struct SieveArgs {
   int count_only;               // 1: count survivors, emit no candidates
   unsigned long long *cand_count;  // fill count of `cand` (DevState::cand_count[ring])
   int parts;                    // tiles per block of starts, each 35 / parts of its j59
+  int64_t *raw;                 // the first raw_cap candidates' n go here instead of `cand`
+  long long raw_cap;
 };
 
 struct ChainArgs {
@@ -238,7 +240,9 @@ __device__ __forceinline__ int emit_word(const SieveArgs &A, uint64_t n59, int w
       kept++;
       if (!A.count_only) {
         unsigned long long i = atomicAdd(A.cand_count, 1ull);
-        if ((long long)i < A.cand_cap) {
+        if ((long long)i < A.raw_cap) {
+          A.raw[i] = n;
+        } else if ((long long)i < A.cand_cap) {
           A.cand[i].n = n;
           A.cand[i].job = job;
         } else {
