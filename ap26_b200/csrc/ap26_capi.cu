@@ -926,6 +926,9 @@ extern "C" const char *ap26_last_error(const ap26_ctx *ctx) {
   return ctx ? ctx->last_error.c_str() : "";
 }
 
+// Tiles per launch unless opts.chunk_tiles says otherwise.
+constexpr int kDefaultChunkTiles = 131072;
+
 // K-jobs per run of ap26_search_batch (ap26_opts.batch_wave): by default
 // about 3 minutes of device time and at most a few hundred thousand raw
 // reports (the main set holds 2^20); at most 2048 (about 12 minutes).
@@ -938,7 +941,7 @@ static int default_opts(ap26_opts *o) {
   if (!o->block_threads) o->block_threads = kVariants[0].WARPS * 32;
   if (!o->late_stage) o->late_stage = kVariants[0].SL;
   if (!o->tail_group) o->tail_group = kVariants[0].R;
-  if (!o->chunk_tiles) o->chunk_tiles = 131072;
+  if (!o->chunk_tiles) o->chunk_tiles = kDefaultChunkTiles;
   if (!o->use_graphs) o->use_graphs = 1;
   if (!o->cand_ring_log2) o->cand_ring_log2 = 26;
   if (!(o->wait_timeout_s > 0)) o->wait_timeout_s = 3600.0;
@@ -1238,12 +1241,34 @@ static cudaError_t emit_plan(const KJob *job, ClassPlan *plan, int num_sms, cuda
   return cudaGetLastError();
 }
 
-// Class-sieve units per launch for chunks of chunk_tiles tiles of tile_n53
-// starts (at least one unit), made equal over a K's launches.
-static int class_chunk_units(int chunk_tiles, int64_t tile_n53) {
+// Survivors expected of a whole K: 36.82 to 36.86 M over the 155 known counts
+// (four SHIFTs), times (p - 1) / (p - 24) for each sieve prime p that divides K
+// and so excludes one residue, not 24.
+static double expected_survivors(int K) {
+  double n = 36.9e6;
+  for (int p : PRIMES)
+    if (K % p == 0) n *= (p - 1) / (double)(p - 24);
+  return n;
+}
+
+// Class-sieve units per launch of a run.  A set chunk_tiles bounds it: chunks
+// of chunk_tiles tiles of tile_n53 starts, at least one unit, equal over a K.
+// At the default a launch takes a whole K when nothing is kept of it but counts,
+// or when the survivors of the densest K of the run fit a ring with a quarter to
+// spare, and as large a part as fits when they do not.  Each launch ends with
+// CTAs that wait for the last one and with the last walks of its chains: a K
+// took 137.3 to 137.8 ms in five launches and takes 135.5 to 136.2 in one.
+static int class_chunk_units(const KJob *jobs, int njobs, bool count_only, long long cand_cap,
+                             int chunk_tiles, int64_t tile_n53) {
   const int64_t most = std::max<int64_t>(
       1, std::min<int64_t>(UNITS_PER_K, (int64_t)chunk_tiles * tile_n53 * UNITS_PER_K / N53_PER_K));
-  const int64_t n = (UNITS_PER_K + most - 1) / most;
+  int64_t n = (UNITS_PER_K + most - 1) / most;
+  if (chunk_tiles == kDefaultChunkTiles) {
+    double survivors = 0;
+    for (int j = 0; j < njobs && !count_only; j++)
+      survivors = std::max(survivors, expected_survivors(jobs[j].K));
+    n = std::min(n, 1 + (int64_t)(1.25 * survivors / (double)cand_cap));
+  }
   return (int)((UNITS_PER_K + n - 1) / n);
 }
 static int class_chunks(int chunk_units) { return (UNITS_PER_K + chunk_units - 1) / chunk_units; }
@@ -1388,7 +1413,7 @@ static int enqueue_jobs(ap26_ctx *ctx, JobSet &S, int njobs, bool count_only, bo
   S.by_class = njobs > 0;
   for (int j = 0; j < njobs; j++)
     if (S.h_jobs[j].q_begin != 0 || S.h_jobs[j].q_end != N53_PER_K) S.by_class = false;
-  S.chunk_units = class_chunk_units(chunk_tiles, tile_n53);
+  S.chunk_units = class_chunk_units(S.h_jobs, njobs, count_only, ctx->cand_cap, chunk_tiles, tile_n53);
   S.nchunks = S.by_class ? (unsigned long long)njobs * class_chunks(S.chunk_units)
               : tiles    ? (tiles + chunk_tiles - 1) / chunk_tiles
                          : 0;

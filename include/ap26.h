@@ -56,8 +56,11 @@ typedef struct {
   int32_t block_threads;  /* sieve CTA size (multiple of 32)                  */
   int32_t late_stage;     /* prime index where items move to the late queue   */
   int32_t chunk_tiles;    /* sieve tiles (one n53 start per CTA thread) per
-                             launch (default 131072, about a quarter of a K;
-                             the autotuner times the sizes the rings hold)    */
+                             launch; a whole K's launches take their share of
+                             its units.  At the default, 131072 (about a
+                             quarter of a K), a launch takes the whole K where
+                             its survivors fit a ring.  The autotuner times
+                             the sizes the rings hold                         */
   int32_t use_graphs;     /* 1 (default) = every run (set-up, chunks, chain
                              walks, ReportSolution, read-backs) is one CUDA
                              graph launch, captured once per run shape and

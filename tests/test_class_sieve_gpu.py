@@ -41,3 +41,25 @@ def test_whole_k_survivors_equal_the_window_sieves(K, shift, chunk_tiles):
         aps, st = ctx.search_k(K, shift)
         assert st.candidates == st.chain_walks == counts[0]
         assert st.error_flags == 0
+
+
+@pytest.mark.parametrize("K,ring,sieves", [
+    (43241061, 27, 1),                   # 36.9 M fit with a quarter to spare
+    (43241061, 25, 2),                   # 33.5 M entries: two launches
+    (61 * 7019, 26, 2),                  # 61 | K: 59.8 M, too near to 67.1 M
+    (21182921, 26, 4),                   # the densest K: 201 M
+    (43241061, 22, 5),                   # never more launches than chunk_tiles asks for
+])
+def test_launches_of_a_k_by_the_survivors_a_ring_holds(K, ring, sieves):
+    with A.Context(0, cand_ring_log2=ring) as ctx:
+        counts, st = ctx.sieve_count([K], 0)
+        assert st.launches == 1 + 5 + 3              # counts alone: one launch
+        aps, st = ctx.search_k(K, 0)
+        assert st.candidates == st.chain_walks == counts[0]
+        if ring > 22:                                # there a chunk overflows and is redone
+            assert st.launches == 1 + 5 + 4 * sieves + 1
+            assert st.error_flags == 0
+    with A.Context(0, chunk_tiles=131071) as ctx:    # a set size bounds the launches
+        want, st = ctx.search_k(K, 0)
+        assert st.launches == 1 + 5 + 4 * 5 + 1
+        assert aps == want
