@@ -89,6 +89,46 @@ def test_sprp_forms_at_their_limits(ctx, oracle):
         assert np.array_equal(got, exp), a
 
 
+def _is_prime(n):
+    return all(n == p or (n % p and _strong(n, p)) for p in (2, 3, 5, 7, 11, 13, 17, 19, 23, 29, 31, 37))
+
+
+def _strong(n, a):
+    d, t = n - 1, 0
+    while d % 2 == 0:
+        d, t = d // 2, t + 1
+    x = pow(a, d, n)
+    return x in (1, n - 1) or any((x := x * x % n) == n - 1 for _ in range(t - 1))
+
+
+@pytest.mark.parametrize("bits", [35, 59, 61])
+def test_sprp_over_the_powers_of_two_in_n_minus_one(ctx, bits):
+    """2^-d and the squares after it are looked for in the last squares of one
+    loop: primes and composites with every 2^t in N - 1 on both sides of that
+    length, and products p(2p - 1) and p(3p - 2), many of which are
+    pseudoprimes whose square roots of 1 decide."""
+    rng = np.random.default_rng(bits)
+    N, psp = [], 0
+    for t in range(1, 24 if bits < 40 else 40):
+        primes = 0
+        while primes < 12:
+            n = (int(rng.integers(1 << (bits - t - 1), 1 << (bits - t))) | 1) << t | 1
+            N.append(n)
+            primes += _is_prime(n)
+    for m in (2, 3):
+        p = int(2 ** (bits / 2)) // m | 1
+        while psp < 40 * (m - 1):
+            p += 2
+            if _is_prime(p) and _is_prime(m * (p - 1) + 1):
+                N.append(p * (m * (p - 1) + 1))
+                psp += 1
+    exp = np.array([_strong(n, 2) for n in N], np.uint8)
+    got, _ = ctx.sprp_batch(np.array(N, np.uint64))
+    assert np.array_equal(got, exp)
+    assert np.array_equal(ctx.sprp_bases(np.array(N, np.uint64), np.full(len(N), 2, np.uint32))[0],
+                          exp)
+
+
 def test_chain_terms_past_the_end_of_a_walk_do_not_count(ctx):
     """Terms are tested ahead of a walk: one at 2^62 or beyond is an error only
     where the walk reaches it (2^62 is the domain of the reference's PrimeQ)."""
