@@ -161,68 +161,94 @@ __global__ void int_probe_kernel(int iters, unsigned *sink) {
 }
 
 // ---- PRP microbenchmark kernel: verdicts of sprp2 over an array ----------------
-// A block sorts its values: those of sprp2's small range and the others wait
-// in a queue each, and a queue is tested when a block's worth waits (the rest
-// at the end), so a warp runs only one form of the test.  With values spread
-// over the logarithm of [2^40, 2^63), of which 13% are not small, both forms
-// in most warps would cost twice the time.  A block takes `take` values at a
-// time; with take = half its threads, both queues' last tests run side by
-// side.
+// A block sorts up to SPRP_BATCH values by length, the longest first, and its
+// warps test them 32 at a time, as they come free: so the lanes of a warp do
+// equally many squares, and one form of the test serves them (the general one
+// where some value needs it).  The verdicts are gathered and written in the
+// order of the values.  Bound by the multiply pipe.  Unsorted, a warp of values
+// spread over the logarithm of [2^40, 2^63) did the squares of its longest, and
+// the block waited for it: 2^20 values 134 us, now 105 (2^24: 2.30 and 1.83 ms;
+// 2^20 of one length 112 and 105).  Batches of 2048 and four blocks an SM: 109.
 // The squarings go to squarings[warp of the grid], or added to *squarings.
+constexpr int SPRP_BATCH = 512, SPRP_GRID = 8;   // blocks an SM
 __global__ void __launch_bounds__(SPRP_BLOCK)
 sprp_batch_kernel(const uint64_t *N, long long count, uint8_t *verdict,
                   unsigned long long *squarings, int per_warp, int take) {
-  __shared__ uint64_t value[2][2 * SPRP_BLOCK];
-  __shared__ uint32_t index[2][2 * SPRP_BLOCK];
-  __shared__ int waiting[2];
+  constexpr int EACH = SPRP_BATCH / SPRP_BLOCK;     // values a thread sorts
+  __shared__ uint64_t value[SPRP_BATCH];
+  __shared__ uint16_t order[SPRP_BATCH];
+  __shared__ uint8_t result[SPRP_BATCH];
+  __shared__ int bin[32], next, valid;
   const int tid = threadIdx.x, lane = tid & 31, block = blockDim.x;
-  if (tid < 2) waiting[tid] = 0;
-  __syncthreads();
   unsigned sq = 0;
-  // takes n0 and n1 values off the queues, the second by whole other warps;
-  // called by all threads
-  auto test = [&](int n0, int n1) {
-    const int second = (n0 + 31) & ~31;
-    if (tid < n0) {
-      const int at = waiting[0] - n0 + tid;
-      verdict[index[0][at]] = (uint8_t)sprp2_as<true>(value[0][at], sq);
-    } else if (tid >= second && tid < second + n1) {
-      const int at = waiting[1] - n1 + tid - second;
-      verdict[index[1][at]] = (uint8_t)sprp2_as<false>(value[1][at], sq);
-    }
-    __syncthreads();
-    if (tid == 0) {
-      waiting[0] -= n0;
-      waiting[1] -= n1;
-    }
-    __syncthreads();
-  };
   for (long long i0 = blockIdx.x * (long long)take; i0 < count;
        i0 += (long long)gridDim.x * take) {
-    const long long i = i0 + tid;
-    const bool here = tid < take && i < count;
-    const uint64_t x = here ? N[i] : 0;
-    const bool valid = (x & 1) && x >= 3 && x < (1ull << 63);
-    if (here && !valid) verdict[i] = 0;
-    const bool small = valid && sprp2_small(x);
+    const int n = (int)min((long long)take, count - i0);
+    if (tid < 32) bin[tid] = 0;
+    __syncthreads();
+    // bins: general values of 63, 62 and 61 bits, small ones of 60 to 34 bits,
+    // and the few others that need the general form
+    int place[EACH];                  // bin << 16 | position in it, -1: not valid
 #pragma unroll
-    for (int form = 0; form < 2; form++) {
-      const bool mine = form ? valid && !small : small;
-      const unsigned bal = __ballot_sync(FULL, mine);
+    for (int u = 0; u < EACH; u++) {
+      const int i = tid + u * block;
+      const uint64_t x = i < n ? N[i0 + i] : 0;
+      const bool ok = (x & 1) && x >= 3 && x < (1ull << 63);
+      const int len = 64 - __clzll((long long)x);
+      const int key = !ok ? -1 : len > 60 || sprp2_small(x) ? 63 - len : 31;
+      place[u] = -1;
+      if (u * block >= n) continue;   // uniform
+      const unsigned same = __match_any_sync(FULL, key);
       int at = 0;
-      if (lane == 0 && bal) at = atomicAdd(&waiting[form], __popc(bal));
-      at = __shfl_sync(FULL, at, 0) + __popc(bal & ((1u << lane) - 1u));
-      if (mine) {
-        value[form][at] = x;
-        index[form][at] = (uint32_t)i;
+      if (ok && lane == __ffs(same) - 1) at = atomicAdd(&bin[key], __popc(same));
+      at = __shfl_sync(FULL, at, __ffs(same) - 1) + __popc(same & ((1u << lane) - 1u));
+      if (ok) place[u] = key << 16 | at;
+      if (i < n) {
+        value[i] = x;
+        result[i] = 0;
       }
     }
     __syncthreads();
-    if (waiting[0] >= block) test(block, 0);
-    if (waiting[1] >= block) test(0, block);
+    if (tid < 32) {
+      const int own = bin[tid];
+      int sum = own;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(FULL, sum, o);
+        if (lane >= o) sum += y;
+      }
+      bin[tid] = sum - own;
+      if (tid == 31) {
+        valid = sum;
+        next = 0;
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < EACH; u++)
+      if (place[u] >= 0) order[bin[place[u] >> 16] + (place[u] & 0xffff)] = (uint16_t)(tid + u * block);
+    __syncthreads();
+    for (;;) {
+      int at = 0;
+      if (lane == 0) at = atomicAdd(&next, 32);
+      at = __shfl_sync(FULL, at, 0);
+      if (at >= valid) break;
+      const bool mine = at + lane < valid;
+      const int i = order[mine ? at + lane : at];
+      const uint64_t x = value[i];
+      bool prp;
+      unsigned done = 0;
+      if (__all_sync(FULL, sprp2_small(x)))
+        prp = sprp2_as<true>(x, done);
+      else
+        prp = sprp2_as<false>(x, done);
+      if (mine) {
+        result[i] = (uint8_t)prp;
+        sq += done;
+      }
+    }
+    __syncthreads();
+    for (int i = tid; i < n; i += block) verdict[i0 + i] = result[i];
   }
-  if (((waiting[0] + 31) & ~31) + waiting[1] > block) test(waiting[0], 0);
-  test(waiting[0], waiting[1]);
   unsigned v = sq;
   for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
   if (lane == 0) {
@@ -2220,6 +2246,16 @@ extern "C" int ap26_sieve_count(ap26_ctx *ctx, const int32_t *Ks, int nK, int sh
   return AP26_OK;
 }
 
+// Values a block of sprp_batch_kernel takes at a time, and the blocks: one batch
+// each, in whole warps, unless it would be longer than the block can sort.
+static int sprp_take(const ap26_ctx *ctx, int64_t n, bool small, int *blocks) {
+  const int64_t most = (int64_t)ctx->num_sms * SPRP_GRID, each = ((n + most - 1) / most + 31) & ~31;
+  const int take = (int)(small ? std::min<int64_t>(std::max<int64_t>(each, 64), SPRP_BATCH / 2)
+                               : std::min<int64_t>(std::max<int64_t>(each, 256), SPRP_BATCH));
+  *blocks = (int)std::min<int64_t>((n + take - 1) / take, most);
+  return take;
+}
+
 extern "C" int ap26_sprp_batch(ap26_ctx *ctx, const uint64_t *N, int64_t count, uint8_t *verdict,
                                ap26_stats *stats) {
   if (!ctx || !N || !verdict || count < 0) return AP26_E_ARG;
@@ -2228,7 +2264,9 @@ extern "C" int ap26_sprp_batch(ap26_ctx *ctx, const uint64_t *N, int64_t count, 
   if (count == 0) return AP26_OK;
   // a short call's warps leave their counts behind the verdicts
   const bool small = count * (int64_t)sizeof(uint64_t) <= kZeroCopyBytes;
-  const int64_t warps = std::min<int64_t>((count + 63) / 64, ctx->num_sms * 4) * 4;
+  int small_blocks;
+  sprp_take(ctx, count, true, &small_blocks);
+  const int64_t warps = (int64_t)small_blocks * (SPRP_BLOCK / 2 / 32);
   unsigned long long *const tally =
       small ? (unsigned long long *)(ctx->sets[0].h_out + kZeroCopyBytes) : ctx->d_tally;
   if (!small) CK(cudaMemsetAsync(ctx->d_tally, 0, sizeof(*ctx->d_tally), ctx->stream));
@@ -2236,10 +2274,10 @@ extern "C" int ap26_sprp_batch(ap26_ctx *ctx, const uint64_t *N, int64_t count, 
   int rc = staged(
       ctx, count, {{(char *)N, sizeof(uint64_t)}}, {{(char *)verdict, 1}}, &ms,
       [&](int64_t n, const char *in, char *out, cudaStream_t s) {
-        const int block = small ? 128 : SPRP_BLOCK, take = small ? block / 2 : block;
-        const int64_t blocks = std::min<int64_t>((n + take - 1) / take, ctx->num_sms * 4);
-        sprp_batch_kernel<<<(int)blocks, block, 0, s>>>((const uint64_t *)in, n, (uint8_t *)out,
-                                                        tally, small, take);
+        int blocks;
+        const int take = sprp_take(ctx, n, small, &blocks);
+        sprp_batch_kernel<<<blocks, small ? SPRP_BLOCK / 2 : SPRP_BLOCK, 0, s>>>(
+            (const uint64_t *)in, n, (uint8_t *)out, tally, small, take);
         return cudaGetLastError();
       });
   if (rc != AP26_OK) return rc;

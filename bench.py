@@ -15,9 +15,10 @@ search).
   e2e      K/s wall-clock through the C ABI with host buffers: ap26_search_batch
            (raw reports, result_hash) and ap26_report_batch (SOL lines), with
            their host<->device copies; ReportSolution runs on the device
-  roofline the sieve kernel: algorithmic table bytes (16.62 mean
-           consults per shift word x 8 B, oracle-measured) / measured sieve
-           launch time, against the measured shared-memory peak
+  roofline the class sieve kernel: the table rows that its dense phase reads
+           (20 moduli x 64 bytes for every point and row that 71 does not
+           exclude) / measured sieve launch time, against the measured
+           shared-memory peak
   cpu_baseline  the reference CPU build (oracle/_ref/ref_harness: the
            reference's own Search_avx2) on every host core, bounded samples
   cpu_avx512    companion: the AVX-512 restatement of the same search
@@ -42,8 +43,11 @@ RANGE_K = 64
 STEP_K = 8
 SHIFT = 0
 N59_PER_K = 4808136200          # lattice positions per K (10840 n43 x 443555)
-CONSULTS_PER_WORD = 16.62       # oracle: mean table lookups per shift word (canonical order)
-BYTES_PER_CONSULT = 8
+# The class sieve's dense rows, per lattice value and shift word: a point is 8
+# lattice values of 10 words each, its (b, j) that pass 61 and 67 fill 4 rows of
+# 512 bits, 27.6% of their quarters are excluded by 71, and the others are read
+# in the tables of 20 moduli.
+ROW_BYTES_PER_CELL = 4 * 64 * 20 * 0.724 / 80
 # H2D/D2H payload per K-job and per call (sizes of the C ABI structures)
 KJOB_BYTES, DEVSTATE_BYTES, APREC_BYTES, COUNT_BYTES, FINAL_BYTES = 128, 128, 24, 8, 56
 REF_HARNESS = os.path.join(ROOT, "oracle", "_ref", "ref_harness")
@@ -320,9 +324,9 @@ def run_reference(args, rank, world):
 
 
 # ---- secondary keys of the default line -------------------------------------------
-IMAD_PER_MULMOD = 12   # 32-bit multiply-adds of one 64-bit Montgomery product:
-                       # 4 for a*b, 3 for m = lo*n', 4 for hi(m*N), 1 carry
-ALG_BYTES_PER_K = N59_PER_K * 10 * CONSULTS_PER_WORD * BYTES_PER_CONSULT
+IMAD_PER_MULMOD = 9    # 32 x 32 products of one 64-bit Montgomery square:
+                       # 3 for x*x, 3 for m = lo*n', 3 for the high half of m*N
+ALG_BYTES_PER_K = N59_PER_K * 10 * ROW_BYTES_PER_CELL
 
 
 def _mixed_items(rng, n, max_len, shifts=(0, 640, 1280)):
@@ -522,7 +526,7 @@ def measure_sieve_pair(ctx, A, smem_gbs, n=SIEVE_PAIR_K):
         sieve_ms += st.sieve_ms
         cells += st.sieve_cells
     counts = np.concatenate(counts)
-    achieved = cells * CONSULTS_PER_WORD * BYTES_PER_CONSULT / (sieve_ms / 1e3) / 1e9
+    achieved = cells * ROW_BYTES_PER_CELL / (sieve_ms / 1e3) / 1e9
     pinned = ref_counts()
     chk = [(k, int(c), pinned[(k, SIEVE_PAIR_SHIFT)]) for k, c in zip(ks, counts)
            if (k, SIEVE_PAIR_SHIFT) in pinned]
@@ -532,7 +536,7 @@ def measure_sieve_pair(ctx, A, smem_gbs, n=SIEVE_PAIR_K):
         "k_count": len(ks), "kps": len(ks) / (dev_ms / 1e3),
         "raw_kps": len(ks) / (dev_ms / 1e3),
         "roofline": {"bound": "smem", "achieved": achieved, "peak": smem_gbs, "unit": "GB/s",
-                     "frac": achieved / smem_gbs, "kernel": "sieve_kernel"},
+                     "frac": achieved / smem_gbs, "kernel": "class_sieve_kernel"},
         "survivors_total": int(counts.sum()),
         "parity": {"k_checked_vs_reference": len(chk),
                    "mismatched": [k for k, c, r in chk if c != r],
@@ -770,7 +774,7 @@ def main():
     if rank == 0:
         sieve_launch_ms = tot["sieve_ms"] / max(1, tot["launches"])
         cells_per_launch = tot["cells"] / max(1, tot["launches"])
-        alg_bytes = cells_per_launch * CONSULTS_PER_WORD * BYTES_PER_CONSULT
+        alg_bytes = cells_per_launch * ROW_BYTES_PER_CELL
         achieved = alg_bytes / (sieve_launch_ms / 1000.0) / 1e9
         hash_par = {"items": 0, "ok": True}
         for h, a, b in item_hash.values():
@@ -793,8 +797,8 @@ def main():
                        "kmin": KMIN_SEEDED, "k_per_rank": RANGE_K, "shift": SHIFT,
                        "searched_k": int(ks_total), "raw_k": int(raw_total),
                        "parallelism": f"replicas x{world} (disjoint K ranges)",
-                       "l2": "working set is an 11 KB table per K in shared memory; no "
-                             "HBM-resident inputs to flush",
+                       "l2": "row tables in shared memory, a 15 MB plan per K built on the "
+                             "device; no HBM-resident inputs to flush",
                        "autotuned": tuned},
             "raw_kps": raw_total / (dev_ms / 1000.0),
             "e2e": {"value": ks_total / wall_max, "unit": "K/s",
@@ -807,8 +811,8 @@ def main():
                          "unit": "GB/s", "frac": achieved / smem_gbs,
                          "traffic": cells_per_launch * SIEVE_DRAM_BYTES_PER_CELL,
                          "traffic_unit": "DRAM bytes per launch",
-                         "kernel": "sieve_kernel",
-                         "note": "algorithmic bytes = cells x 16.62 consults x 8 B; peak = "
+                         "kernel": "class_sieve_kernel",
+                         "note": "algorithmic bytes = cells x 46.3 B of the 20 dense moduli's rows; peak = "
                                  "measured conflict-free LDS.128 bandwidth of this GPU "
                                  "(ap26_probe_peaks); HBM and tensor cores are not on the path",
                          "launch_ms": sieve_launch_ms, "int_tops_peak": int_tops,

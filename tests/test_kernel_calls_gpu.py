@@ -89,6 +89,28 @@ def test_sprp_forms_at_their_limits(ctx, oracle):
         assert np.array_equal(got, exp), a
 
 
+@pytest.mark.parametrize("n", [1, 31, 33, 64, 65, 255, 257, 18_943, 131_072, 131_073,
+                               606_208, 606_209])
+def test_sprp_batches_of_mixed_lengths_keep_their_order(ctx, oracle, n):
+    """Values are tested in the order of their length, a block's batch at a
+    time: verdicts and squarings belong to their values at the edges of warps,
+    batches and grids, with values that are not tested among them."""
+    rng = np.random.default_rng(7)
+    some = np.exp2(rng.uniform(1, 63.9, 2000)).astype(np.uint64) | np.uint64(1)
+    some[::7] += np.uint64(1)                    # even
+    some[:4] = 0, 1, 2, 3
+    some[4:400] = [p for p in range(1 << 40, (1 << 40) + 20000) if _is_prime(p)][:396]
+    tested = (some & np.uint64(1) > 0) & (some >= 3) & (some < np.uint64(1 << 63))
+    exp = np.array([t and oracle.ao_sprp(ctypes.c_int64(int(x)), ctypes.c_int64(2))
+                    for x, t in zip(some, tested)], np.uint8)
+    assert 300 < exp.sum() < 800
+    each = np.array([ctx.sprp_batch(some[i:i + 1])[1].late_items for i in range(len(some))])
+    pick = rng.integers(0, len(some), n)
+    got, st = ctx.sprp_batch(some[pick])
+    assert np.array_equal(got, exp[pick])
+    assert st.late_items == each[pick].sum()
+
+
 def _is_prime(n):
     return all(n == p or (n % p and _strong(n, p)) for p in (2, 3, 5, 7, 11, 13, 17, 19, 23, 29, 31, 37))
 
