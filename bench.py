@@ -591,14 +591,12 @@ def measure_sprp(ctx, A, int_tops, log2=24):
 
 
 # ---- our arm ---------------------------------------------------------------------
-# DRAM bytes per sieve cell: dram__bytes_read.sum + dram__bytes_write.sum of a
-# 131072-tile launch (1.174e10 cells) of the default variant in one ncu
-# capture, 137.7 MB read + 137.1 MB written (mean of three launches, which
-# agree within 1%).  Nearly all of it is the candidate ring: about 9.5 M
-# survivors x 16 B written, and the L2's fills of the partly written sectors
-# read back; it grows with the survivors, so with the cells, and scales to
-# any launch.
-SIEVE_DRAM_BYTES_PER_CELL = (137.67e6 + 137.15e6) / (131072 * 256 * 35 * 10)
+# DRAM bytes per sieve cell: dram__bytes_read.sum + dram__bytes_write.sum of the
+# one class sieve launch of a K (4.808e10 cells) in an ncu capture, 637.3 MB read
+# + 623.3 MB written.  Nearly all of it is the candidate ring: 38.8 M survivors
+# x 16 B written, and the L2's fills of the partly written sectors read back; it
+# grows with the survivors, so with the cells, and scales to any launch.
+SIEVE_DRAM_BYTES_PER_CELL = (637.27e6 + 623.30e6) / (N59_PER_K * 10)
 
 
 def main():

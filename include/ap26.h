@@ -49,7 +49,9 @@ extern "C" {
 typedef struct ap26_ctx ap26_ctx;
 
 /* Tuning knobs; zero fields take the context's defaults (or autotuned values,
- * see ap26_autotune). */
+ * see ap26_autotune).  dense_primes, warp_queue, block_threads, late_stage and
+ * tail_group choose a variant of the window sieve, which serves parts of a K
+ * (ap26_sieve_range); the class sieve of whole K has one form. */
 typedef struct {
   int32_t dense_primes;   /* primes sieved for all 10 words before compaction */
   int32_t warp_queue;     /* per-warp shared-memory queue depth (items)       */
@@ -103,7 +105,9 @@ typedef struct {
 typedef struct {
   int64_t candidates;   /* sieve survivors after the 7..23 filter; the
                            reference's "total n" (src/opencl/AP26.h:343)     */
-  int64_t late_items;   /* shift words that reached the late sieve stage     */
+  int64_t late_items;   /* shift words (of a whole K: candidates) that reached
+                           the late sieve stages; ap26_sprp_batch: modular
+                           squarings                                         */
   int64_t prp_tests;    /* base-2 SPRP tests run by the chain walk           */
   int64_t aps;          /* raw reports (k >= 10)                             */
   double device_ms;     /* CUDA-event time of the device work                */
