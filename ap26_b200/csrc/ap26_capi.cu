@@ -343,7 +343,7 @@ static cudaError_t upload_constants() {
     single[i] = make_param_p(PRIMES[FIRST_SINGLE + i], single_off(i));
   ResParam res[NDENSE + 2];
   int str[NDENSE], slot[NSLOTS];
-  uint16_t task[NTASKS];
+  uint16_t task[NTASKS], inv[NDENSE];
   int nt = 0;
   for (int k = 0; k < NDENSE + 2; k++) {
     const PrimeParam p =
@@ -351,9 +351,16 @@ static cudaError_t upload_constants() {
     res[k] = ResParam{p.p, p.A, p.B, p.C, p.k, p.M};
     if (k >= NDENSE) continue;
     str[k] = dense_str_off(k);
-    for (int b = 0; b < (DENSE_M[k] + 31) / 32; b++)
-      for (int w = 0; w < 4; w++) task[nt++] = (uint16_t)(k | b << 5 | w << 8);
+    inv[k] = (uint16_t)dense_inv(DENSE_M[k]);
   }
+  // the long tasks first
+  for (int blocks = 3; blocks > 0; blocks--)
+    for (int k = 0; k < NDENSE; k++)
+      for (int half = 0; half < 2; half++) {
+        const int n = row_blocks(k), first = half ? (n + 1) / 2 : 0;
+        if ((half ? n / 2 : (n + 1) / 2) != blocks) continue;
+        for (int w = 0; w < 4; w++) task[nt++] = (uint16_t)(k | first << 5 | blocks << 8 | w << 10);
+      }
   for (int i = 0; i < NSLOTS; i++) slot[i] = slot_base(i);
   cudaError_t e;
   if ((e = cudaMemcpyToSymbol(c_triples, trip, sizeof(trip))) != cudaSuccess) return e;
@@ -361,6 +368,7 @@ static cudaError_t upload_constants() {
   if ((e = cudaMemcpyToSymbol(c_single, single, sizeof(single))) != cudaSuccess) return e;
   if ((e = cudaMemcpyToSymbol(c_res, res, sizeof(res))) != cudaSuccess) return e;
   if ((e = cudaMemcpyToSymbol(c_task, task, sizeof(task))) != cudaSuccess) return e;
+  if ((e = cudaMemcpyToSymbol(c_dense_inv, inv, sizeof(inv))) != cudaSuccess) return e;
   if ((e = cudaMemcpyToSymbol(c_dense_str, str, sizeof(str))) != cudaSuccess) return e;
   return cudaMemcpyToSymbol(c_slot_base, slot, sizeof(slot));
 }

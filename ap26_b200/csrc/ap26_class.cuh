@@ -38,11 +38,12 @@
 // 331 ms.  Classes alone took 156 ms, with 71 skipped by quarters and the
 // masks queued in 64-bit halves 140 ms, with the last single primes in two
 // stages and every shared address a constant (80 registers, hardly a spill)
-// 130 in one launch, where that had taken 135.  It is bound by shared memory
+// 129.1 in one launch, where that had taken 135, and with the rows built in
+// half the time 127.6.  It is bound by shared memory
 // and L1: 91% of their wavefront slots (issue 67%), half of them the dense
 // rows', 14% the v records' (the four quarters read four parts of a bucket),
 // the rest the queues and the lookups of the tail, most of them in stage A.
-// Of the 135 ms, building the rows took 3, reading them 82, the masks' queue
+// Of the 135 ms, a unit's list took 1, building the rows 3, reading them 82, the masks' queue
 // and stage A 33, the stages behind it 18.  Warps: 16 with more registers 143
 // ms, 20 132, 22 131, 24 130, 26 and 28 143.  22 dense moduli, which only fit
 // with 20 warps, gained 0.6 ms; v records as one 256-bit load lost 5, a branch
@@ -112,13 +113,16 @@ constexpr int dense_str_off(int k) {
 }
 constexpr int DENSE_STR_WORDS = dense_str_off(NDENSE);
 
-// Row-building tasks: (modulus, 32 rows, 128 bits) triples.
-constexpr int build_tasks() {
-  int t = 0;
-  for (int k = 0; k < NDENSE; k++) t += (DENSE_M[k] + 31) / 32 * 4;
-  return t;
-}
-constexpr int NTASKS = build_tasks();
+// Row-building tasks: half of a modulus's blocks of 32 rows, 128 bits of each.
+// Bound by instructions.  A bit's residue is found once a task and serves its
+// two or three blocks; found for each block, with a division by the modulus, and
+// with a transposition of 25 instructions where 13 do, the rows of a K took 3.2
+// ms, now 1.7.
+constexpr int row_blocks(int k) { return (DENSE_M[k] + 31) / 32; }
+constexpr int NTASKS = NDENSE * 2 * 4;
+static_assert(row_blocks(0) >= 2 && (row_blocks(NDENSE - 1) + 1) / 2 < 4, "task fields");
+// v / m = v * DENSE_INV >> 20 for v below 5 m and 2^20 / m
+constexpr uint32_t dense_inv(int m) { return ((1u << 20) + m - 1) / m; }
 
 // Tail moduli: products of two or three primes, one lookup each (about 3.4
 // wavefronts at 32 random bits), then the remaining primes singly.
@@ -174,7 +178,8 @@ struct ResParam { int p, A, B, C, k; uint32_t M; };
 constexpr int RES_CLASS = NDENSE, RES_SKIP = NDENSE + 1;
 __constant__ ResParam c_res[NDENSE + 2];
 __constant__ PrimeParam c_single[NSINGLE];     // off: word of the tail strings
-__constant__ uint16_t c_task[NTASKS];          // modulus | row block << 5 | 128-bit word << 8
+__constant__ uint16_t c_task[NTASKS];          // modulus | row block << 5 | blocks << 8 | 128-bit word << 10
+__constant__ uint16_t c_dense_inv[NDENSE];
 __constant__ int c_dense_str[NDENSE];          // word offset of a modulus's string
 __constant__ int c_slot_base[NSLOTS];
 
@@ -501,16 +506,33 @@ __device__ __forceinline__ bool tail_test(uint32_t x, uint32_t y,
 
 // Transposes the 32 x 32 bit matrix whose row r is lane r's word: lane s
 // gets bit s of every row, row r at bit r.
-__device__ __forceinline__ uint32_t transpose32(uint32_t x, int lane) {
-  uint32_t m = 0x0000ffffu;
+// The lane exchanges 16, 8, 4, 2 and 1 bits with the lane that far away: halves
+// and bytes by one permutation, the others by a rotation and a select, whose
+// selectors depend on the lane alone.
+struct Transpose {
+  uint32_t half, byte, mask[3], turn[3];
+  __device__ __forceinline__ explicit Transpose(int lane) {
+    half = lane & 16 ? 0x3276 : 0x5410;
+    byte = lane & 8 ? 0x3715 : 0x6240;
 #pragma unroll
-  for (int j = 16; j; j >>= 1) {
-    const uint32_t y = __shfl_xor_sync(FULL, x, j);
-    x = lane & j ? (x & ~m) | ((y >> j) & m) : (x & m) | ((y << j) & ~m);
-    m ^= m << (j >> 1);
+    for (int i = 0; i < 3; i++) {
+      const int j = 4 >> i;
+      const uint32_t low = j == 4 ? 0x0f0f0f0fu : j == 2 ? 0x33333333u : 0x55555555u;
+      mask[i] = lane & j ? ~low : low;         // bits that stay
+      turn[i] = lane & j ? 32 - j : j;
+    }
   }
-  return x;
-}
+  __device__ __forceinline__ uint32_t operator()(uint32_t x) const {
+    x = __byte_perm(x, __shfl_xor_sync(FULL, x, 16), half);
+    x = __byte_perm(x, __shfl_xor_sync(FULL, x, 8), byte);
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      const uint32_t y = __shfl_xor_sync(FULL, x, 4 >> i);
+      x = (x & mask[i]) | (__funnelshift_l(y, y, turn[i]) & ~mask[i]);
+    }
+    return x;
+  }
+};
 
 // acc &= the two rows of slot k.  w holds residue bytes of v (its slot's in
 // the low or high half), u the slot's packed residues of x and the lane's
@@ -796,28 +818,37 @@ __global__ void __launch_bounds__(CLASS_WARPS * 32, 1) class_sieve_kernel(ClassA
       }
       __syncthreads();
 
-      // rows of every dense modulus: 32 rows x 128 bits a task
-      for (int t = warp; t < NTASKS; t += CLASS_WARPS) {
-        const uint32_t task = c_task[t];
-        const int k = task & 31, s0 = (int)((task >> 5) & 7) * 32, wq = (int)(task >> 8);
-        const int m = c_res[k].p;
-        const uint32_t *str = P.dense_str + c_dense_str[k];
-        uint32_t w[4];
+      // rows of every dense modulus
+      {
+        const Transpose transpose(lane);
+        for (int t = warp; t < NTASKS; t += CLASS_WARPS) {
+          const uint32_t task = c_task[t];
+          const int k = task & 31, wq = (int)(task >> 10), m = c_res[k].p;
+          const uint32_t *str = P.dense_str + c_dense_str[k];
+          int at[4];
+          uint32_t here[4];
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
-          const int e = wq * 128 + u * 32 + lane;
-          uint32_t x = 0;
-          if (e < ne) {
-            const int b = eb[e], j = ev[e] & 0x3ff;
-            const int at = (P.bres[k][b] + j + m - MAX_WRAPS) % m + s0;
-            x = __funnelshift_r(str[at >> 5], str[(at >> 5) + 1], at & 31);
+          for (int u = 0; u < 4; u++) {
+            const int e = wq * 128 + u * 32 + lane;
+            here[u] = e < ne ? FULL : 0u;
+            const uint32_t v = e < ne ? P.bres[k][eb[e]] + (ev[e] & 0x3ff) + m - MAX_WRAPS : 0;
+            at[u] = (int)(v - (v * c_dense_inv[k] >> 20) * m);
           }
-          w[u] = transpose32(x, lane);
+          int block = (task >> 5) & 7;
+          for (const int end = block + (int)((task >> 8) & 3); block < end; block++) {
+            uint32_t w[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+              const uint32_t *from = str + (at[u] >> 5) + block;
+              w[u] = transpose(__funnelshift_r(from[0], from[1], at[u] & 31) & here[u]);
+            }
+            const int row = block * 32 + lane;
+            if (row < m)
+              *reinterpret_cast<uint4 *>(rows + c_slot_base[k >> 1] + row * ROW_STRIDE +
+                                         (k & 1) * (ROW_BITS / 8) + wq * 16) =
+                  make_uint4(w[0], w[1], w[2], w[3]);
+          }
         }
-        if (s0 + lane < m)
-          *reinterpret_cast<uint4 *>(rows + c_slot_base[k >> 1] + (s0 + lane) * ROW_STRIDE +
-                                     (k & 1) * (ROW_BITS / 8) + wq * 16) =
-              make_uint4(w[0], w[1], w[2], w[3]);
       }
       __syncthreads();
 
