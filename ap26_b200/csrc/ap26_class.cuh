@@ -38,8 +38,8 @@
 // 331 ms.  Classes alone took 156 ms, with 71 skipped by quarters and the
 // masks queued in 64-bit halves 140 ms, with the last single primes in two
 // stages and every shared address a constant (80 registers, hardly a spill)
-// 129.1 in one launch, where that had taken 135, and with the rows built in
-// half the time 127.6.  It is bound by shared memory
+// 129.1 in one launch, where that had taken 135, with the rows built in half
+// the time 127.6 and with the units' lists made by coordinate 126.5.  It is bound by shared memory
 // and L1: 91% of their wavefront slots (issue 67%), half of them the dense
 // rows', 14% the v records' (the four quarters read four parts of a bucket),
 // the rest the queues and the lookups of the tail, most of them in stage A.
@@ -769,23 +769,25 @@ __global__ void __launch_bounds__(CLASS_WARPS * 32, 1) class_sieve_kernel(ClassA
     // row h of the class, then h + 4, ... while the class has more (b, j)
     // than four rows hold
     for (int h = unit % ROWS_PER_CLASS;; h += ROWS_PER_CLASS) {
-      // the (b, j) that pass 61 and 67, in the order of their coordinate
-      // mod 71: LIST slots (coordinate, b, one of its j), EACH a thread
-      constexpr int JS = (J_COUNT + SKIP - 1) / SKIP;       // j of one coordinate, 10
-      constexpr int LIST = SKIP * NB * JS;
-      constexpr int EACH = (LIST + CLASS_WARPS * 32 - 1) / (CLASS_WARPS * 32);
+      // the (b, j) that pass 61 and 67, in the order of their coordinate mod
+      // 71: a thread has one coordinate and b, whose j are SKIP apart (eight
+      // consecutive entries a thread, each divided into coordinate, b and j,
+      // took 1.2 ms of a K and spilled registers, this 0.8)
+      constexpr int JS = (J_COUNT + SKIP - 1) / SKIP;       // at most 10 of them
+      static_assert(SKIP * NB <= CLASS_WARPS * 32, "a thread for each coordinate and b");
+      const int o = threadIdx.x / NB, b = threadIdx.x % NB;
+      const int j0 = (o * P.skip_inv + SKIP - P.bskip[b]) % SKIP;
       uint32_t mine = 0;
+      if (o < SKIP) {
+        int at = cls + P.bres[RES_CLASS][b] + j0 - MAX_WRAPS;
+        at += at < 0 ? CLASSES : 0;
+        at -= at >= CLASSES ? CLASSES : 0;
+        at -= at >= CLASSES ? CLASSES : 0;
 #pragma unroll
-      for (int u = 0; u < EACH; u++) {
-        const int slot = (int)threadIdx.x * EACH + u;
-        if (slot < LIST) {
-          const int o = slot / (NB * JS), b = slot / JS % NB;
-          const int j = (o * P.skip_inv + SKIP - P.bskip[b]) % SKIP + slot % JS * SKIP;
-          int at = cls + P.bres[RES_CLASS][b] + j - MAX_WRAPS;
-          at += at < 0 ? CLASSES : 0;
+        for (int u = 0; u < JS; u++) {
+          if (j0 + u * SKIP < J_COUNT && (table[at >> 5] >> (at & 31) & 1u)) mine |= 1u << u;
+          at += SKIP;
           at -= at >= CLASSES ? CLASSES : 0;
-          at -= at >= CLASSES ? CLASSES : 0;
-          if (j < J_COUNT && (table[at >> 5] >> (at & 31) & 1u)) mine |= 1u << u;
         }
       }
       int before = __popc(mine);
@@ -807,10 +809,8 @@ __global__ void __launch_bounds__(CLASS_WARPS * 32, 1) class_sieve_kernel(ClassA
       if (e0 >= total) break;                  // uniform over the CTA
       const int ne = min(ROW_BITS, total - e0);
       for (; mine; mine &= mine - 1) {
-        const int slot = (int)threadIdx.x * EACH + __ffs(mine) - 1, e = before++ - e0;
+        const int j = j0 + (__ffs(mine) - 1) * SKIP, e = before++ - e0;
         if (e < 0 || e >= ROW_BITS) continue;
-        const int o = slot / (NB * JS), b = slot / JS % NB;
-        const int j = (o * P.skip_inv + SKIP - P.bskip[b]) % SKIP + slot % JS * SKIP;
         ev[e] = (uint16_t)(P.bmul[b] << 10 | j);
         eb[e] = (uint8_t)b;
         if ((e & 127) == 0) s_o0[e >> 7] = o;
