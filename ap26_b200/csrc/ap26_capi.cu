@@ -930,7 +930,9 @@ static int staged(ap26_ctx *ctx, int64_t count, std::initializer_list<Column> in
   ctx->team.run(team, work);
   *ms = total;
   if (failed.load()) {
-    // nothing may still write the buffers when the next call reuses them
+    // nothing may still read or write the buffers when the next call reuses them
+    for (cudaStream_t v : ctx->copy_in)
+      if (v) cudaStreamSynchronize(v);
     cudaStreamSynchronize(ctx->stream);
     cudaStreamSynchronize(ctx->back_stream);
     return cuda_fail(ctx, (cudaError_t)failed.load(), "staged call");
