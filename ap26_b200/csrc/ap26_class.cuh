@@ -39,12 +39,13 @@
 // masks queued in 64-bit halves 140 ms, with the last single primes in two
 // stages and every shared address a constant (80 registers, hardly a spill)
 // 129.1 in one launch, where that had taken 135, with the rows built in half
-// the time 127.6 and with the units' lists made by coordinate 126.5.  It is bound by shared memory
-// and L1: 91% of their wavefront slots (issue 67%), half of them the dense
-// rows', 14% the v records' (the four quarters read four parts of a bucket),
-// the rest the queues and the lookups of the tail, most of them in stage A.
-// Of the 135 ms, a unit's list took 1, building the rows 3, reading them 82, the masks' queue
-// and stage A 33, the stages behind it 18.  Warps: 16 with more registers 143
+// the time 127.6 and with the units' lists made by coordinate 126.5.  It is
+// bound by shared memory and L1: 91% of their wavefront slots (issue 67%), half
+// of them the dense rows', 14% the v records' (the four quarters read four parts
+// of a bucket), the rest the queues and the lookups of the tail, most of them in
+// stage A.  Of the 135 ms, a unit's list took 1, building the rows 3 (now 0.8 and
+// 1.7), reading them 82, the masks' queue and stage A 33, the stages behind it
+// 18.  Warps: 16 with more registers 143
 // ms, 20 132, 22 131, 24 130, 26 and 28 143.  22 dense moduli, which only fit
 // with 20 warps, gained 0.6 ms; v records as one 256-bit load lost 5, a branch
 // around the tail lookups of dead lanes 1, two or four products in stage A 1,
@@ -121,8 +122,10 @@ constexpr int DENSE_STR_WORDS = dense_str_off(NDENSE);
 constexpr int row_blocks(int k) { return (DENSE_M[k] + 31) / 32; }
 constexpr int NTASKS = NDENSE * 2 * 4;
 static_assert(row_blocks(0) >= 2 && (row_blocks(NDENSE - 1) + 1) / 2 < 4, "task fields");
-// v / m = v * DENSE_INV >> 20 for v below 5 m and 2^20 / m
+// v / m = v * dense_inv(m) >> 20 for every v with v * m < 2^20: s(b) + j + m stays below
+// 2 m + J_COUNT
 constexpr uint32_t dense_inv(int m) { return ((1u << 20) + m - 1) / m; }
+static_assert((2 * DENSE_M[NDENSE - 1] + J_COUNT) * DENSE_M[NDENSE - 1] < 1 << 20, "exact quotient");
 
 // Tail moduli: products of two or three primes, one lookup each (about 3.4
 // wavefronts at 32 random bits), then the remaining primes singly.
