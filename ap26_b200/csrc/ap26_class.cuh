@@ -40,7 +40,7 @@
 // stages and every shared address a constant (80 registers, hardly a spill)
 // 129.1 in one launch, where that had taken 135, with the rows built in half
 // the time 127.6 and with the units' lists made by coordinate 126.5.  It is
-// bound by shared memory and L1: 91% of their wavefront slots (issue 67%), half
+// bound by shared memory and L1: 92% of their wavefront slots (issue 64%), half
 // of them the dense rows', 14% the v records' (the four quarters read four parts
 // of a bucket), the rest the queues and the lookups of the tail, most of them in
 // stage A.  Of the 135 ms, a unit's list took 1, building the rows 3 (now 0.8 and
