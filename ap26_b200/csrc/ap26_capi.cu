@@ -2382,9 +2382,12 @@ extern "C" int ap26_chain_batch(ap26_ctx *ctx, int K, const int64_t *n, int64_t 
   drain(ctx);
   if (count == 0) return AP26_OK;
   JobSet &S = ctx->main;
+  int rc;
+  // none is left of a set that a longer batch could not grow
+  if ((rc = jobset_ensure(ctx, S, 1)) != AP26_OK) return rc;
   memset(S.h_st, 0, sizeof(DevState));     // pinned: the kernel sets its error flags there
   double ms = 0;
-  int rc = staged(
+  rc = staged(
       ctx, count, {{(char *)n, sizeof(int64_t)}},
       {{(char *)first_out, sizeof(int64_t)}, {(char *)k_out, sizeof(int32_t)}}, &ms,
       [&](int64_t m, const char *in, char *out, cudaStream_t s) {

@@ -1,0 +1,100 @@
+"""The host code where a CUDA call fails, and where it has to count or to wait.
+
+The library's own objects are linked with tests/fake_cuda.cpp, a runtime whose
+kernels do nothing and whose calls fail when a test says so: no GPU is used and
+none is needed.  A test runs in a process of its own, so that a crash or a hang
+of the library is a failed test.
+"""
+import glob
+import importlib.util
+import os
+import shutil
+import subprocess
+import sys
+import textwrap
+
+import pytest
+
+from conftest import ROOT
+
+PRELUDE = """
+import ctypes, os, sys, time
+import numpy as np
+sys.path.insert(0, {root!r})
+import ap26_b200 as A
+A.LIB_PATH = {lib!r}
+A.lib = fake = A._load()
+fake.fake_fail.argtypes = [ctypes.c_char_p] + [ctypes.c_int] * 3
+OOM, OTHER = 2, 999        # cudaErrorMemoryAllocation, cudaErrorUnknown
+ALL = 1 << 30
+def fail(call, skip=0, times=ALL, code=OTHER):
+    fake.fake_fail(call.encode(), skip, times, code)
+"""
+
+
+def _built_objects():
+    """The library's objects, brought up to date as the build does it."""
+    spec = importlib.util.spec_from_file_location(
+        "ap26_build", os.path.join(ROOT, "ap26_b200", "build.py"))
+    build = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(build)
+    objs = [os.path.join(build.BUILD, f) for f in ("ap26_capi.o", "ap26_host.o")]
+    srcs = glob.glob(os.path.join(build.CSRC, "*")) + [os.path.join(ROOT, "include", "ap26.h")]
+    if not all(build._newer(o, srcs) for o in objs):
+        if not os.path.exists(build.NVCC):
+            pytest.skip("the library's objects are not built")
+        build.build()
+    return objs
+
+
+@pytest.fixture(scope="module")
+def fake_lib(tmp_path_factory):
+    inc = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
+    if shutil.which("g++") is None or not os.path.exists(os.path.join(inc, "cuda_runtime_api.h")):
+        pytest.skip("no host C++ compiler or no CUDA headers")
+    so = str(tmp_path_factory.mktemp("fake") / "libap26_fake.so")
+    subprocess.run(["g++", "-O1", "-fPIC", "-shared", "-std=c++17", "-Wl,-Bsymbolic", "-I", inc,
+                    os.path.join(ROOT, "tests", "fake_cuda.cpp")] + _built_objects() +
+                   ["-lpthread", "-o", so], check=True)
+    return so
+
+
+@pytest.fixture
+def child(fake_lib):
+    def run(code, timeout=60):
+        p = subprocess.run([sys.executable, "-c",
+                            PRELUDE.format(root=ROOT, lib=fake_lib) + textwrap.dedent(code)],
+                           capture_output=True, text=True, timeout=timeout)
+        assert p.returncode == 0, (p.returncode, p.stdout, p.stderr)
+        return p.stdout
+    return run
+
+
+def test_chain_walks_after_the_job_set_could_not_grow(child):
+    """A batch of more K than the job set holds frees it to make a larger one.
+    Where that fails the batch fails, and the calls after it get a set of their
+    own or an error: chain_batch keeps its error flags there."""
+    child("""
+        ctx = A.Context(0, cand_ring_log2=12)
+        n = np.arange(1, 2001, 2, dtype=np.int64)
+        ctx.chain_batch(1, n)
+        fail("cudaMalloc", code=OOM)
+        try:
+            ctx.sieve_count(range(1, 200), 0)
+            raise SystemExit("no memory, and a count all the same")
+        except A.AP26Error as e:
+            assert e.code == A.E_CUDA
+        for _ in range(2):
+            try:
+                ctx.chain_batch(1, n)
+                raise SystemExit("no memory, and a walk all the same")
+            except A.AP26Error as e:
+                assert e.code == A.E_CUDA
+        fail("cudaMalloc", times=0)
+        try:
+            ctx.chain_batch(1, n)
+        except A.AP26Error:               # the failed call's own pending error
+            pass
+        ctx.chain_batch(1, n)
+        ctx.close()
+    """)
