@@ -1265,14 +1265,20 @@ static int ensure_prof_events(ap26_ctx *ctx, unsigned long long n) {
   return AP26_OK;
 }
 
-// Enqueues one K-job's plan.
+// Enqueues one K-job's plan.  Stops at the first error, which it takes: none is
+// left pending.
 static cudaError_t emit_plan(const KJob *job, ClassPlan *plan, int num_sms, cudaStream_t s) {
-  cudaError_t e = cudaMemsetAsync(plan->vfill, 0, sizeof(plan->vfill), s);
-  if (e != cudaSuccess) return e;
+  cudaError_t e;
+  cudaMemsetAsync(plan->vfill, 0, sizeof(plan->vfill), s);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
   class_plan_count_kernel<<<num_sms * 4, 256, 0, s>>>(job, plan);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
   class_plan_sum_kernel<<<(CLASSES + 7) / 8, 256, 0, s>>>(plan);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
   class_plan_scan_kernel<<<1, 1024, 0, s>>>(plan);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
   class_plan_start_kernel<<<(CLASSES + 7) / 8, 256, 0, s>>>(plan);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
   class_plan_scatter_kernel<<<num_sms * 8, 256, 0, s>>>(job, plan);
   return cudaGetLastError();
 }
@@ -2609,6 +2615,7 @@ extern "C" int ap26_sieve_count_noalloc(int device, const int32_t *d_Ks, int nK,
           break;
         }
         class_begin_kernel<<<1, 1, 0, s>>>(&S->st, 0);
+        if (noalloc_launch_failed()) { rc = AP26_E_CUDA; break; }
         class_sieve_kernel<<<d->num_sms, CLASS_WARPS * 32, CLASS_SMEM, s>>>(
             class_args(S->jobs, j, &S->plan, &S->tables[0][0], &S->st, 0, UNITS_PER_K, d->num_sms,
                        nullptr, 0, &S->st.cand_count[0], S->counts, 1));

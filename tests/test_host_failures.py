@@ -98,3 +98,27 @@ def test_chain_walks_after_the_job_set_could_not_grow(child):
         ctx.chain_batch(1, n)
         ctx.close()
     """)
+
+
+def test_noalloc_takes_the_errors_of_its_own_launches(child):
+    """A pending error is the caller's: the call that finds one launches nothing.
+    So a call that fails leaves none of its own, whichever launch failed, and
+    launches nothing after it."""
+    child("""
+        Ks = (ctypes.c_int32 * 2)(1, 2)
+        out = (ctypes.c_int64 * 2)()
+        def count():
+            before = fake.fake_launches()
+            rc = A.lib.ap26_sieve_count_noalloc(0, Ks, 2, 0, out, None)
+            return rc, fake.fake_launches() - before
+        rc, launches = count()
+        assert rc == A.OK and launches == 2 + 2 * 7 + 1
+        for call, steps in (("cudaMemsetAsync", 2), ("cudaLaunchKernel", launches)):
+            for i in range(steps):
+                fail(call, skip=i, times=1)
+                rc, done = count()
+                assert rc == A.E_CUDA, (call, i)
+                assert done == (i if call == "cudaLaunchKernel" else 2 + 7 * i), (call, i, done)
+                assert fake.cudaPeekAtLastError() == 0, (call, i)
+                assert count() == (A.OK, launches), (call, i)
+    """)
