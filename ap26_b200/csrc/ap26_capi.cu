@@ -821,8 +821,8 @@ static void stage_free(ap26_ctx *ctx) {
 // Runs `count` values, given in the arrays `in`, through a kernel that fills
 // the arrays `out`.  launch(n, in, out, stream) starts it on n values, whose
 // arrays lie one after the other in its buffers.  Kernels run in ctx->stream,
-// behind whatever is queued there; *ms is the sum of their times.  Returns
-// once all is done.
+// behind whatever is queued there; *ms is the sum of their times, *launches
+// their number.  Returns once all is done.
 //
 // The time of a long call is its copies: ap26_sprp_batch of 2^24 values spent
 // 16 of 18.4 ms in one thread's pageable copies and in allocations.  Here its
@@ -833,12 +833,14 @@ static void stage_free(ap26_ctx *ctx) {
 // (61 values 62 us, now 32).
 template <class Launch>
 static int staged(ap26_ctx *ctx, int64_t count, std::initializer_list<Column> in,
-                  std::initializer_list<Column> out, double *ms, const Launch &launch) {
+                  std::initializer_list<Column> out, double *ms, int32_t *launches,
+                  const Launch &launch) {
   int64_t in_per = 0, out_per = 0;
   for (const Column &c : in) in_per += c.size;
   for (const Column &c : out) out_per += c.size;
   const int64_t per = std::max(in_per, out_per);
   *ms = 0;
+  *launches = 1;
   // part [from, to) of a slice of n values that starts with value `first`
   const auto fill = [&](char *buf, int64_t first, int64_t n, int64_t from, int64_t to) {
     for (const Column &c : in) {
@@ -866,6 +868,7 @@ static int staged(ap26_ctx *ctx, int64_t count, std::initializer_list<Column> in
     return AP26_OK;
   }
   const int64_t slice = kSetBytes / per, slices = (count + slice - 1) / slice;
+  *launches = (int32_t)slices;
   const int team = ctx->team.size((int)std::max<int64_t>(
       1, std::min<int64_t>({(int64_t)kTeam, (int64_t)std::thread::hardware_concurrency(),
                             count * (in_per + out_per) / kThreadBytes})));
@@ -2216,6 +2219,7 @@ extern "C" int ap26_sieve_range(ap26_ctx *ctx, int K, int shift, int64_t q_begin
   *n_cand = nc;
   if (nc > ctx->cand_cap) return AP26_E_OVERFLOW;
   if (nc > cap) return AP26_E_CAPACITY;
+  int32_t launches = 2;
   for (long long at = 0; at < nc; at += most) {
     const long long n = std::min(most, nc - at);
     if (at > 0) {
@@ -2223,6 +2227,7 @@ extern "C" int ap26_sieve_range(ap26_ctx *ctx, int K, int shift, int64_t q_begin
                                                      most, (int64_t *)G.h_out);
       CK(cudaGetLastError());
       CK(cudaStreamSynchronize(s));
+      launches++;
     }
     memcpy(cand + at, G.h_out, sizeof(int64_t) * n);
   }
@@ -2234,7 +2239,7 @@ extern "C" int ap26_sieve_range(ap26_ctx *ctx, int K, int shift, int64_t q_begin
     stats->late_items = (int64_t)S.h_st->late_items;
     stats->device_ms = ms;
     stats->error_flags = (int32_t)S.h_st->err_flags;
-    stats->launches = 2;
+    stats->launches = launches;
   }
   return AP26_OK;
 }
@@ -2287,8 +2292,9 @@ extern "C" int ap26_sprp_batch(ap26_ctx *ctx, const uint64_t *N, int64_t count, 
       small ? (unsigned long long *)(ctx->sets[0].h_out + kZeroCopyBytes) : ctx->d_tally;
   if (!small) CK(cudaMemsetAsync(ctx->d_tally, 0, sizeof(*ctx->d_tally), ctx->stream));
   double ms = 0;
+  int32_t launches = 0;
   int rc = staged(
-      ctx, count, {{(char *)N, sizeof(uint64_t)}}, {{(char *)verdict, 1}}, &ms,
+      ctx, count, {{(char *)N, sizeof(uint64_t)}}, {{(char *)verdict, 1}}, &ms, &launches,
       [&](int64_t n, const char *in, char *out, cudaStream_t s) {
         int blocks;
         const int take = sprp_take(ctx, n, small, &blocks);
@@ -2307,7 +2313,7 @@ extern "C" int ap26_sprp_batch(ap26_ctx *ctx, const uint64_t *N, int64_t count, 
     stats->prp_tests = count;
     stats->device_ms = ms;
     stats->late_items = (int64_t)hsq;   // modular squarings performed
-    stats->launches = 1;
+    stats->launches = launches;
   }
   return AP26_OK;
 }
@@ -2322,9 +2328,10 @@ extern "C" int ap26_sprp_bases(ap26_ctx *ctx, const uint64_t *N, const uint32_t 
   if (count == 0) return AP26_OK;
   drain(ctx);
   double ms = 0;
+  int32_t launches = 0;
   int rc = staged(
       ctx, count, {{(char *)N, sizeof(uint64_t)}, {(char *)a, sizeof(uint32_t)}},
-      {{(char *)verdict, 1}}, &ms,
+      {{(char *)verdict, 1}}, &ms, &launches,
       [&](int64_t n, const char *in, char *out, cudaStream_t s) {
         const int64_t blocks = std::min<int64_t>((n + 63) / 64, ctx->num_sms * 32);
         sprp_bases_kernel<<<(int)blocks, 64, 0, s>>>(
@@ -2337,7 +2344,7 @@ extern "C" int ap26_sprp_bases(ap26_ctx *ctx, const uint64_t *N, const uint32_t 
     memset(stats, 0, sizeof(*stats));
     stats->prp_tests = count;
     stats->device_ms = ms;
-    stats->launches = 1;
+    stats->launches = launches;
   }
   return AP26_OK;
 }
@@ -2351,8 +2358,9 @@ extern "C" int ap26_report_batch(ap26_ctx *ctx, const ap26_ap *raw, int64_t n, a
   if (n == 0) return AP26_OK;
   drain(ctx);
   double ms = 0;
+  int32_t launches = 0;
   int rc = staged(
-      ctx, n, {{(char *)raw, sizeof(APRec)}}, {{(char *)out, sizeof(FinRec)}}, &ms,
+      ctx, n, {{(char *)raw, sizeof(APRec)}}, {{(char *)out, sizeof(FinRec)}}, &ms, &launches,
       [&](int64_t m, const char *in, char *fin, cudaStream_t s) {
         // ap26_ap and APRec share a layout; with jobs == null the job field is K
         ReportArgs ra;
@@ -2369,7 +2377,7 @@ extern "C" int ap26_report_batch(ap26_ctx *ctx, const ap26_ap *raw, int64_t n, a
   if (stats) {
     stats->aps = n;
     stats->device_ms = ms;
-    stats->launches = 1;
+    stats->launches = launches;
   }
   unsigned long long add = 0;
   for (int64_t i = 0; i < n; i++) {
@@ -2393,9 +2401,10 @@ extern "C" int ap26_chain_batch(ap26_ctx *ctx, int K, const int64_t *n, int64_t 
   if ((rc = jobset_ensure(ctx, S, 1)) != AP26_OK) return rc;
   memset(S.h_st, 0, sizeof(DevState));     // pinned: the kernel sets its error flags there
   double ms = 0;
+  int32_t launches = 0;
   rc = staged(
       ctx, count, {{(char *)n, sizeof(int64_t)}},
-      {{(char *)first_out, sizeof(int64_t)}, {(char *)k_out, sizeof(int32_t)}}, &ms,
+      {{(char *)first_out, sizeof(int64_t)}, {(char *)k_out, sizeof(int32_t)}}, &ms, &launches,
       [&](int64_t m, const char *in, char *out, cudaStream_t s) {
         const int64_t blocks = std::min<int64_t>((m + 63) / 64, ctx->num_sms * 16);
         chain_explicit_kernel<<<(int)blocks, CHAIN_WARPS * 32, 0, s>>>(
@@ -2408,7 +2417,7 @@ extern "C" int ap26_chain_batch(ap26_ctx *ctx, int K, const int64_t *n, int64_t 
     memset(stats, 0, sizeof(*stats));
     stats->device_ms = ms;
     stats->error_flags = (int32_t)S.h_st->err_flags;
-    stats->launches = 1;
+    stats->launches = launches;
   }
   return (S.h_st->err_flags & ERR_DOMAIN) ? AP26_E_DOMAIN : AP26_OK;
 }

@@ -24,6 +24,7 @@ std::map<const void *, std::string> g_names;  // host stub -> kernel
 std::map<const void *, std::pair<void *, size_t>> g_vars;
 std::vector<std::string> g_launched;
 int g_slow_ms = 0;
+struct Patch { size_t bytes, offset; unsigned long long value; } g_patch = {};
 
 cudaError_t result(const char *call) {
   std::lock_guard<std::mutex> lock(g_mu);
@@ -44,8 +45,12 @@ void fake_fail(const char *call, int skip, int times, int code) {
   g_failures[call] = Failure{skip, times, (cudaError_t)code};
 }
 int fake_launches(void) { return (int)g_launched.size(); }
-// Every host-to-device copy of the next call's first slice takes this long.
-void fake_slow_copies(int ms) { g_slow_ms = ms; }
+// The next copy to the device takes this long.
+void fake_slow_copy(int ms) { g_slow_ms = ms; }
+// The next copy of `bytes` bytes back to the host has `value` at `offset`.
+void fake_read_back(size_t bytes, size_t offset, unsigned long long value) {
+  g_patch = Patch{bytes, offset, value};
+}
 
 // ---- the runtime's --------------------------------------------------------------
 #define FAKE(name, args, ...)                       \
@@ -71,6 +76,10 @@ cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind kin
   const cudaError_t e = result("cudaMemcpyAsync");
   if (e != cudaSuccess) return e;
   memcpy(d, s, n);
+  if (kind == cudaMemcpyDeviceToHost && n == g_patch.bytes) {
+    memcpy((char *)d + g_patch.offset, &g_patch.value, sizeof(g_patch.value));
+    g_patch.bytes = 0;
+  }
   int ms = 0;
   if (kind == cudaMemcpyHostToDevice) {
     std::lock_guard<std::mutex> lock(g_mu);

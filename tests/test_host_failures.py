@@ -25,6 +25,7 @@ import ap26_b200 as A
 A.LIB_PATH = {lib!r}
 A.lib = fake = A._load()
 fake.fake_fail.argtypes = [ctypes.c_char_p] + [ctypes.c_int] * 3
+fake.fake_read_back.argtypes = [ctypes.c_size_t, ctypes.c_size_t, ctypes.c_ulonglong]
 OOM, OTHER = 2, 999        # cudaErrorMemoryAllocation, cudaErrorUnknown
 ALL = 1 << 30
 def fail(call, skip=0, times=ALL, code=OTHER):
@@ -121,4 +122,35 @@ def test_noalloc_takes_the_errors_of_its_own_launches(child):
                 assert done == (i if call == "cudaLaunchKernel" else 2 + 7 * i), (call, i, done)
                 assert fake.cudaPeekAtLastError() == 0, (call, i)
                 assert count() == (A.OK, launches), (call, i)
+    """)
+
+
+def test_launches_of_long_calls_are_counted(child):
+    """stats.launches of a call that is cut in slices counts each slice's kernel;
+    a range's candidates behind the first 2^20 take a kernel for each 2^20."""
+    child("""
+        ctx = A.Context(0, cand_ring_log2=12)
+        def launched(call):
+            before = fake.fake_launches()
+            st = call()
+            return fake.fake_launches() - before, st.launches
+        for n, slices in ((1, 1), (1 << 17, 1), (1 << 20, 1), ((1 << 20) + 1, 2), (5 << 20, 5)):
+            N = np.full(n, 9, np.uint64)
+            assert launched(lambda: ctx.sprp_batch(N)[1]) == (slices, slices), n
+        n = 3_000_001
+        a = np.full(n, 2, np.uint32)
+        assert launched(lambda: ctx.sprp_bases(np.full(n, 9, np.uint64), a)[1]) == (5, 5)
+        assert launched(lambda: ctx.chain_batch(1, np.full(n, 9, np.int64))[2]) == (5, 5)
+        reps, fin, st = np.zeros(n, A._AP), np.zeros(n, "V56"), A.Stats()
+        def report():
+            A.lib.ap26_report_batch(ctx.h, A._ptr(reps), n, A._ptr(fin), None, ctypes.byref(st))
+            return st
+        assert launched(report) == (21, 21)
+        DEVSTATE, CAND_COUNT = 128, 40
+        for n, more in ((0, 0), (1 << 20, 0), ((1 << 20) + 1, 1), (5 << 20, 4)):
+            with A.Context(0, cand_ring_log2=23) as big:
+                fake.fake_read_back(DEVSTATE, CAND_COUNT, n)
+                call = lambda: big.sieve_range(1, 0, 0, A.N53_PER_K, cap=1 << 23)
+                assert launched(lambda: call()[1]) == (2 + more, 2 + more), n
+        ctx.close()
     """)
