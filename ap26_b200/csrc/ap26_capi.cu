@@ -886,9 +886,13 @@ static int staged(ap26_ctx *ctx, int64_t count, std::initializer_list<Column> in
     // slice i's results, this thread's part
     const auto take = [&](int64_t i) {
       StageSet &G = ctx->sets[i % kSets];
-      // its kernel is launched by whoever fills it last
-      while (filled[(size_t)i].load() < team + 1)
+      // its kernel is launched by whoever fills it last, mostly at once; a thread
+      // that the system holds back gets the processors of those that wait
+      for (int spins = 0; filled[(size_t)i].load() < team + 1; spins++) {
         if (failed.load()) return;
+        if (spins < 200) std::this_thread::yield();
+        else std::this_thread::sleep_for(std::chrono::microseconds(20));
+      }
       if (!ok(cudaEventSynchronize(G.back))) return;
       if (t == 0) {
         float ms1 = 0;

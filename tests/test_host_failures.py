@@ -154,3 +154,21 @@ def test_launches_of_long_calls_are_counted(child):
                 assert launched(lambda: call()[1]) == (2 + more, 2 + more), n
         ctx.close()
     """)
+
+
+def test_threads_of_a_long_call_do_not_spin_while_one_is_late(child):
+    """A slice's kernel starts when every thread has copied its part.  A thread
+    that the system holds back keeps the others waiting: they wait asleep, and
+    leave it their share of the processor time."""
+    child("""
+        ctx = A.Context(0, cand_ring_log2=12)
+        N = np.full(1 << 22, 9, np.uint64)
+        ctx.sprp_batch(N)                       # starts the threads
+        fake.fake_slow_copy(1000)
+        cpu, wall = time.process_time(), time.perf_counter()
+        ctx.sprp_batch(N)
+        cpu, wall = time.process_time() - cpu, time.perf_counter() - wall
+        assert wall >= 1, wall
+        assert cpu < 0.5 * wall, (cpu, wall)
+        ctx.close()
+    """)
