@@ -775,7 +775,17 @@ static int cuda_fail(ap26_ctx *ctx, cudaError_t e, const char *what) {
 
 constexpr int kChainThreads = 256;   // chain_kernel block size
 
-static cudaError_t stage_ensure(ap26_ctx *ctx, int sets, int team) {
+static void set_free(StageSet &G) {
+  cudaFree(G.d_in);
+  cudaFree(G.d_out);
+  cudaFreeHost(G.h_in);
+  cudaFreeHost(G.h_out);
+  G.d_in = G.d_out = G.h_in = G.h_out = nullptr;
+}
+
+// Makes sure of *sets sets and of the copy streams of *team threads, or, where
+// memory runs out, of as many as there are, at least one (the context's own).
+static cudaError_t stage_ensure(ap26_ctx *ctx, int *sets, int *team) {
   cudaError_t e = cudaSuccess;
   const auto event = [&](cudaEvent_t &v, unsigned flags) {
     if (e == cudaSuccess && !v) e = cudaEventCreateWithFlags(&v, flags);
@@ -783,7 +793,14 @@ static cudaError_t stage_ensure(ap26_ctx *ctx, int sets, int team) {
   const auto stream = [&](cudaStream_t &v) {
     if (e == cudaSuccess && !v) e = cudaStreamCreateWithFlags(&v, cudaStreamNonBlocking);
   };
-  for (int i = 0; i < sets; i++) {
+  // number i (from 0) was not to be had: the ones before it serve
+  const auto enough = [&](int i) {
+    if (e != cudaErrorMemoryAllocation || i == 0) return false;
+    cudaGetLastError();
+    e = cudaSuccess;
+    return true;
+  };
+  for (int i = 0; i < *sets; i++) {
     StageSet &G = ctx->sets[i];
     event(G.k0, cudaEventDefault);
     event(G.k1, cudaEventDefault);
@@ -793,9 +810,18 @@ static cudaError_t stage_ensure(ap26_ctx *ctx, int sets, int team) {
     if (e == cudaSuccess && !G.h_out) e = cudaMallocHost(&G.h_out, kSetBytes);
     if (e == cudaSuccess && !G.d_in) e = cudaMalloc(&G.d_in, kSetBytes);
     if (e == cudaSuccess && !G.d_out) e = cudaMalloc(&G.d_out, kSetBytes);
+    if (e == cudaSuccess) continue;
+    set_free(G);
+    if (!enough(i)) return e;
+    *sets = i;
   }
-  for (int t = 0; t < team; t++) stream(ctx->copy_in[t]);
   stream(ctx->back_stream);
+  for (int t = 0; t < *team; t++) {
+    stream(ctx->copy_in[t]);
+    if (e == cudaSuccess) continue;
+    if (!enough(t)) return e;
+    *team = t;
+  }
   return e;
 }
 
@@ -804,10 +830,7 @@ static void stage_free(ap26_ctx *ctx) {
     if (v) cudaStreamSynchronize(v);
   if (ctx->back_stream) cudaStreamSynchronize(ctx->back_stream);
   for (StageSet &G : ctx->sets) {
-    cudaFree(G.d_in);
-    cudaFree(G.d_out);
-    cudaFreeHost(G.h_in);
-    cudaFreeHost(G.h_out);
+    set_free(G);
     for (cudaEvent_t v : {G.k0, G.k1, G.back})
       if (v) cudaEventDestroy(v);
     for (cudaEvent_t v : G.in)
@@ -826,7 +849,7 @@ static void stage_free(ap26_ctx *ctx) {
 //
 // The time of a long call is its copies: ap26_sprp_batch of 2^24 values spent
 // 16 of 18.4 ms in one thread's pageable copies and in allocations.  Here its
-// slices go through kSets sets of buffers, each slice filled and emptied by
+// slices go through up to kSets sets of buffers, each slice filled and emptied by
 // up to kTeam threads, so that copies, transfers both ways and kernels
 // overlap.  The time of a short call is its number of driver calls: it has
 // one launch and one wait, and the kernel reaches the pinned buffers itself
@@ -869,10 +892,11 @@ static int staged(ap26_ctx *ctx, int64_t count, std::initializer_list<Column> in
   }
   const int64_t slice = kSetBytes / per, slices = (count + slice - 1) / slice;
   *launches = (int32_t)slices;
-  const int team = ctx->team.size((int)std::max<int64_t>(
+  int team = ctx->team.size((int)std::max<int64_t>(
       1, std::min<int64_t>({(int64_t)kTeam, (int64_t)std::thread::hardware_concurrency(),
                             count * (in_per + out_per) / kThreadBytes})));
-  CK(stage_ensure(ctx, (int)std::min<int64_t>(slices, kSets), team));
+  int sets = (int)std::min<int64_t>(slices, kSets);
+  CK(stage_ensure(ctx, &sets, &team));
   std::vector<std::atomic<int>> filled((size_t)slices);   // threads done with a slice's copies
   std::atomic<int> failed{0};
   double total = 0;
@@ -885,7 +909,7 @@ static int staged(ap26_ctx *ctx, int64_t count, std::initializer_list<Column> in
     const auto part = [&](int64_t n, int k) { return n * k / team; };
     // slice i's results, this thread's part
     const auto take = [&](int64_t i) {
-      StageSet &G = ctx->sets[i % kSets];
+      StageSet &G = ctx->sets[i % sets];
       // its kernel is launched by whoever fills it last, mostly at once; a thread
       // that the system holds back gets the processors of those that wait
       for (int spins = 0; filled[(size_t)i].load() < team + 1; spins++) {
@@ -903,8 +927,8 @@ static int staged(ap26_ctx *ctx, int64_t count, std::initializer_list<Column> in
       empty(G.h_out, first, n, part(n, t), part(n, t + 1));
     };
     for (int64_t i = 0; i < slices && e == cudaSuccess && !failed.load(); i++) {
-      StageSet &G = ctx->sets[i % kSets];
-      if (i >= kSets) take(i - kSets);
+      StageSet &G = ctx->sets[i % sets];
+      if (i >= sets) take(i - sets);
       if (e != cudaSuccess || failed.load()) break;
       const int64_t first = i * slice, n = std::min(slice, count - first);
       const int64_t from = part(n, t), to = part(n, t + 1);
@@ -929,7 +953,7 @@ static int staged(ap26_ctx *ctx, int64_t count, std::initializer_list<Column> in
       ok(cudaEventRecord(G.back, ctx->back_stream));
       if (e == cudaSuccess) filled[(size_t)i].fetch_add(1);
     }
-    for (int64_t i = std::max<int64_t>(0, slices - kSets);
+    for (int64_t i = std::max<int64_t>(0, slices - sets);
          i < slices && e == cudaSuccess && !failed.load(); i++)
       take(i);
     if (e != cudaSuccess) failed.store((int)e);
@@ -1122,7 +1146,8 @@ extern "C" int ap26_create(int device, const ap26_opts *opts, ap26_ctx **out) {
                              CLASS_SMEM));
     CKC(cudaMalloc(&ctx->d_plan, sizeof(ClassPlan)));
     CKC(cudaMalloc(&ctx->d_tally, sizeof(unsigned long long)));
-    CKC(stage_ensure(ctx, 1, 1));
+    int sets = 1, team = 1;
+    CKC(stage_ensure(ctx, &sets, &team));
     // buffers
     if (ctx->opts.cand_ring_log2 < 12 || ctx->opts.cand_ring_log2 > 27 ||
         ctx->opts.batch_wave > kMaxBatchWave) {

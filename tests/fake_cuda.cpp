@@ -33,9 +33,18 @@ cudaError_t result(const char *call) {
   if (--f->second.from >= 0 || f->second.times-- <= 0) return cudaSuccess;
   return g_last = f->second.code;
 }
+bool g_no_host_memory = false;
 struct Launch { dim3 grid, block; size_t smem; cudaStream_t stream; };
 thread_local std::vector<Launch> g_config;
 }  // namespace
+
+void *operator new(size_t n) {
+  void *p = g_no_host_memory ? nullptr : malloc(n ? n : 1);
+  if (!p) throw std::bad_alloc();
+  return p;
+}
+void operator delete(void *p) noexcept { free(p); }
+void operator delete(void *p, size_t) noexcept { free(p); }
 
 extern "C" {
 // ---- the test's side -------------------------------------------------------------
@@ -51,6 +60,9 @@ void fake_slow_copy(int ms) { g_slow_ms = ms; }
 void fake_read_back(size_t bytes, size_t offset, unsigned long long value) {
   g_patch = Patch{bytes, offset, value};
 }
+
+// operator new fails, as when the host has no memory left.
+void fake_no_host_memory(int on) { g_no_host_memory = on != 0; }
 
 // ---- the runtime's --------------------------------------------------------------
 #define FAKE(name, args, ...)                       \

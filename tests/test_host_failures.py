@@ -172,3 +172,23 @@ def test_threads_of_a_long_call_do_not_spin_while_one_is_late(child):
         assert cpu < 0.5 * wall, (cpu, wall)
         ctx.close()
     """)
+
+
+def test_long_calls_with_memory_for_one_set_of_buffers(child):
+    """The context has one set of buffers from the start.  A long call uses three;
+    where there is no memory for the others it goes through those there are, and
+    a later one gets the rest."""
+    child("""
+        ctx = A.Context(0, cand_ring_log2=12)
+        n = (5 << 20) + 3
+        N = np.arange(n, dtype=np.uint64)
+        a = np.full(n, 2, np.uint32)
+        for call in ("cudaMalloc", "cudaHostAlloc"):
+            for skip in (0, 1):                  # the first or the second buffer
+                fail(call, skip=skip, code=OOM)
+                assert ctx.sprp_batch(N)[1].launches == 6
+                assert ctx.sprp_bases(N, a)[1].launches == 8
+                fail(call, times=0)
+        assert ctx.sprp_batch(N)[1].launches == 6
+        ctx.close()
+    """)
