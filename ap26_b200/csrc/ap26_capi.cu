@@ -915,7 +915,7 @@ static int staged(ap26_ctx *ctx, int64_t count, std::initializer_list<Column> in
       for (int spins = 0; filled[(size_t)i].load() < team + 1; spins++) {
         if (failed.load()) return;
         if (spins < 200) std::this_thread::yield();
-        else std::this_thread::sleep_for(std::chrono::microseconds(20));
+        else std::this_thread::sleep_for(std::chrono::microseconds(20 << std::min(spins - 200, 6)));
       }
       if (!ok(cudaEventSynchronize(G.back))) return;
       if (t == 0) {
