@@ -897,7 +897,9 @@ static int staged(ap26_ctx *ctx, int64_t count, std::initializer_list<Column> in
                             count * (in_per + out_per) / kThreadBytes})));
   int sets = (int)std::min<int64_t>(slices, kSets);
   CK(stage_ensure(ctx, &sets, &team));
-  std::vector<std::atomic<int>> filled((size_t)slices);   // threads done with a slice's copies
+  // how far each set has come, over all of its slices: one for each thread that
+  // has copied its part of a slice in, and one for the slice's launch
+  std::atomic<int64_t> filled[kSets] = {};
   std::atomic<int> failed{0};
   double total = 0;
   const auto work = [&](int t) {
@@ -912,7 +914,7 @@ static int staged(ap26_ctx *ctx, int64_t count, std::initializer_list<Column> in
       StageSet &G = ctx->sets[i % sets];
       // its kernel is launched by whoever fills it last, mostly at once; a thread
       // that the system holds back gets the processors of those that wait
-      for (int spins = 0; filled[(size_t)i].load() < team + 1; spins++) {
+      for (int spins = 0; filled[i % sets].load() < (i / sets + 1) * (team + 1); spins++) {
         if (failed.load()) return;
         if (spins < 200) std::this_thread::yield();
         else std::this_thread::sleep_for(std::chrono::microseconds(20 << std::min(spins - 200, 6)));
@@ -941,7 +943,7 @@ static int staged(ap26_ctx *ctx, int64_t count, std::initializer_list<Column> in
       }
       ok(cudaEventRecord(G.in[t], ctx->copy_in[t]));
       if (e != cudaSuccess) break;
-      if (filled[(size_t)i].fetch_add(1) != team - 1) continue;
+      if (filled[i % sets].fetch_add(1) != i / sets * (team + 1) + team - 1) continue;
       // the last thread to fill the slice starts its kernel
       for (int k = 0; k < team; k++) ok(cudaStreamWaitEvent(ctx->stream, G.in[k], 0));
       ok(cudaEventRecord(G.k0, ctx->stream));
@@ -951,14 +953,14 @@ static int staged(ap26_ctx *ctx, int64_t count, std::initializer_list<Column> in
       ok(cudaMemcpyAsync(G.h_out, G.d_out, (size_t)(n * out_per), cudaMemcpyDeviceToHost,
                          ctx->back_stream));
       ok(cudaEventRecord(G.back, ctx->back_stream));
-      if (e == cudaSuccess) filled[(size_t)i].fetch_add(1);
+      if (e == cudaSuccess) filled[i % sets].fetch_add(1);
     }
     for (int64_t i = std::max<int64_t>(0, slices - sets);
          i < slices && e == cudaSuccess && !failed.load(); i++)
       take(i);
     if (e != cudaSuccess) failed.store((int)e);
   };
-  ctx->team.run(team, work);
+  ctx->team.run(team, std::ref(work));       // by reference: no copy on the heap
   *ms = total;
   if (failed.load()) {
     // nothing may still read or write the buffers when the next call reuses them

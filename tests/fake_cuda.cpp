@@ -26,7 +26,15 @@ std::vector<std::string> g_launched;
 int g_slow_ms = 0;
 struct Patch { size_t bytes, offset; unsigned long long value; } g_patch = {};
 
+// The fake's own containers always have memory.
+thread_local int g_inside = 0;
+struct Inside {
+  Inside() { g_inside++; }
+  ~Inside() { g_inside--; }
+};
+
 cudaError_t result(const char *call) {
+  Inside inside;
   std::lock_guard<std::mutex> lock(g_mu);
   auto f = g_failures.find(call);
   if (f == g_failures.end()) return cudaSuccess;
@@ -39,7 +47,7 @@ thread_local std::vector<Launch> g_config;
 }  // namespace
 
 void *operator new(size_t n) {
-  void *p = g_no_host_memory ? nullptr : malloc(n ? n : 1);
+  void *p = g_no_host_memory && !g_inside ? nullptr : malloc(n ? n : 1);
   if (!p) throw std::bad_alloc();
   return p;
 }
@@ -138,6 +146,7 @@ const char *cudaGetErrorString(cudaError_t) { return "an error of the test's"; }
 cudaError_t cudaLaunchKernel(const void *f, dim3, dim3, void **, size_t, cudaStream_t) {
   const cudaError_t e = result("cudaLaunchKernel");
   if (e != cudaSuccess) return e;
+  Inside inside;
   std::lock_guard<std::mutex> lock(g_mu);
   g_launched.push_back(g_names[f]);
   return cudaSuccess;
@@ -145,6 +154,7 @@ cudaError_t cudaLaunchKernel(const void *f, dim3, dim3, void **, size_t, cudaStr
 
 // what the compiler's stubs call
 unsigned __cudaPushCallConfiguration(dim3 grid, dim3 block, size_t smem, cudaStream_t s) {
+  Inside inside;
   g_config.push_back(Launch{grid, block, smem, s});
   return 0;
 }

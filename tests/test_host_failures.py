@@ -192,3 +192,18 @@ def test_long_calls_with_memory_for_one_set_of_buffers(child):
         assert ctx.sprp_batch(N)[1].launches == 6
         ctx.close()
     """)
+
+
+def test_long_calls_need_no_host_memory_of_their_own(child):
+    """No exception leaves a C entry point: a long call allocates nothing on the
+    host but its threads, and does without those."""
+    child("""
+        ctx = A.Context(0, cand_ring_log2=12)
+        N = np.arange(5 << 20, dtype=np.uint64)
+        v, st = np.empty(len(N), np.uint8), A.Stats()
+        fake.fake_no_host_memory(1)
+        rc = A.lib.ap26_sprp_batch(ctx.h, A._ptr(N), len(N), A._ptr(v), ctypes.byref(st))
+        fake.fake_no_host_memory(0)
+        assert rc == A.OK and st.launches == 5
+        ctx.close()
+    """)
