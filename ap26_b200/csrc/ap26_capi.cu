@@ -17,11 +17,14 @@
 #include <deque>
 #include <functional>
 #include <initializer_list>
+#include <memory>
 #include <string>
 #include <mutex>
 #include <system_error>
 #include <thread>
 #include <vector>
+
+#include <unistd.h>
 
 #include "../../include/ap26.h"
 #include "ap26_class.cuh"
@@ -646,7 +649,8 @@ struct Column {
 
 // The host threads of staged calls: started with the first call that wants
 // them (starting one takes 20-30 us, as long as a short call), asleep between
-// calls, ended with the context.  One call at a time uses them.
+// calls, ended with the context.  One call at a time uses them.  They are not
+// there in a child that the process forked: see ours().
 class Team {
  public:
   ~Team() {
@@ -657,8 +661,14 @@ class Team {
     wake_.notify_all();
     for (std::thread &t : threads_) t.join();
   }
+  // Whether the threads are this process's.  A forked child has copies of the
+  // objects but no threads: joining them, or destroying what they wait on, hangs
+  // or crashes.
+  bool ours() const { return threads_.empty() || pid_ == getpid(); }
   // Threads a call can have, itself included: `wanted`, or fewer where no more start.
   int size(int wanted) {
+    if (!ours()) return 1;
+    pid_ = getpid();
     try {
       while ((int)threads_.size() + 1 < wanted) {
         const int i = (int)threads_.size() + 1;
@@ -706,6 +716,7 @@ class Team {
     }
   }
   std::vector<std::thread> threads_;
+  pid_t pid_ = 0;
   std::mutex mu_;
   std::condition_variable wake_, done_;
   const std::function<void(int)> *job_ = nullptr;
@@ -745,7 +756,7 @@ struct ap26_ctx {
   UnitState *d_units = nullptr;                // kUnitSlots serving-unit states
   std::vector<int> free_slots;
   StageSet sets[kSets];
-  Team team;
+  std::unique_ptr<Team> team{new Team};
   cudaStream_t copy_in[kTeam] = {};            // one thread's copies each
   cudaStream_t back_stream = nullptr;          // results
   unsigned long long *d_tally = nullptr;       // squarings of an ap26_sprp_batch call
@@ -892,7 +903,7 @@ static int staged(ap26_ctx *ctx, int64_t count, std::initializer_list<Column> in
   }
   const int64_t slice = kSetBytes / per, slices = (count + slice - 1) / slice;
   *launches = (int32_t)slices;
-  int team = ctx->team.size((int)std::max<int64_t>(
+  int team = ctx->team->size((int)std::max<int64_t>(
       1, std::min<int64_t>({(int64_t)kTeam, (int64_t)std::thread::hardware_concurrency(),
                             count * (in_per + out_per) / kThreadBytes})));
   int sets = (int)std::min<int64_t>(slices, kSets);
@@ -960,7 +971,7 @@ static int staged(ap26_ctx *ctx, int64_t count, std::initializer_list<Column> in
       take(i);
     if (e != cudaSuccess) failed.store((int)e);
   };
-  ctx->team.run(team, std::ref(work));       // by reference: no copy on the heap
+  ctx->team->run(team, std::ref(work));       // by reference: no copy on the heap
   *ms = total;
   if (failed.load()) {
     // nothing may still read or write the buffers when the next call reuses them
@@ -1205,6 +1216,7 @@ extern "C" void ap26_destroy(ap26_ctx *ctx) {
   if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
   if (ctx->stream2) cudaStreamDestroy(ctx->stream2);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
+  if (!ctx->team->ours()) (void)ctx->team.release();
   delete ctx;
 }
 

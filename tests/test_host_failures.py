@@ -207,3 +207,29 @@ def test_long_calls_need_no_host_memory_of_their_own(child):
         assert rc == A.OK and st.launches == 5
         ctx.close()
     """)
+
+
+def test_a_forked_child_lets_go_of_the_context(child):
+    """The host threads of long calls are not there in a forked child: a context
+    that goes there, as an interpreter's last act, waits for none of them."""
+    child("""
+        ctx = A.Context(0, cand_ring_log2=12)
+        ctx.sprp_batch(np.full(1 << 22, 9, np.uint64))
+        pid = os.fork()
+        if pid == 0:
+            ctx.close()
+            os._exit(0)
+        end = time.time() + 20
+        while time.time() < end:
+            done, status = os.waitpid(pid, os.WNOHANG)
+            if done:
+                break
+            time.sleep(0.01)
+        else:
+            os.kill(pid, 9)
+            os.waitpid(pid, 0)
+            raise SystemExit("the child hangs")
+        assert status == 0, status
+        ctx.sprp_batch(np.full(1 << 22, 9, np.uint64))
+        ctx.close()
+    """)
