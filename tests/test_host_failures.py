@@ -233,3 +233,32 @@ def test_a_forked_child_lets_go_of_the_context(child):
         ctx.sprp_batch(np.full(1 << 22, 9, np.uint64))
         ctx.close()
     """)
+
+
+def test_reports_with_numbers_beyond_their_fields_reach_the_library(child):
+    """k, K, first and n go to the library as C integers of their fields, whatever
+    was given: a status for each report, and no exception of the binding's."""
+    child("""
+        ctx = A.Context(0, cand_ring_log2=12)
+        seen = []
+        real = fake.ap26_report_batch
+        class Lib:
+            def __getattr__(self, name):
+                return getattr(fake, name)
+            def ap26_report_batch(self, h, aps, n, *rest):
+                buf = aps if isinstance(aps, ctypes.Array) else ctypes.cast(aps, ctypes.POINTER(A.AP))
+                seen.append([(buf[i].k, buf[i].K, buf[i].first, buf[i].n) for i in range(n)])
+                return real(h, aps, n, *rest)
+        A.lib = Lib()
+        rows = [(10, 1 << 31, 31, 7), (1 << 32, 5, 1 << 63, -1), (-1, -(1 << 31) - 1, -(1 << 63), 2),
+                (10.0, 3, np.int64(37)), (11, 4, (1 << 64) + 3, 1 << 64)]
+        rc, fin, h = ctx.report_batch(rows, result_hash=5)
+        assert len(fin) == 5
+        want = [A.AP(int(r[0]), int(r[1]), int(r[2]), int(r[3]) if len(r) > 3 else 0) for r in rows]
+        assert seen == [[(w.k, w.K, w.first, w.n) for w in want]]
+        assert ctx.report_batch([])[1] == []
+        ordinary = [(10 + i, 366384, 10**15 + i, 10**15) for i in range(40)]
+        ctx.report_batch(ordinary)
+        assert seen[-1] == ordinary
+        ctx.close()
+    """)
