@@ -13,6 +13,7 @@ The reference interface it mirrors (ibethune/ap26):
   * ``hash_hex(...)`` <-> ``write_hash`` (AP26.cpp:295-357).
 """
 import ctypes
+import math
 import os
 
 import numpy as np
@@ -231,7 +232,8 @@ _AP = np.dtype([("k", np.int32), ("K", np.int32), ("first", np.int64), ("n", np.
 assert _AP.itemsize == ctypes.sizeof(AP)
 
 
-_DENSITY_PRIMES = (61, 67, 71, 73, 79, 83, 89, 97, 101, 103, 107, 109, 113, 127, 131, 137, 139)
+_SIEVE_PRIMES = [p for p in range(61, 542) if all(p % d for d in range(2, 24))]
+_SIEVE_PRODUCT = math.prod(_SIEVE_PRIMES)
 
 
 def _aps_to_list(arr, n):
@@ -367,8 +369,9 @@ class Context:
         # room for the survivors expected of this K (a prime that divides it
         # excludes one residue, not 24), the rest of cap only if they are more
         room = 0.37 * max(0, int(q1) - int(q0))
-        for p in _DENSITY_PRIMES:
-            if int(K) % p == 0:
+        common = math.gcd(int(K), _SIEVE_PRODUCT % max(1, int(K)))
+        for p in _SIEVE_PRIMES if common > 1 else ():
+            if common % p == 0:
                 room *= (p - 1) / (p - 24)
         room = min(int(cap), int(room) + 1024)
         n = ctypes.c_int64(0)

@@ -262,3 +262,31 @@ def test_reports_with_numbers_beyond_their_fields_reach_the_library(child):
         assert seen[-1] == ordinary
         ctx.close()
     """)
+
+
+@pytest.mark.parametrize("K", [43241061, 61 * 67 * 71 * 73, 149 * 151 * 157 * 113, 199 * 541,
+                               523 * 541, 139 * 149 * 151])
+def test_a_range_is_sieved_once_whatever_divides_k(child, K):
+    """The binding makes room for the candidates it expects and sieves again where
+    they are more: every sieve prime that divides K counts, so they are not."""
+    child(f"""
+        K, starts = {K}, 2_000_000
+        rooms = []
+        class Lib:
+            def __getattr__(self, name):
+                return getattr(fake, name)
+            def ap26_sieve_range(self, h, K, shift, q0, q1, cand, cap, n, st):
+                rooms.append(cap)
+                n._obj.value = found
+                return A.OK if found <= cap else A.E_CAPACITY
+        density = 36.9e6 / A.N53_PER_K           # of a K that no sieve prime divides
+        for p in range(61, 542):
+            if K % p == 0 and all(p % d for d in range(2, 24)):
+                density *= (p - 1) / (p - 24)
+        found = int(1.1 * density * starts)
+        ctx = A.Context(0, cand_ring_log2=12)
+        A.lib = Lib()
+        cand, st = ctx.sieve_range(K, 0, 0, starts)
+        assert len(cand) == found and len(rooms) == 1, (rooms, found)
+        ctx.close()
+    """)
