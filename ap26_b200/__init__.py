@@ -232,8 +232,10 @@ _AP = np.dtype([("k", np.int32), ("K", np.int32), ("first", np.int64), ("n", np.
 assert _AP.itemsize == ctypes.sizeof(AP)
 
 
-_SIEVE_PRIMES = [p for p in range(61, 542) if all(p % d for d in range(2, 24))]
-_SIEVE_PRODUCT = math.prod(_SIEVE_PRIMES)
+# What a sieve prime that divides K does to the number of candidates: it excludes
+# one residue, not 24.
+_DENSITY = {p: (p - 1) / (p - 24) for p in range(61, 542) if all(p % d for d in range(2, 24))}
+_SIEVE_PRODUCT = math.prod(_DENSITY)
 
 
 def _aps_to_list(arr, n):
@@ -366,13 +368,12 @@ class Context:
         return per, list(res), st
 
     def sieve_range(self, K, shift, q0, q1, cap=1 << 22):
-        # room for the survivors expected of this K (a prime that divides it
-        # excludes one residue, not 24), the rest of cap only if they are more
+        # room for the survivors expected of this K, the rest of cap only if they are more
         room = 0.37 * max(0, int(q1) - int(q0))
         common = math.gcd(int(K), _SIEVE_PRODUCT % max(1, int(K)))
-        for p in _SIEVE_PRIMES if common > 1 else ():
-            if common % p == 0:
-                room *= (p - 1) / (p - 24)
+        if common > 1:              # a prime, mostly
+            room *= _DENSITY.get(common) or math.prod(
+                f for p, f in _DENSITY.items() if common % p == 0)
         room = min(int(cap), int(room) + 1024)
         n = ctypes.c_int64(0)
         st = Stats()
