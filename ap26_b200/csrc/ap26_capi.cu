@@ -1472,10 +1472,11 @@ static cudaError_t capture_run(ap26_ctx *ctx, JobSet &S, const uint32_t *tables,
 // Enqueues the run of S.h_jobs[0..njobs) and returns without waiting:
 // S.done fires once the run state, counts and hash sums are in the pinned
 // mirrors.  With opts.use_graphs the run is one CUDA-graph launch, captured
-// once per run shape and replayed from the cache.
+// once per run shape and replayed from the cache.  `windows`: whole K too by
+// the window sieve.
 static int enqueue_jobs(ap26_ctx *ctx, JobSet &S, int njobs, bool count_only, bool overlap,
                         const uint32_t *tables = nullptr, int build_tables = 1,
-                        bool record_done = true, int chunk_tiles = 0) {
+                        bool record_done = true, int chunk_tiles = 0, bool windows = false) {
   if (chunk_tiles <= 0) chunk_tiles = ctx->opts.chunk_tiles;
   int rc;
   if ((rc = jobset_ensure(ctx, S, njobs)) != AP26_OK) return rc;
@@ -1498,7 +1499,7 @@ static int enqueue_jobs(ap26_ctx *ctx, JobSet &S, int njobs, bool count_only, bo
   S.h_st->total_tiles = tiles;
   S.njobs = njobs;
   S.count_only = count_only;
-  S.by_class = njobs > 0;
+  S.by_class = njobs > 0 && !windows;
   for (int j = 0; j < njobs; j++)
     if (S.h_jobs[j].q_begin != 0 || S.h_jobs[j].q_end != N53_PER_K) S.by_class = false;
   S.chunk_units = class_chunk_units(S.h_jobs, njobs, count_only, ctx->cand_cap, chunk_tiles, tile_n53);
@@ -1632,10 +1633,12 @@ static int collect_run(ap26_ctx *ctx, JobSet &S, cudaStream_t cs, ap26_stats *st
 
 // Synchronous run on the main job set.
 static int run_jobs(ap26_ctx *ctx, int njobs, bool count_only, ap26_stats *stats,
-                    long long *n_aps_out, bool overlap = false) {
+                    long long *n_aps_out, bool overlap = false, bool windows = false) {
   int rc;
   drain(ctx);
-  if ((rc = enqueue_jobs(ctx, ctx->main, njobs, count_only, overlap)) != AP26_OK) return rc;
+  if ((rc = enqueue_jobs(ctx, ctx->main, njobs, count_only, overlap, nullptr, 1, true, 0,
+                         windows)) != AP26_OK)
+    return rc;
   if ((rc = wait_event(ctx, ctx->main.done, ctx->opts.wait_timeout_s)) != AP26_OK) return rc;
   return collect_run(ctx, ctx->main, ctx->stream, stats, n_aps_out);
 }
@@ -1651,21 +1654,29 @@ static void fill_job(KJob &J, int K, int shift, int item, int64_t q0, int64_t q1
   J.word_begin = word_begin;
 }
 
-// Runs jobs, retrying with smaller chunks on a candidate-buffer overflow.
+// Runs jobs, retrying with smaller chunks on a candidate-buffer overflow.  The
+// class sieve's smallest launch is a unit, of about 2400 survivors of an ordinary
+// K and 15200 of the densest, and the largest units have a quarter more than the
+// mean; a window chunk can be one tile of 70 to 370.  So where the class sieve
+// still overflows the ring, the windows have the last try, with the chunks it had.
 static int run_jobs_retry(ap26_ctx *ctx, int njobs, bool count_only, ap26_stats *stats,
                           long long *n_aps, bool overlap = false) {
   const int saved = ctx->opts.chunk_tiles;
   std::vector<KJob> keep(ctx->main.h_jobs, ctx->main.h_jobs + njobs);
   int rc = run_jobs(ctx, njobs, count_only, stats, n_aps, overlap);
-  int tries = 0;
-  while (rc == AP26_E_OVERFLOW && (ctx->main.h_st->err_flags & ERR_CAND_OVERFLOW) &&
-         ctx->opts.chunk_tiles > 64 && tries < 6) {
-    ctx->opts.chunk_tiles /= 4;
+  const auto overflowed = [&] {
+    return rc == AP26_E_OVERFLOW && (ctx->main.h_st->err_flags & ERR_CAND_OVERFLOW);
+  };
+  const auto again = [&](bool windows) {
     memcpy(ctx->main.h_jobs, keep.data(), sizeof(KJob) * njobs);
-    rc = run_jobs(ctx, njobs, count_only, stats, n_aps, overlap);
+    rc = run_jobs(ctx, njobs, count_only, stats, n_aps, overlap, windows);
     if (stats) stats->error_flags |= 1;
-    tries++;
+  };
+  for (int tries = 0; overflowed() && ctx->opts.chunk_tiles > 64 && tries < 6; tries++) {
+    ctx->opts.chunk_tiles /= 4;
+    again(false);
   }
+  if (overflowed() && ctx->main.by_class) again(true);
   ctx->opts.chunk_tiles = saved;
   return rc;
 }
