@@ -911,6 +911,7 @@ static int staged(ap26_ctx *ctx, int64_t count, std::initializer_list<Column> in
   // how far each set has come, over all of its slices: one for each thread that
   // has copied its part of a slice in, and one for the slice's launch
   std::atomic<int64_t> filled[kSets] = {};
+  std::atomic<int64_t> back[kSets] = {};      // slices of each set whose results are back
   std::atomic<int> failed{0};
   double total = 0;
   const auto work = [&](int t) {
@@ -920,21 +921,34 @@ static int staged(ap26_ctx *ctx, int64_t count, std::initializer_list<Column> in
       return e == cudaSuccess;
     };
     const auto part = [&](int64_t n, int k) { return n * k / team; };
-    // slice i's results, this thread's part
-    const auto take = [&](int64_t i) {
-      StageSet &G = ctx->sets[i % sets];
-      // its kernel is launched by whoever fills it last, mostly at once; a thread
-      // that the system holds back gets the processors of those that wait
-      for (int spins = 0; filled[i % sets].load() < (i / sets + 1) * (team + 1); spins++) {
-        if (failed.load()) return;
-        if (spins < 200) std::this_thread::yield();
-        else std::this_thread::sleep_for(std::chrono::microseconds(20 << std::min(spins - 200, 6)));
+    // Until `there` has come to `enough`, mostly at once or within a slice's time;
+    // threads that wait longer than a millisecond sleep, and leave the processors to
+    // those they wait for.
+    const auto reached = [&](const std::atomic<int64_t> &there, int64_t enough) {
+      const auto t0 = std::chrono::steady_clock::now();
+      int sleeps = 0;
+      while (there.load() < enough) {
+        if (failed.load()) return false;
+        if (std::chrono::steady_clock::now() - t0 > std::chrono::milliseconds(1))
+          std::this_thread::sleep_for(std::chrono::microseconds(20 << std::min(sleeps++, 6)));
       }
-      if (!ok(cudaEventSynchronize(G.back))) return;
+      return true;
+    };
+    // slice i's results, this thread's part; the first thread waits for them, and
+    // the runtime's wait spins
+    const auto take = [&](int64_t i) {
+      const int64_t s = i % sets, round = i / sets + 1;
+      StageSet &G = ctx->sets[s];
       if (t == 0) {
+        // its kernel is launched by whoever fills it last
+        if (!reached(filled[s], round * (team + 1))) return;
+        if (!ok(cudaEventSynchronize(G.back))) return;
+        back[s].store(round);
         float ms1 = 0;
         cudaEventElapsedTime(&ms1, G.k0, G.k1);
         total += ms1;
+      } else if (!reached(back[s], round)) {
+        return;
       }
       const int64_t first = i * slice, n = std::min(slice, count - first);
       empty(G.h_out, first, n, part(n, t), part(n, t + 1));

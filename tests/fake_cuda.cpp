@@ -23,7 +23,7 @@ std::map<std::string, Failure> g_failures;    // call -> the calls of it that fa
 std::map<const void *, std::string> g_names;  // host stub -> kernel
 std::map<const void *, std::pair<void *, size_t>> g_vars;
 std::vector<std::string> g_launched;
-int g_slow_ms = 0;
+int g_slow_ms = 0, g_busy_ms = 0;
 struct Patch { size_t bytes, offset; unsigned long long value; } g_patch = {};
 
 // The fake's own containers always have memory.
@@ -64,6 +64,8 @@ void fake_fail(const char *call, int skip, int times, int code) {
 int fake_launches(void) { return (int)g_launched.size(); }
 // The next copy to the device takes this long.
 void fake_slow_copy(int ms) { g_slow_ms = ms; }
+// An event takes this long to come, from the wait for it on.
+void fake_busy_device(int ms) { g_busy_ms = ms; }
 // The next copy of `bytes` bytes back to the host has `value` at `offset`.
 void fake_read_back(size_t bytes, size_t offset, unsigned long long value) {
   g_patch = Patch{bytes, offset, value};
@@ -121,7 +123,13 @@ FAKE(cudaEventDestroy, (cudaEvent_t v), free(v))
 FAKE(cudaEventRecord, (cudaEvent_t, cudaStream_t), )
 FAKE(cudaEventRecordWithFlags, (cudaEvent_t, cudaStream_t, unsigned), )
 FAKE(cudaEventQuery, (cudaEvent_t), )
-FAKE(cudaEventSynchronize, (cudaEvent_t), )
+cudaError_t cudaEventSynchronize(cudaEvent_t) {
+  const cudaError_t e = result("cudaEventSynchronize");
+  // the runtime's wait spins, by default
+  const auto until = std::chrono::steady_clock::now() + std::chrono::milliseconds(g_busy_ms);
+  while (std::chrono::steady_clock::now() < until) {}
+  return e;
+}
 FAKE(cudaEventElapsedTime, (float *ms, cudaEvent_t, cudaEvent_t), *ms = 0)
 FAKE(cudaFuncSetAttribute, (const void *, cudaFuncAttribute, int), )
 FAKE(cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags,

@@ -174,6 +174,23 @@ def test_threads_of_a_long_call_do_not_spin_while_one_is_late(child):
     """)
 
 
+def test_one_thread_of_a_long_call_waits_for_the_device(child):
+    """A long call may wait for work that is queued before it, such as a serving
+    slice.  The runtime's wait spins: one thread takes it, the others sleep."""
+    child("""
+        ctx = A.Context(0, cand_ring_log2=12)
+        N = np.full(1 << 22, 9, np.uint64)
+        ctx.sprp_batch(N)                       # starts the threads
+        fake.fake_busy_device(200)
+        cpu, wall = time.process_time(), time.perf_counter()
+        ctx.sprp_batch(N)                       # four slices
+        cpu, wall = time.process_time() - cpu, time.perf_counter() - wall
+        assert wall >= 0.8, wall
+        assert cpu < 1.5 * wall, (cpu, wall)
+        ctx.close()
+    """)
+
+
 def test_long_calls_with_memory_for_one_set_of_buffers(child):
     """The context has one set of buffers from the start.  A long call uses three;
     where there is no memory for the others it goes through those there are, and
