@@ -998,7 +998,7 @@ static int staged(ap26_ctx *ctx, int64_t count, std::initializer_list<Column> in
   return AP26_OK;
 }
 
-extern "C" int ap26_version(void) { return 10100; }
+extern "C" int ap26_version(void) { return 10200; }
 
 extern "C" const char *ap26_strerror(int code) {
   switch (code) {

@@ -172,6 +172,9 @@ typedef struct {
 } ap26_sol;
 
 /* ---- library / context --------------------------------------------------- */
+/* major * 10000 + minor * 100.  10200: AP26_NOALLOC_SCRATCH_BYTES is 15,591,200
+ * (10100: 2,349,440); ap26_stats.late_items of a whole K counts candidates
+ * (10100: shift words); ap26_stats.launches counts every slice of a call. */
 int ap26_version(void);
 const char *ap26_strerror(int code);
 /* Text of the last CUDA error / timeout seen by ctx ("" if none). */

@@ -8,6 +8,7 @@ of the library is a failed test.
 import glob
 import importlib.util
 import os
+import re
 import shutil
 import subprocess
 import sys
@@ -307,3 +308,12 @@ def test_a_range_is_sieved_once_whatever_divides_k(child, K):
         assert len(cand) == found and len(rooms) == 1, (rooms, found)
         ctx.close()
     """)
+
+
+def test_the_version_tells_the_scratch_size_and_late_items(child):
+    """A program asks ap26_version() which of the header's figures hold: the size
+    of the allocation-free scratch, and what late_items counts for a whole K."""
+    with open(os.path.join(ROOT, "include", "ap26.h")) as f:
+        size = int(re.search(r"#define AP26_NOALLOC_SCRATCH_BYTES (\d+)", f.read()).group(1))
+    out = child("print(A.lib.ap26_version())")
+    assert {10100: 2349440, 10200: 15591200}[int(out)] == size
