@@ -918,6 +918,8 @@ static int staged(ap26_ctx *ctx, int64_t count, std::initializer_list<Column> in
   std::atomic<int64_t> filled[kSets] = {};
   std::atomic<int64_t> back[kSets] = {};      // slices of each set whose results are back
   std::atomic<int> failed{0};
+  std::mutex mu;
+  std::condition_variable moved;
   double total = 0;
   const auto work = [&](int t) {
     cudaError_t e = cudaSetDevice(ctx->device);
@@ -927,17 +929,25 @@ static int staged(ap26_ctx *ctx, int64_t count, std::initializer_list<Column> in
     };
     const auto part = [&](int64_t n, int k) { return n * k / team; };
     // Until `there` has come to `enough`, mostly at once or within a slice's time;
-    // threads that wait longer than a millisecond sleep, and leave the processors to
-    // those they wait for.
+    // threads that wait for longer sleep, and leave the processors to those they
+    // wait for.
     const auto reached = [&](const std::atomic<int64_t> &there, int64_t enough) {
       const auto t0 = std::chrono::steady_clock::now();
-      int sleeps = 0;
       while (there.load() < enough) {
         if (failed.load()) return false;
-        if (std::chrono::steady_clock::now() - t0 > std::chrono::milliseconds(1))
-          std::this_thread::sleep_for(std::chrono::microseconds(20 << std::min(sleeps++, 6)));
+        if (std::chrono::steady_clock::now() - t0 < std::chrono::milliseconds(10)) continue;
+        std::unique_lock<std::mutex> lock(mu);
+        moved.wait(lock, [&] { return there.load() >= enough || failed.load(); });
       }
       return true;
+    };
+    // ... and those that a step there may wake
+    const auto step = [&](const auto &f) {
+      {
+        std::lock_guard<std::mutex> lock(mu);
+        f();
+      }
+      moved.notify_all();
     };
     // slice i's results, this thread's part; the first thread waits for them, and
     // the runtime's wait spins
@@ -948,7 +958,7 @@ static int staged(ap26_ctx *ctx, int64_t count, std::initializer_list<Column> in
         // its kernel is launched by whoever fills it last
         if (!reached(filled[s], round * (team + 1))) return;
         if (!ok(cudaEventSynchronize(G.back))) return;
-        back[s].store(round);
+        step([&] { back[s].store(round); });
         float ms1 = 0;
         cudaEventElapsedTime(&ms1, G.k0, G.k1);
         total += ms1;
@@ -983,12 +993,12 @@ static int staged(ap26_ctx *ctx, int64_t count, std::initializer_list<Column> in
       ok(cudaMemcpyAsync(G.h_out, G.d_out, (size_t)(n * out_per), cudaMemcpyDeviceToHost,
                          ctx->back_stream));
       ok(cudaEventRecord(G.back, ctx->back_stream));
-      if (e == cudaSuccess) filled[i % sets].fetch_add(1);
+      if (e == cudaSuccess) step([&] { filled[i % sets].fetch_add(1); });
     }
     for (int64_t i = std::max<int64_t>(0, slices - sets);
          i < slices && e == cudaSuccess && !failed.load(); i++)
       take(i);
-    if (e != cudaSuccess) failed.store((int)e);
+    if (e != cudaSuccess) step([&] { failed.store((int)e); });
   };
   ctx->team->run(team, std::ref(work));       // by reference: no copy on the heap
   *ms = total;

@@ -192,6 +192,26 @@ def test_one_thread_of_a_long_call_waits_for_the_device(child):
     """)
 
 
+def test_threads_of_a_long_call_wake_in_time(child):
+    """A slice's results are copied out as soon as they are there, also where its
+    kernel takes some milliseconds, as that of 140000 reports does."""
+    child("""
+        ctx = A.Context(0, cand_ring_log2=12)
+        N = np.full(1 << 20, 9, np.uint64)      # one slice
+        fake.fake_busy_device(6)
+        def call():
+            t = time.perf_counter()
+            ctx.sprp_batch(N)
+            return 1e3 * (time.perf_counter() - t)
+        call()
+        least = min(call() for _ in range(20))
+        fake.fake_busy_device(0)
+        without = min(call() for _ in range(20))
+        assert least < 6.25 + without, (least, without)
+        ctx.close()
+    """)
+
+
 def test_long_calls_with_memory_for_one_set_of_buffers(child):
     """The context has one set of buffers from the start.  A long call uses three;
     where there is no memory for the others it goes through those there are, and
