@@ -864,6 +864,22 @@ constexpr int REPORT_THREADS = 96;
 constexpr int REPORT_BASES = 9;      // 2 and validate_ap26's 3..23 (AP26.cpp:519)
 enum : uint32_t { TERM_P2 = 1, TERM_P9 = (1 << REPORT_BASES) - 1, TERM_DOM = 1 << REPORT_BASES };
 
+// The terms of a report of more than REPORT_LONG to base 2, all threads of the
+// block.  No progression of that many primes is known (27), so the report has
+// composites, and the other bases of those tell nothing: a report of 128 of them
+// took 93 us with the nine bases at once and takes 23, 9600 such reports 1.81 and
+// 0.67 ms.  Up to there a step less is what counts: the nine bases of 32 terms are
+// three.  Not inlined: the other reports' code stays as short as it was.
+constexpr int REPORT_LONG = 32;
+__device__ __noinline__ void long_report(uint32_t *fl, int k, int64_t first, uint64_t D) {
+  for (int j = threadIdx.x; j < k; j += REPORT_THREADS) {
+    const uint64_t jd = (uint64_t)j * D, N = (uint64_t)first + jd;
+    if (jd < (1ull << 62) && N < (1ull << 62))
+      fl[j] = TERM_DOM | ((N & 1) && sprp_base(2, N) ? TERM_P2 : 0u);
+  }
+  __syncthreads();
+}
+
 // One block per report: a thread tests one term to one base (terms in the
 // domain 0 <= N < 2^62 of the reference's mulmod, AP26.cpp:494/529), then
 // thread 0 replays the recursion of ReportSolution over the per-term
@@ -899,8 +915,10 @@ __global__ void __launch_bounds__(REPORT_THREADS) report_kernel(ReportArgs A) {
       __syncthreads();
       const uint64_t D = (uint64_t)K * (uint64_t)PRIM23;     // < 2^57
       const uint32_t bases[REPORT_BASES] = {2, 3, 5, 7, 11, 13, 17, 19, 23};
+      if (k > REPORT_LONG) long_report(fl, k, first, D);
       for (int t = threadIdx.x; t < k * REPORT_BASES; t += REPORT_THREADS) {
         const int j = t / REPORT_BASES, b = t - j * REPORT_BASES;
+        if (k > REPORT_LONG && !(fl[j] & TERM_P2)) continue;
         const uint64_t jd = (uint64_t)j * D;                   // < 2^64
         const uint64_t N = (uint64_t)first + jd;
         if (jd < (1ull << 62) && N < (1ull << 62))
