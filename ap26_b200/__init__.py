@@ -331,12 +331,14 @@ class Context:
         """Device-side ReportSolution of raw reports [(k, K, first[, n])]:
         returns (rc, [Final], new result_hash or None).  rc is the first
         non-OK status (the per-report statuses are in the Finals)."""
-        rows = [(int(a[0]), int(a[1]), int(a[2]), int(a[3]) if len(a) > 3 else 0) for a in aps]
         try:
-            arr = np.zeros(max(1, len(rows)), _AP)
-            arr[:len(rows)] = rows
+            arr = np.zeros(max(1, len(aps)), _AP)
+            arr[:len(aps)] = [(int(a[0]), int(a[1]), int(a[2]), int(a[3]) if len(a) > 3 else 0)
+                              for a in aps]
         except OverflowError:       # numpy refuses what a C integer takes modulo its range
-            arr = np.frombuffer((AP * len(rows))(*[AP(*r) for r in rows]), _AP)
+            arr = np.frombuffer((AP * len(aps))(*[AP(int(a[0]), int(a[1]), int(a[2]),
+                                                     int(a[3]) if len(a) > 3 else 0)
+                                                  for a in aps]), _AP)
         fin = (Final * max(1, len(aps)))()
         h = ctypes.c_int32(result_hash or 0)
         rc = lib.ap26_report_batch(self.h, _ptr(arr), len(aps), fin,
