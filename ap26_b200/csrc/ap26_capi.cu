@@ -61,12 +61,7 @@ __device__ void build_table(int K, int shift, uint32_t *tab, int first, int stri
   }
 }
 
-// Blocks (j, y): job j.  Thread 0 of y = 0 sets the reference's per-K
-// constants; the blocks share the first `words` words of the job's bitstrings
-// at KJob::table: all of them for the window sieve, the 61 * 67 pair's for
-// the class sieve, none where a serving unit built them at admission.  A word
-// is a chain of some 600 instructions, so one word a thread: a block of 256
-// that built eleven each (and sorted a lattice order) took 0.3 ms.
+// The reference's per-K constants.
 __device__ void set_constants(KJob &J) {
   const int K = J.K;
   J.STEP = (int64_t)K * PRIM23;
@@ -80,6 +75,12 @@ __device__ void set_constants(KJob &J) {
   kmul_mod(PRES8, K, &J.S59);
 }
 
+// Blocks (j, y): job j.  Thread 0 of y = 0 sets the reference's per-K
+// constants; the blocks share the first `words` words of the job's bitstrings
+// at KJob::table: all of them for the window sieve, the 61 * 67 pair's for
+// the class sieve, none where a serving unit built them at admission.  A word
+// is a chain of some 600 instructions, so one word a thread: a block of 256
+// that built eleven each (and sorted a lattice order) took 0.3 ms.
 __global__ void setup_jobs_kernel(KJob *jobs, uint32_t *tables, int words) {
   KJob &J = jobs[blockIdx.x];
   const int K = J.K;
@@ -592,7 +593,7 @@ struct JobSet {
   int njobs = 0;
   int chunk_tiles = 0;
   bool count_only = false;
-  bool by_class = false;              // whole K-jobs: the class sieve, else the window sieve
+  bool by_class = false;              // the class sieve (whole K-jobs), else the window sieve
   int chunk_units = 0;                // class sieve: units per launch
   unsigned long long nchunks = 0, nprof = 0;
   int launches = 0;
@@ -635,11 +636,25 @@ struct Slice {
 // their device counterparts, used in turn by a call's slices, and a copy
 // stream for each of a call's host threads.  Allocated with the context (the
 // first set) or with the first call that needs them, freed with the context.
+//
+// The figures are calls of sprp_batch (9 bytes a value) on a 16-core host, one
+// constant changed at a time.
+// Sets: 2^24 values 4.84 ms with two, 3.98 with three, 3.78 with four.
 constexpr int kSets = 3;
-constexpr int kTeam = 8;                        // host threads of a call, at most
-constexpr int64_t kSetBytes = 8 << 20;          // in, and out, per set
-constexpr int64_t kZeroCopyBytes = 1 << 20;     // up to here kernels use the pinned buffers
-constexpr int64_t kThreadBytes = 512 << 10;     // a thread copies at least this much
+// Host threads of a call, at most: 2^24 values 13.4, 6.7, 3.85, 3.98 and 4.9 ms with
+// 1, 2, 4, 8 and 16; 2^22 2.64, 1.54, 1.09, 1.18 and 1.37; 2^20 0.90, 0.63, 0.52,
+// 0.50 and 0.55.
+constexpr int kTeam = 8;
+// In, and out, per set: 2^24 values 7.2, 5.2, 3.98 and 3.5 ms with 2, 4, 8 and 16 MB,
+// 2^22 1.84, 1.38, 1.18 and 1.25.
+constexpr int64_t kSetBytes = 8 << 20;
+// Up to here kernels use the pinned buffers, further on copies are cheaper: 2^15,
+// 2^16 and 2^17 values (256 KB to 1 MB) 57, 77 and 124 us so and 82, 105 and 138
+// through copies, 2^18 and 2^19 242 and 413, and 197 and 317.
+constexpr int64_t kZeroCopyBytes = 1 << 20;
+// A thread copies at least this much: 2^18 values 212, 198 and 278 us with 128 KB,
+// 512 KB and 2 MB, 2^19 319, 318 and 358.
+constexpr int64_t kThreadBytes = 512 << 10;
 struct StageSet {
   char *h_in = nullptr, *h_out = nullptr, *d_in = nullptr, *d_out = nullptr;
   cudaEvent_t k0 = nullptr, k1 = nullptr, back = nullptr;   // kernel, results copied back
@@ -1372,9 +1387,12 @@ static double expected_survivors(int K) {
 // of chunk_tiles tiles of tile_n53 starts, at least one unit, equal over a K.
 // At the default a launch takes a whole K when nothing is kept of it but counts,
 // or when the survivors of the densest K of the run fit a ring with a quarter to
-// spare, and as large a part as fits when they do not.  Each launch ends with
-// CTAs that wait for the last one and with the last walks of its chains: a K
-// took 137.3 to 137.8 ms in five launches and takes 135.5 to 136.2 in one.
+// spare, and else as large a part as fits, but no less than its chunk of tiles:
+// with a ring too small for that (up to 2^22 for an ordinary K, 2^25 for the
+// densest) the first run overflows and is redone, as with a chunk that is set.  Each
+// launch ends with CTAs that wait for the last one and with the last walks of its
+// chains: a K took 137.3 to 137.8 ms in five launches and takes 135.5 to 136.2 in
+// one.
 static int class_chunk_units(const KJob *jobs, int njobs, bool count_only, long long cand_cap,
                              int chunk_tiles, int64_t tile_n53) {
   const int64_t most = std::max<int64_t>(
@@ -2537,13 +2555,12 @@ extern "C" int ap26_probe_peaks(ap26_ctx *ctx, double *smem_gbs, double *int_top
 }
 
 // ---- autotuner -------------------------------------------------------------------------------
-// Two stages.  (1) Every compiled sieve variant (dense primes, tail group,
-// late stage, queue depth, CTA size) on the same slice of K's lattice, the
-// first 1/64 of its starts, count-only in one launch, so only the sieve is
-// timed.  (2) For the fastest variant, the whole pipeline (sieve, chain walk
-// on the second stream, ReportSolution) over one whole K at each chunk size
-// the candidate rings can hold: a chunk is the unit the chain walk overlaps
-// and each chunk boundary drains the persistent sieve once.
+// Two stages.  (1) Every compiled variant of the window sieve (dense primes, tail
+// group, late stage, queue depth, CTA size) on the same slice of K's lattice, the
+// first 1/64 of its starts, count-only in one launch, a start's 35 n59 in one
+// tile as in ap26_sieve_range's long ranges.  (2) The whole pipeline (class sieve,
+// chain walk, ReportSolution) over one whole K at each chunk size whose survivors
+// the candidate rings can hold; the default, one launch a K, is among them.
 extern "C" int ap26_autotune(ap26_ctx *ctx, int K, int shift, ap26_opts *chosen) {
   if (!ctx) return AP26_E_ARG;
   if (!k_in_domain(K, shift) || !ap26_will_search(K)) return AP26_E_DOMAIN;
@@ -2570,7 +2587,7 @@ extern "C" int ap26_autotune(ap26_ctx *ctx, int K, int shift, ap26_opts *chosen)
     if (t < best_ms) { best_ms = t; best_v = vi; }
   }
   if ((rc = set_variant(ctx, best_v)) != AP26_OK) return rc;
-  // chunk sizes whose worst-case survivors (about 115 per tile) fit a ring
+  // chunk sizes that fit a ring at 115 survivors per 256 starts (an ordinary K has 69)
   const int tile_n53 = kVariants[best_v].WARPS * 32;
   int best_chunk = saved_chunk;
   best_ms = 1e30;

@@ -4,11 +4,12 @@
 //   x  one of the 1355 admissible (i31, i37, i41) triples' values,
 //   v  one of the 443555 (j43, j47, j53, j59) values,
 //   b  one of the 8 (i3, i5) values,
-// each reduced mod MOD, so x + v + b = n59 + wraps * MOD with wraps 0..2.  In
-// the window coordinate of ap26_kernels.cuh, bit i of n59's 640-bit mask is
-//   B_m[(s(x) + s(v) + s(b) + i + wraps) mod m],  s(y) = y * MOD^-1 mod m,
+// each reduced mod MOD, so x + v + b = n59 + wraps * MOD with wraps 0..2, and
+// s(x) + s(v) + s(b) = s(n59) + wraps for s(y) = y * MOD^-1 mod m.  In the window
+// coordinate of ap26_kernels.cuh, bit i of n59's 640-bit mask is
+//   B_m[s(n59) + i] = B_m[(s(x) + s(v) + s(b) + j - 2) mod m],  j = i - wraps + 2,
 // for every modulus m, so each modulus sees one sum of three residues and an
-// index j = i + wraps.  All points (x, v) with the same s(x) + s(v) mod 4087
+// index j = 0..641.  All points (x, v) with the same s(x) + s(v) mod 4087
 // form a class; for a class, the (b, j) that pass 61 and 67 are the same for
 // every point: about 2000 of 8 * 642.  Only those are sieved, in rows of 512
 // bits (one bit per surviving (b, j)), four rows a class.
@@ -53,11 +54,11 @@
 // bits instead of masks in the first queue 32.
 //
 // The class sieve takes every whole K.  A K that 61 or 67 divides has more
-// (b, j) per class (up to thirteen rows) and is still faster than by windows:
-// 230 against 389 ms for 61 | K, 326 against 463 for 61 * 67 | K, 550 against
-// 695 for 61 * 67 * 71 * 73 | K, the densest.  Parts of a
-// K (sieve_range) stay with the window sieve: a class's points are spread over
-// the whole lattice.
+// (b, j) per class (six or seven rows, ten for both) and is still faster than by
+// windows: counts of 42700061 (61) 209 against 388 ms, 28686653 (61 * 67) 292
+// against 464, 21182921 (61 * 67 * 71 * 73, the densest) 491 against 695.  Parts
+// of a K (sieve_range) stay with the window sieve, a class's points being spread
+// over the whole lattice, and so does a K whose units overflow a small ring.
 //
 // Bits that survive the dense rows become single candidates, tested against
 // the other moduli (primes 7..23 included) in full batches of 32 lanes that

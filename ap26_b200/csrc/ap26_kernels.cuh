@@ -10,7 +10,8 @@
 //   chunk_begin_kernel  resets per-chunk counters
 //   class_plan_*, class_sieve_kernel (ap26_class.cuh)
 //                       the sieve of a whole K, by residue classes
-//   sieve_kernel        the sieve of a part of a K's lattice: persistent,
+//   sieve_kernel        the sieve of a part of a K's lattice, and of a whole K
+//                       whose class sieve overflows a small ring: persistent,
 //                       work-stealing over tiles of n53 starts;
 //                       replaces setupn.cl + sieve.cl (the 1.1 GB n59 array
 //                       of the reference is never materialised: starts are

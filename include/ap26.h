@@ -51,7 +51,8 @@ typedef struct ap26_ctx ap26_ctx;
 /* Tuning knobs; zero fields take the context's defaults (or autotuned values,
  * see ap26_autotune).  dense_primes, warp_queue, block_threads, late_stage and
  * tail_group choose a variant of the window sieve, which serves parts of a K
- * (ap26_sieve_range); the class sieve of whole K has one form. */
+ * (ap26_sieve_range) and whole K that a small ring cannot hold otherwise; the
+ * class sieve of whole K has one form. */
 typedef struct {
   int32_t dense_primes;   /* primes sieved for all 10 words before compaction */
   int32_t warp_queue;     /* per-warp shared-memory queue depth (items)       */
@@ -73,7 +74,9 @@ typedef struct {
   int32_t cand_ring_log2; /* each of the two candidate rings holds 2^n
                              entries of 16 bytes (default 26; 12..27).  A
                              chunk whose survivors overflow it is redone with
-                             4x fewer tiles per launch (at most six times);
+                             4x fewer tiles per launch (at most six times,
+                             then by the window sieve, whose chunks can be
+                             smaller);
                              serving slices use chunks small enough for the
                              densest K                                        */
   int64_t mem_budget;     /* serving: device bytes for admitted units' tables
@@ -342,7 +345,7 @@ int ap26_chain_batch(ap26_ctx *ctx, int K, const int64_t *n, int64_t count,
  *   file-scope device array of AP26_NOALLOC_SCRATCH_BYTES (15,591,200 bytes)
  *   that every GPU loading the library keeps until process exit.  At most
  *   AP26_NOALLOC_MAX_K values of K per call; more returns AP26_E_CAPACITY.
- *   An invalid K costs no sieve time.
+ *   An invalid K costs no sieve time (its launches take about 30 us).
  * - A CUDA error already pending in the calling thread when the call starts
  *   is neither returned as this call's own nor cleared: the call launches
  *   nothing and returns AP26_E_CUDA.
