@@ -794,7 +794,10 @@ static void drain(ap26_ctx *ctx) {
   ctx->pending = false;
 }
 
+// The call ends with the error; none is left pending in the thread, where the next
+// call would find it behind its launches.
 static int cuda_fail(ap26_ctx *ctx, cudaError_t e, const char *what) {
+  cudaGetLastError();
   if (ctx) ctx->last_error = std::string(what) + ": " + cudaGetErrorString(e);
   return AP26_E_CUDA;
 }
@@ -1013,7 +1016,9 @@ static int staged(ap26_ctx *ctx, int64_t count, std::initializer_list<Column> in
     for (int64_t i = std::max<int64_t>(0, slices - sets);
          i < slices && e == cudaSuccess && !failed.load(); i++)
       take(i);
-    if (e != cudaSuccess) step([&] { failed.store((int)e); });
+    if (e == cudaSuccess) return;
+    cudaGetLastError();                       // this thread's: see cuda_fail
+    step([&] { failed.store((int)e); });
   };
   ctx->team->run(team, std::ref(work));       // by reference: no copy on the heap
   *ms = total;

@@ -337,3 +337,27 @@ def test_the_version_tells_the_scratch_size_and_late_items(child):
         size = int(re.search(r"#define AP26_NOALLOC_SCRATCH_BYTES (\d+)", f.read()).group(1))
     out = child("print(A.lib.ap26_version())")
     assert {10100: 2349440, 10200: 15591200}[int(out)] == size
+
+
+def test_a_long_call_that_fails_leaves_the_next_one_alone(child):
+    """Whichever step of whichever thread fails: the call ends with AP26_E_CUDA, no
+    thread hangs, and none keeps the error for a later call to find."""
+    child("""
+        ctx = A.Context(0, cand_ring_log2=12)
+        N = np.full(5 << 20, 9, np.uint64)      # five slices, eight threads
+        calls = 0
+        for call in ("cudaMemcpyAsync", "cudaEventRecord", "cudaStreamWaitEvent",
+                     "cudaEventSynchronize", "cudaLaunchKernel", "cudaSetDevice"):
+            for skip in (0, 1, 3, 4, 7, 12, 20, 33):
+                fail(call, skip=skip, times=1)
+                try:
+                    ctx.sprp_batch(N)
+                except A.AP26Error as e:
+                    assert e.code == A.E_CUDA, (call, skip)
+                    calls += 1
+                fail(call, times=0)
+                for _ in range(4):
+                    assert ctx.sprp_batch(N)[1].launches == 5
+        assert calls > 24, calls
+        ctx.close()
+    """, timeout=120)
