@@ -1388,8 +1388,9 @@ static double expected_survivors(int K) {
   return n;
 }
 
-// Class-sieve units per launch of a run.  A set chunk_tiles bounds it: chunks
-// of chunk_tiles tiles of tile_n53 starts, at least one unit, equal over a K.
+// Class-sieve units per launch of a run.  A chunk_tiles other than the default's
+// bounds it: chunks of as many tiles of tile_n53 starts, at least one unit, equal
+// over a K.
 // At the default a launch takes a whole K when nothing is kept of it but counts,
 // or when the survivors of the densest K of the run fit a ring with a quarter to
 // spare, and else as large a part as fits, but no less than its chunk of tiles:
