@@ -4,7 +4,11 @@
 // calls that a test names fail, and leave the pending error that a failing call
 // of the runtime leaves.
 #include <cuda_runtime_api.h>
+#include <sys/syscall.h>
+#include <time.h>
+#include <unistd.h>
 
+#include <atomic>
 #include <chrono>
 #include <cstdlib>
 #include <cstring>
@@ -66,6 +70,13 @@ int fake_launches(void) { return (int)g_launched.size(); }
 void fake_slow_copy(int ms) { g_slow_ms = ms; }
 // An event takes this long to come, from the wait for it on.
 void fake_busy_device(int ms) { g_busy_ms = ms; }
+// How often a thread has slept for a time (not until it is woken).
+std::atomic<int> g_sleeps{0};
+int fake_sleeps(void) { return g_sleeps; }
+int nanosleep(const timespec *t, timespec *left) {
+  g_sleeps++;
+  return (int)syscall(SYS_nanosleep, t, left);
+}
 // The next copy of `bytes` bytes back to the host has `value` at `offset`.
 void fake_read_back(size_t bytes, size_t offset, unsigned long long value) {
   g_patch = Patch{bytes, offset, value};

@@ -194,20 +194,17 @@ def test_one_thread_of_a_long_call_waits_for_the_device(child):
 
 def test_threads_of_a_long_call_wake_in_time(child):
     """A slice's results are copied out as soon as they are there, also where its
-    kernel takes some milliseconds, as that of 140000 reports does."""
+    kernel takes some milliseconds, as that of 140000 reports does: no thread
+    sleeps for a time, each waits until it is woken."""
     child("""
         ctx = A.Context(0, cand_ring_log2=12)
         N = np.full(1 << 20, 9, np.uint64)      # one slice
-        fake.fake_busy_device(6)
-        def call():
-            t = time.perf_counter()
+        ctx.sprp_batch(N)
+        for ms in (2, 6, 20):
+            fake.fake_busy_device(ms)
+            before = fake.fake_sleeps()
             ctx.sprp_batch(N)
-            return 1e3 * (time.perf_counter() - t)
-        call()
-        least = min(call() for _ in range(20))
-        fake.fake_busy_device(0)
-        without = min(call() for _ in range(20))
-        assert least < 6.25 + without, (least, without)
+            assert fake.fake_sleeps() == before, ms
         ctx.close()
     """)
 
