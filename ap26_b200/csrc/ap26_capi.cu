@@ -1161,11 +1161,31 @@ static unsigned long long job_hash_total(const JobSet &S, int j) {
   return h;
 }
 
+static void free_rings(ap26_ctx *ctx) {
+  for (Cand *&d : ctx->d_cand) {
+    cudaFree(d);
+    d = nullptr;
+  }
+  ctx->cand_cap = 0;
+}
+
+// Both rings or, after an error, none, with no room in them.
 static int alloc_rings(ap26_ctx *ctx, int log2) {
+  const size_t bytes = sizeof(Cand) << log2;
+  cudaError_t e = cudaMalloc(&ctx->d_cand[0], bytes);
+  if (e == cudaSuccess) e = cudaMalloc(&ctx->d_cand[1], bytes);
+  if (e != cudaSuccess) {
+    free_rings(ctx);
+    return cuda_fail(ctx, e, "candidate rings");
+  }
   ctx->cand_cap = 1ll << log2;
-  CK(cudaMalloc(&ctx->d_cand[0], sizeof(Cand) * ctx->cand_cap));
-  CK(cudaMalloc(&ctx->d_cand[1], sizeof(Cand) * ctx->cand_cap));
   return AP26_OK;
+}
+
+// Before every use of the rings: ap26_set_opts may have freed them and found no
+// memory for others.
+static int rings_ensure(ap26_ctx *ctx) {
+  return ctx->cand_cap ? AP26_OK : alloc_rings(ctx, ctx->opts.cand_ring_log2);
 }
 
 extern "C" int ap26_create(int device, const ap26_opts *opts, ap26_ctx **out) {
@@ -1255,7 +1275,7 @@ extern "C" void ap26_destroy(ap26_ctx *ctx) {
   cudaFree(ctx->d_plan);
   cudaFree(ctx->d_tally);
   stage_free(ctx);
-  cudaFree(ctx->d_cand[0]); cudaFree(ctx->d_cand[1]);
+  free_rings(ctx);
   for (int r = 0; r < 2; r++) {
     if (ctx->sieve_done[r]) cudaEventDestroy(ctx->sieve_done[r]);
     if (ctx->chain_done[r]) cudaEventDestroy(ctx->chain_done[r]);
@@ -1309,9 +1329,7 @@ extern "C" int ap26_set_opts(ap26_ctx *ctx, const ap26_opts *opts) {
   if (o.cand_ring_log2 != ctx->opts.cand_ring_log2) {
     CK(cudaStreamSynchronize(ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream2));
-    cudaFree(ctx->d_cand[0]);
-    cudaFree(ctx->d_cand[1]);
-    ctx->d_cand[0] = ctx->d_cand[1] = nullptr;
+    free_rings(ctx);
     drop_graphs(ctx);
     int rc = alloc_rings(ctx, o.cand_ring_log2);
     if (rc != AP26_OK) return rc;
@@ -1532,6 +1550,7 @@ static int enqueue_jobs(ap26_ctx *ctx, JobSet &S, int njobs, bool count_only, bo
                         bool record_done = true, int chunk_tiles = 0, bool windows = false) {
   if (chunk_tiles <= 0) chunk_tiles = ctx->opts.chunk_tiles;
   int rc;
+  if ((rc = rings_ensure(ctx)) != AP26_OK) return rc;
   if ((rc = jobset_ensure(ctx, S, njobs)) != AP26_OK) return rc;
   if (!tables) tables = S.d_tables;
   // tile prefix; a tile is one start per thread of the variant's CTA
@@ -2132,6 +2151,7 @@ static int launch_slice(ap26_ctx *ctx, Slice &sl) {
   if (picked.empty()) return AP26_OK;
   JobSet &S = sl.set;
   int rc;
+  if ((rc = rings_ensure(ctx)) != AP26_OK) return rc;
   if ((rc = jobset_ensure(ctx, S, (int)picked.size())) != AP26_OK) return rc;
   sl.unit_ids.clear();
   for (size_t j = 0; j < picked.size(); j++) {
@@ -2294,6 +2314,7 @@ extern "C" int ap26_sieve_range(ap26_ctx *ctx, int K, int shift, int64_t q_begin
   drain(ctx);
   JobSet &S = ctx->main;
   int rc;
+  if ((rc = rings_ensure(ctx)) != AP26_OK) return rc;
   if ((rc = jobset_ensure(ctx, S, 1)) != AP26_OK) return rc;
   // set-up and sieve only, in one launch over the whole range, candidates kept
   fill_job(S.h_jobs[0], K, shift, 0, q_begin, q_end);

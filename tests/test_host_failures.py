@@ -358,3 +358,35 @@ def test_a_long_call_that_fails_leaves_the_next_one_alone(child):
         assert calls > 24, calls
         ctx.close()
     """, timeout=120)
+
+
+def test_rings_that_could_not_be_resized_are_made_again_before_use(child):
+    """set_opts frees the candidate rings to make others.  Where that fails, no
+    kernel gets the pointers that are left: the next call makes the rings again,
+    of the size the options still have, or fails."""
+    child("""
+        ctx = A.Context(0, cand_ring_log2=13)
+        uses = [lambda: ctx.sieve_range(1, 0, 0, 1000), lambda: ctx.search_k(43241061),
+                lambda: ctx.search_batch([(1, 43241061, 43241062, 0)])]
+        for use in uses:
+            for skip in (0, 1):                  # the first or the second ring
+                fail("cudaMalloc", skip=skip, code=OOM)
+                try:
+                    ctx.set_opts(cand_ring_log2=14)
+                    raise SystemExit("no memory, and rings all the same")
+                except A.AP26Error as e:
+                    assert e.code == A.E_CUDA
+                assert ctx.opts["cand_ring_log2"] == 13
+                before = fake.fake_launches()
+                try:
+                    use()
+                    raise SystemExit("no rings, and a run all the same")
+                except A.AP26Error as e:
+                    assert e.code == A.E_CUDA
+                assert fake.fake_launches() == before
+                fail("cudaMalloc", times=0)
+                use()
+                assert fake.fake_launches() > before
+        assert ctx.set_opts(cand_ring_log2=14)["cand_ring_log2"] == 14
+        ctx.close()
+    """)
