@@ -1529,7 +1529,10 @@ static cudaError_t emit_run(ap26_ctx *ctx, JobSet &S, const uint32_t *tables, in
 static cudaError_t capture_run(ap26_ctx *ctx, JobSet &S, const uint32_t *tables,
                                int build_tables, bool two_streams, cudaGraphExec_t *exec) {
   cudaError_t e = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal);
-  if (e != cudaSuccess) return e;
+  if (e != cudaSuccess) {
+    cudaGetLastError();   // taken: the caller's launches look for errors of their own
+    return e;
+  }
   cudaError_t em = emit_run(ctx, S, tables, build_tables, two_streams, true);
   cudaGraph_t g = nullptr;
   e = cudaStreamEndCapture(ctx->stream, &g);
