@@ -2011,18 +2011,19 @@ static int serve_pool_init(ap26_ctx *ctx) {
     ctx->last_error = "serving memory budget below its fixed buffers";
     return AP26_E_NOMEM;
   }
+  // the pool last: it stands for all of them
+  for (Slice &sl : ctx->slices) {
+    int rc = jobset_ensure(ctx, sl.set, kSliceJobs);
+    if (rc != AP26_OK) return rc;
+    if (!sl.d_snap) CK(cudaMalloc(&sl.d_snap, sizeof(UnitState) * kSliceJobs));
+    if (!sl.h_snap) CK(cudaMallocHost(&sl.h_snap, sizeof(UnitState) * kSliceJobs));
+  }
   CK(cudaMalloc(&ctx->d_pool, (size_t)n * kTableBytes));
   ctx->pool_tables = (int)std::min<int64_t>(n, INT32_MAX);
   ctx->serve_budget = fixed + n * kTableBytes;
   ctx->bytes_in_use = fixed;
   ctx->free_tables.clear();
   for (int i = ctx->pool_tables - 1; i >= 0; i--) ctx->free_tables.push_back(i);
-  for (int i = 0; i < 2; i++) {
-    int rc = jobset_ensure(ctx, ctx->slices[i].set, kSliceJobs);
-    if (rc != AP26_OK) return rc;
-    CK(cudaMalloc(&ctx->slices[i].d_snap, sizeof(UnitState) * kSliceJobs));
-    CK(cudaMallocHost(&ctx->slices[i].h_snap, sizeof(UnitState) * kSliceJobs));
-  }
   return AP26_OK;
 }
 

@@ -390,3 +390,25 @@ def test_rings_that_could_not_be_resized_are_made_again_before_use(child):
         assert ctx.set_opts(cand_ring_log2=14)["cand_ring_log2"] == 14
         ctx.close()
     """)
+
+
+def test_serving_buffers_that_could_not_be_made_are_made_later(child):
+    """The first admission makes serving's buffers.  Where one of them fails the
+    admission fails, and a later one makes what is missing: no slice runs without."""
+    child("""
+        for call in ("cudaMalloc", "cudaHostAlloc"):
+            for skip in range(24):
+                ctx = A.Context(0, cand_ring_log2=12)
+                fail(call, skip=skip, code=OOM)
+                made = ctx.serve_submit(1, 43241061, 43241063, 0)
+                assert made in (A.OK, A.E_CUDA), (call, skip)
+                fail(call, times=0)
+                if made != A.OK:
+                    assert ctx.serve_submit(1, 43241061, 43241063, 0) == A.OK
+                for _ in range(4):
+                    ctx.serve_step()
+                ctx.close()
+                if made == A.OK:
+                    break
+            assert made == A.OK and skip > 3, (call, skip)
+    """)
