@@ -2140,6 +2140,11 @@ static int harvest_slice(ap26_ctx *ctx, Slice &sl) {
 // Builds and enqueues one slice: up to kSliceJobs K-jobs, one per admitted
 // unit per round (round-robin), each unit's K in ascending order.
 static int launch_slice(ap26_ctx *ctx, Slice &sl) {
+  // first what can fail: a K that is picked counts as searched
+  JobSet &S = sl.set;
+  int rc;
+  if ((rc = rings_ensure(ctx)) != AP26_OK) return rc;
+  if ((rc = jobset_ensure(ctx, S, kSliceJobs)) != AP26_OK) return rc;
   std::vector<std::pair<ServeUnit *, size_t>> picked;
   bool progress = true;
   while ((int)picked.size() < kSliceJobs && progress) {
@@ -2153,10 +2158,6 @@ static int launch_slice(ap26_ctx *ctx, Slice &sl) {
     }
   }
   if (picked.empty()) return AP26_OK;
-  JobSet &S = sl.set;
-  int rc;
-  if ((rc = rings_ensure(ctx)) != AP26_OK) return rc;
-  if ((rc = jobset_ensure(ctx, S, (int)picked.size())) != AP26_OK) return rc;
   sl.unit_ids.clear();
   for (size_t j = 0; j < picked.size(); j++) {
     ServeUnit *u = picked[j].first;
@@ -2225,9 +2226,9 @@ extern "C" int ap26_serve_step(ap26_ctx *ctx, int *active_units) {
     int idx = ctx->slices[0].busy ? 1 : 0;
     if (ctx->slices[idx].busy) break;
     int r = launch_slice(ctx, ctx->slices[idx]);
-    if (!ctx->slices[idx].busy) break;   // nothing left to schedule
-    ctx->inflight.push_back(idx);
     if (r != AP26_OK && rc == AP26_OK) rc = r;
+    if (!ctx->slices[idx].busy) break;   // nothing left to schedule, or no memory for it
+    ctx->inflight.push_back(idx);
   }
   retire_units(ctx);
   if (active_units) *active_units = (int)ctx->units.size();

@@ -412,3 +412,28 @@ def test_serving_buffers_that_could_not_be_made_are_made_later(child):
                     break
             assert made == A.OK and skip > 3, (call, skip)
     """)
+
+
+def test_serving_goes_on_once_there_is_memory_for_its_rings(child):
+    """A step that finds no memory for the candidate rings fails and takes no K: the
+    unit's K are all searched once there is some."""
+    child("""
+        ctx = A.Context(0, cand_ring_log2=12)
+        assert ctx.serve_submit(1, 43241061, 43241063, 0) == A.OK
+        fail("cudaMalloc", code=OOM)
+        try:
+            ctx.set_opts(cand_ring_log2=13)
+            raise SystemExit("no memory, and rings all the same")
+        except A.AP26Error:
+            pass
+        for _ in range(3):
+            try:
+                ctx.serve_step()
+                raise SystemExit("no rings, and a step all the same")
+            except A.AP26Error as e:
+                assert e.code == A.E_CUDA
+        fail("cudaMalloc", times=0)
+        ctx.serve_step()
+        assert ctx.serve_step() == 0             # no unit left: all of its K are done
+        ctx.close()
+    """)
